@@ -35,6 +35,12 @@ struct PlanStore {
   DevBuf perm, tw64, tw32;
 };
 
+// The z plan of a precision (FP32 butterflies or FP64 in fixed point).
+template <typename R> const ZPlan<R>& zplan(const FftPlan& p, const FxPlan& f) {
+  if constexpr (sizeof(R) == 4) return p;
+  else return f;
+}
+
 }  // namespace
 
 struct lh_handle {
@@ -75,8 +81,10 @@ struct lh_handle {
   double* tabs = nullptr;  // lu_u, lu_v, u11 (rewritten when dt changes)
   DevScalars* sc = nullptr;
   PlanStore pz, ph, pf;  // z (Ngalz), x half length (Ngalx/2), x full length (Ngalx)
+  FxPlan qz{};           // z in fixed point
   double2* rtw = nullptr;
   PlanStore pz2, ph2, pf2;  // the same for the middle band (bands only)
+  FxPlan qz2{};
   double2* rtw2 = nullptr;
   Dims dmid{};              // the middle band's plane geometry (bands only)
   int tx = 8, chunk = 16;
@@ -210,6 +218,21 @@ int build_plan(lh_handle* h, PlanStore& ps, int n, int keep_half) {
   return LH_OK;
 }
 
+// The fixed-point plan of a length that build_plan accepts.
+int build_fx(lh_handle* h, FxPlan* P, int n) {
+  FxTables t;
+  if (!fx_build(n, P, &t)) return fail(h, LH_EFFT, "transform length %d is too long", n);
+  if (t.tw.empty()) t.tw.push_back(int4{0, 0, 0, 0});
+  short *a, *b, *c, *e;
+  int4* w;
+  int rc;
+  if ((rc = upload(h, &a, t.pos_sample)) || (rc = upload(h, &b, t.pos_freq)) || (rc = upload(h, &c, t.sample_pos)) ||
+      (rc = upload(h, &e, t.freq_pos)) || (rc = upload(h, &w, t.tw)))
+    return rc;
+  P->pos_sample = a; P->pos_freq = b; P->sample_pos = c; P->freq_pos = e; P->tw = w;
+  return LH_OK;
+}
+
 size_t field_elems(const lh_handle* h, char grid) {
   const int ny = grid == 'u' ? h->d.nyu : (grid == 'v' ? h->d.nyv : h->d.nyp);
   return (size_t)ny * h->d.np;
@@ -327,12 +350,13 @@ int build_dt_tables(lh_handle* h) {
 struct BandLaunch {
   const Dims* d;
   const FftPlan *pz, *ph, *pf;
+  const FxPlan* qz;
   const double2* rtw;
   int c_lo, c_hi, f_lo, f_hi;
 };
 int band_launches(const lh_handle* h, BandLaunch* out) {
   const Dims& d = h->d;
-  const BandLaunch fine{&d, &h->pz.plan, &h->ph.plan, &h->pf.plan, h->rtw, 0, 0, 0, 0};
+  const BandLaunch fine{&d, &h->pz.plan, &h->ph.plan, &h->pf.plan, &h->qz, h->rtw, 0, 0, 0, 0};
   if (!d.banded) {
     out[0] = fine;
     out[0].c_lo = 1; out[0].c_hi = d.nyu - 2; out[0].f_lo = 1; out[0].f_hi = d.nyv - 2;
@@ -340,7 +364,7 @@ int band_launches(const lh_handle* h, BandLaunch* out) {
   }
   out[0] = fine;
   out[0].c_lo = 1; out[0].c_hi = d.Nu1; out[0].f_lo = 1; out[0].f_hi = d.Nv1;
-  out[1] = BandLaunch{&h->dmid, &h->pz2.plan, &h->ph2.plan, &h->pf2.plan, h->rtw2, d.Nu1 + 1, d.Nu2, d.Nv1 + 1, d.Nv2};
+  out[1] = BandLaunch{&h->dmid, &h->pz2.plan, &h->ph2.plan, &h->pf2.plan, &h->qz2, h->rtw2, d.Nu1 + 1, d.Nu2, d.Nv1 + 1, d.Nv2};
   out[2] = fine;
   out[2].c_lo = d.Nu2 + 1; out[2].c_hi = d.nyu - 2; out[2].f_lo = d.Nv2 + 1; out[2].f_hi = d.nyv - 2;
   return 3;
@@ -351,7 +375,8 @@ int band_launches(const lh_handle* h, BandLaunch* out) {
 template <typename R>
 struct NlBand {
   const Dims* d;
-  const FftPlan *pz, *ph, *pf;
+  const ZPlan<R>* pz;
+  const FftPlan *ph, *pf;
   const double2* rtw;
   ZJobs<R> zi, zf;
   ProdArgs<R> xp;
@@ -367,7 +392,7 @@ int nl_bands(const lh_handle* h, NlBand<R>* out) {
     const BandLaunch& B = bl[b];
     const Dims& db = *B.d;
     NlBand<R>& o = out[b];
-    o.d = B.d; o.pz = B.pz; o.ph = B.ph; o.pf = B.pf; o.rtw = B.rtw;
+    o.d = B.d; o.pz = &zplan<R>(*B.pz, *B.qz); o.ph = B.ph; o.pf = B.pf; o.rtw = B.rtw;
     const int L0 = std::min(B.c_lo, B.f_lo + 1), L1 = std::max(B.c_hi, B.f_hi + 1);
     {
       const int ul = std::max(1, L0 - 1), uh = std::min(d.nyu - 2, L1);
@@ -530,11 +555,11 @@ int enqueue_substage(lh_handle* h, int k, int upto) {
     ZJobs<R> zi, zf;
     MaskArgs<R> m;
     if (ib_args<R>(h, k, &zi, &m, &zf)) {
-      launch_zinv<R>(zi, d, h->pz.plan, h->tx, st, h->zthreads);
+      launch_zinv<R>(zi, d, zplan<R>(h->pz.plan, h->qz), h->tx, st, h->zthreads);
       mark(h, K_IB_ZINV);
       launch_xmask<R>(m, d, h->ph.plan, h->rtw, st);
       mark(h, K_IB_XMASK);
-      launch_zfwd<R>(zf, d, h->pz.plan, h->tx, 1.0 / d.ngz, st, h->zthreads);
+      launch_zfwd<R>(zf, d, zplan<R>(h->pz.plan, h->qz), h->tx, 1.0 / d.ngz, st, h->zthreads);
       mark(h, K_IB_ZFWD);
     }
   }
@@ -779,7 +804,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
   int rc;
   // FFT plans: z of length ngz, x through a complex transform of ngx/2
   if ((rc = build_plan(h, h->pz, d.ngz, d.nz / 2)) || (rc = build_plan(h, h->ph, d.ngx / 2, 0)) ||
-      (rc = build_plan(h, h->pf, d.ngx, 0)))
+      (rc = build_plan(h, h->pf, d.ngx, 0)) || (rc = build_fx(h, &h->qz, d.ngz)))
     return bail(rc);
   if (d.banded) {
     // the middle band's planes: their own transform lengths and mode counts, the same storage
@@ -788,7 +813,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
     c.ngx = d.ngx2; c.ngz = d.ngz2; c.nkx = d.nkx2; c.nz = d.nz2;
     c.mp = c.nkx * c.ngz;
     if ((rc = build_plan(h, h->pz2, c.ngz, c.nz / 2)) || (rc = build_plan(h, h->ph2, c.ngx / 2, 0)) ||
-        (rc = build_plan(h, h->pf2, c.ngx, 0)))
+        (rc = build_plan(h, h->pf2, c.ngx, 0)) || (rc = build_fx(h, &h->qz2, c.ngz)))
       return bail(rc);
     std::vector<double2> rt(c.ngx / 2 + 1);
     for (int k = 0; k <= c.ngx / 2; ++k) {
@@ -1298,7 +1323,7 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
             zpass_shape<R>(J, *B.d, h->tx, &g, &sm);
             if (g.x == 0) continue;
             ZDesc<R> D{};
-            D.jobs = J; D.d = *B.d; D.p = *B.pz; D.scale = 1.0 / B.d->ngz; D.tx = h->tx;
+            D.jobs = J; D.d = *B.d; D.p = *B.pz; D.scale = 1.0 / B.d->ngz; D.tx = zpass_tile<R>(h->tx);
             D.gx = g.x; D.gy = g.y; D.gz = g.z;
             zd.push_back(D);
           }
@@ -1334,7 +1359,7 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
         size_t sm;
         zpass_shape<R>(a, h->d, h->tx, &g, &sm);
         ZDesc<R> Di{};
-        Di.jobs = a; Di.d = h->d; Di.p = h->pz.plan; Di.scale = 1.0; Di.tx = h->tx; Di.gx = g.x; Di.gy = g.y; Di.gz = g.z;
+        Di.jobs = a; Di.d = h->d; Di.p = zplan<R>(h->pz.plan, h->qz); Di.scale = 1.0; Di.tx = zpass_tile<R>(h->tx); Di.gx = g.x; Di.gy = g.y; Di.gz = g.z;
         zi.push_back(Di); bi.push_back((int)(g.x * g.y * g.z)); si.push_back(sm);
         xmask_shape<R>(mk, h->d, &g, &sm);
         MDesc<R> Dm{};
@@ -1342,7 +1367,7 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
         md.push_back(Dm); bm.push_back((int)(g.x * g.y)); sm_.push_back(sm);
         zpass_shape<R>(c, h->d, h->tx, &g, &sm);
         ZDesc<R> Df{};
-        Df.jobs = c; Df.d = h->d; Df.p = h->pz.plan; Df.scale = 1.0 / h->d.ngz; Df.tx = h->tx;
+        Df.jobs = c; Df.d = h->d; Df.p = zplan<R>(h->pz.plan, h->qz); Df.scale = 1.0 / h->d.ngz; Df.tx = zpass_tile<R>(h->tx);
         Df.gx = g.x; Df.gy = g.y; Df.gz = g.z;
         zf.push_back(Df); bf.push_back((int)(g.x * g.y * g.z)); sf.push_back(sm);
       }
@@ -1777,7 +1802,7 @@ int lh_cfl_dt(lh_handle* h, double cfl, double* dt_out) {
       J.j[2] = ZJob<R>{h->u2, nullptr, (T2*)h->mixv + (size_t)vl * db.mp, nullptr, vl, vh - vl + 1};
       J.njobs = 3;
       J.maxlev = uh - ul + 1;
-      launch_zinv<R>(J, db, *B.pz, h->tx, h->st);
+      launch_zinv<R>(J, db, zplan<R>(*B.pz, *B.qz), h->tx, h->st);
       ProdArgs<R> a{};
       a.mu = (const T2*)h->mixu; a.mw = (const T2*)h->mixw; a.mv = (const T2*)h->mixv;
       for (int i = 0; i < 6; ++i) a.out[i] = (T2*)h->mixp[i];
@@ -1900,7 +1925,7 @@ int lh_cond_accumulate(lh_handle* h) {
     J.j[6] = ZJob<double>{h->r2, nullptr, mx[6], h->cond_vl + 2 * j0, 0, 2 * cvv};
     J.njobs = 7;
     J.maxlev = 2 * std::max(cu, std::max(cvv, cp));
-    launch_zinv<double>(J, d, h->pz.plan, h->tx, st);
+    launch_zinv<double>(J, d, h->qz, h->tx, st);
     CondArgs a{};
     a.mix[0][0] = mx[0]; a.mix[0][1] = mx[1]; a.mix[0][2] = mx[2];
     a.mix[1][0] = mx[3]; a.mix[1][1] = mx[4]; a.mix[1][2] = mx[6];

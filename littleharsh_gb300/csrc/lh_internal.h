@@ -7,6 +7,7 @@
 #include <string>
 
 #include "lh_fft.cuh"
+#include "lh_fxfft.cuh"
 
 struct lh_params;
 
@@ -132,11 +133,16 @@ struct ZJobs {
   int njobs, maxlev;
 };
 
+// The plan a z pass of a precision uses: FP32 butterflies, or 64-bit fixed point for FP64.
+template <typename R> struct ZPlanOf { using T = FftPlan; };
+template <> struct ZPlanOf<double> { using T = FxPlan; };
+template <typename R> using ZPlan = typename ZPlanOf<R>::T;
+
 // Launchers (lh_kernels.cu).  All are asynchronous on `st`.
 template <typename R>
-void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, cudaStream_t st, int threads = 256);
+void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, cudaStream_t st, int threads = 256);
 template <typename R>
-void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, double scale, cudaStream_t st,
+void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, double scale, cudaStream_t st,
                  int threads = 256);
 
 template <typename R>
@@ -248,7 +254,7 @@ template <typename R>
 struct ZDesc {                  // z-inverse or z-forward
   ZJobs<R> jobs;
   Dims d;
-  FftPlan p;
+  ZPlan<R> p;
   double scale;
   int tx, gx, gy, gz;
 };
@@ -323,6 +329,8 @@ void launch_psolve_batch(const Batch<PDesc>& b, cudaStream_t st);
 // grid means no launch).
 template <typename R>
 void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem);
+template <typename R>
+int zpass_tile(int tx);
 template <typename R>
 void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem);
 template <typename R>

@@ -34,9 +34,10 @@ namespace lh {
 // z passes
 // ---------------------------------------------------------------------------
 
-template <typename R>
-__device__ __forceinline__ void zinv_body(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, int bx,
+// FP32 (the mixed form)
+__device__ __forceinline__ void zinv_body(const ZJobs<float>& jobs, const Dims& d, const FftPlan& pz, int tx, int bx,
                                           int by, int bz) {
+  using R = float;
   using T2 = cpx_t<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* sm = reinterpret_cast<T2*>(smraw);  // [ngz][tx]
@@ -71,15 +72,9 @@ __device__ __forceinline__ void zinv_body(const ZJobs<R>& jobs, const Dims& d, c
   }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) k_zinv(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
-                                              const __grid_constant__ FftPlan pz, int tx) {
-  zinv_body<R>(jobs, d, pz, tx, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-template <typename R>
-__device__ __forceinline__ void zfwd_body(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, double scale,
-                                          int bx, int by, int bz) {
+__device__ __forceinline__ void zfwd_body(const ZJobs<float>& jobs, const Dims& d, const FftPlan& pz, int tx,
+                                          double scale, int bx, int by, int bz) {
+  using R = float;
   using T2 = cpx_t<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* sm = reinterpret_cast<T2*>(smraw);  // [ngz][tx]
@@ -100,21 +95,19 @@ __device__ __forceinline__ void zfwd_body(const ZJobs<R>& jobs, const Dims& d, c
   // stage's output is never read when N2/2 = Ngz/3
   fft_dit<R, -1, true>(sm, nb, tx, 1, pz, pz.prune_mid != 0);
   const int h = d.nz / 2, gap = d.ngz - d.nz;
-  if constexpr (sizeof(R) == 4) {
-    if (J.out32) {  // the mixed form's product spectra stay FP32 (only the nonlinear term reads them)
-      T2* __restrict__ dst = reinterpret_cast<T2*>(J.spec_out) + (size_t)lev * d.np;
-      const R sc = (R)scale;
-      for (int e = threadIdx.x; e < d.nz * tx; e += blockDim.x) {
-        const int kk = e / tx, c = e - kk * tx;
-        if (c < nb) {
-          const int slot = kk < h ? kk : kk + gap;
-          const T2 v = sm[slot * tx + c];
-          const int ks = kk < h ? kk : kk - d.nz + d.snz;
-          dst[(size_t)ks * d.spitch + i0 + c] = T2{v.x * sc, v.y * sc};
-        }
+  if (J.out32) {  // the mixed form's product spectra stay FP32 (only the nonlinear term reads them)
+    T2* __restrict__ dst = reinterpret_cast<T2*>(J.spec_out) + (size_t)lev * d.np;
+    const R sc = (R)scale;
+    for (int e = threadIdx.x; e < d.nz * tx; e += blockDim.x) {
+      const int kk = e / tx, c = e - kk * tx;
+      if (c < nb) {
+        const int slot = kk < h ? kk : kk + gap;
+        const T2 v = sm[slot * tx + c];
+        const int ks = kk < h ? kk : kk - d.nz + d.snz;
+        dst[(size_t)ks * d.spitch + i0 + c] = T2{v.x * sc, v.y * sc};
       }
-      return;
     }
+    return;
   }
   double2* __restrict__ dst = J.spec_out + (size_t)lev * d.np;
   for (int e = threadIdx.x; e < d.nz * tx; e += blockDim.x) {
@@ -128,35 +121,195 @@ __device__ __forceinline__ void zfwd_body(const ZJobs<R>& jobs, const Dims& d, c
   }
 }
 
+// FP64: the lines of a tile of columns in 64-bit fixed point (lh_fxfft.cuh).  The tile is copied into shared memory
+// (cp.async: all of it in flight at once; reading it through registers, once for the largest value and once to scale,
+// waited on global memory and took 1.4x as long), a sweep finds each column's largest value, the first pass scales its
+// inputs and the last one writes FP64.  Bound by instruction issue (340 instructions a point, 50-60 % issue) on the
+// integer pipes; the conversions run beside them on the FP64 pipe, in zinv both ways, in zfwd outward with the
+// normalisation (its inputs take integer shifts, or the FP64 pipe would be the bound).  64 registers (four CTAs of 256
+// threads) beat 80.  A step of the 576 x 576 x 450 grid (449 levels transformed) on a GB300: z-inverse 22.9 -> 6.0 ms,
+// z-forward 47.8 -> 11.3 ms against FP64 radix-4/3 butterflies; their memory traffic alone is 1.8 and 3.5 ms.
+
+constexpr int kFxMaxTile = 32;  // columns of a tile (a power of two)
+
+struct FxLines {               // per column of the tile
+  unsigned e[kFxMaxTile];      // high word of the largest |re|, |im|
+  unsigned sum[kFxMaxTile];    // sum of fx_mag
+};
+
+// Combines the threads' values m of their columns into dst: by shuffles over the lanes of the same column, so that one
+// lane per column and warp touches shared memory.
+template <bool SUM>
+__device__ __forceinline__ void fx_combine(unsigned m, unsigned* dst, int tx) {
+  for (int o = 16; o >= tx; o >>= 1) {
+    const unsigned q = __shfl_xor_sync(0xffffffffu, m, o);
+    m = SUM ? m + q : max(m, q);
+  }
+  const int lane = threadIdx.x & 31;
+  if (lane < tx) {
+    if (SUM) atomicAdd(dst + lane, m);
+    else atomicMax(dst + lane, m);
+  }
+}
+
+// After the thread's copies into the tile: biased exponent of the largest value of its column.
+__device__ __forceinline__ int fx_sweep(FxLines& L, const FxCol& C, int n) {
+  const int tx = 1 << C.ltx;
+  if ((int)threadIdx.x < tx) { L.e[threadIdx.x] = 0; L.sum[threadIdx.x] = 0; }
+  fx_copy_wait();
+  __syncthreads();
+  unsigned m = 0;
+#pragma unroll 4
+  for (int r = C.t0; r < n; r += C.dt) m = max(m, fx_hi(reinterpret_cast<const double2*>(C.buf)[r << C.ltx]));
+  fx_combine<false>(m, L.e, tx);
+  __syncthreads();
+  return (int)(L.e[threadIdx.x & (tx - 1)] >> 20);
+}
+
+__device__ __forceinline__ FxCol fx_col(fx2* sm, int tx) {
+  const int ltx = 31 - __clz(tx), c = threadIdx.x & (tx - 1);
+  return FxCol{sm + c, ltx, (int)threadIdx.x >> ltx, (int)blockDim.x >> ltx};
+}
+
+__device__ __forceinline__ void zinv_body(const ZJobs<double>& jobs, const Dims& d, const FxPlan& P, int tx, int bx,
+                                          int by, int bz) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ FxLines L;
+  const ZJob<double> J = jobs.j[bz];
+  const int y = by;
+  if (y >= J.nlev) return;
+  const int lev = J.levels ? J.levels[y] : J.lev0 + y;
+  const FxCol C = fx_col(reinterpret_cast<fx2*>(smraw), tx);  // [ngz][tx]
+  const int i = bx * tx + (threadIdx.x & (tx - 1));
+  const bool in = i < d.nkx;
+  const double2* __restrict__ src = J.spec_in + (size_t)lev * d.np + i;
+  const int h = d.nz / 2, gap = d.ngz - d.nz, pitch = d.spitch;
+  // slots z < nz/2 hold the first rows of the stored mode set, the last nz/2 slots its last rows, the slots between
+  // the 3/2 padding
+  const double2* __restrict__ top = src + (ptrdiff_t)(d.snz - d.ngz) * pitch;
+#pragma unroll 4
+  for (int z = C.t0; z < d.ngz; z += C.dt) {
+    fx2* s = C.buf + ((int)P.pos_sample[z] << C.ltx);
+    if (!in || (unsigned)(z - h) < (unsigned)gap) *s = fx2{0, 0};
+    else fx_copy(s, (z < h ? src : top) + (ptrdiff_t)z * pitch);
+  }
+  const int e = fx_sweep(L, C, d.ngz);
+  const FxIn scale(e);
+  unsigned sum = 0;
+  auto load = [&](double2 v) {
+    const i64 x = scale(v.x), yy = scale(v.y);
+    sum += fx_mag(x) + fx_mag(yy);
+    return fx2{yy, x};  // parts exchanged: an inverse transform
+  };
+  double2* __restrict__ dst = J.mix + (size_t)y * d.mp + i;
+  const int S = fx_scale(e);
+  int g = 0;
+  auto total = [&]() {
+    fx_combine<true>(sum, L.sum, tx);
+    __syncthreads();
+    return g = fx_inv_shift(L.sum[threadIdx.x & (tx - 1)], P.shift);
+  };
+  auto store = [&](int z, fx2 v) {
+    const FxOut out(e, S - g);
+    if (in) dst[(size_t)z * d.nkx] = double2{out(v.y), out(v.x)};
+  };
+  fx_tile(C, P, load, total, store);
+}
+
+__device__ __forceinline__ void zfwd_body(const ZJobs<double>& jobs, const Dims& d, const FxPlan& P, int tx,
+                                          double norm, int bx, int by, int bz) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ FxLines L;
+  const ZJob<double> J = jobs.j[bz];
+  const int y = by;
+  if (y >= J.nlev) return;
+  const int lev = J.levels ? J.levels[y] : J.lev0 + y;
+  const FxCol C = fx_col(reinterpret_cast<fx2*>(smraw), tx);  // [ngz][tx]
+  const int i = bx * tx + (threadIdx.x & (tx - 1));
+  const bool in = i < d.nkx;
+  const double2* __restrict__ src = J.mix + (size_t)y * d.mp + i;
+#pragma unroll 4
+  for (int z = C.t0; z < d.ngz; z += C.dt) {
+    fx2* s = C.buf + ((int)P.pos_sample[z] << C.ltx);
+    if (in) fx_copy(s, src + (size_t)z * d.nkx);
+    else *s = fx2{0, 0};
+  }
+  const int e = fx_sweep(L, C, d.ngz);
+  auto load = [&](double2 v) { return fx2{fx_from(v.x, e), fx_from(v.y, e)}; };
+  auto total = [&]() {
+    __syncthreads();
+    return P.shift;
+  };
+  const int h = d.nz / 2, gap = d.ngz - d.nz;
+  double2* __restrict__ dst = J.spec_out + (size_t)lev * d.np + i;
+  double2* __restrict__ top = dst + (ptrdiff_t)(d.snz - d.ngz) * d.spitch;
+  const FxOut out(e, fx_scale(e) - P.shift);
+  // the integers times norm 2^-S in one product
+  const double f = out.bad ? __longlong_as_double(0x7ff8000000000000ll) : norm * __hiloint2double((int)((unsigned)(1023 - out.S) << 20), 0);
+  auto store = [&](int k, fx2 v) {
+    if (!in || (unsigned)(k - h) < (unsigned)gap) return;  // the truncation
+    (k < h ? dst : top)[(ptrdiff_t)k * d.spitch] =
+        out.far && !out.bad ? double2{out(v.x) * norm, out(v.y) * norm}
+                            : double2{__ll2double_rn(v.x) * f, __ll2double_rn(v.y) * f};
+  };
+  fx_tile(C, P, load, total, store);
+}
+
 template <typename R>
-__global__ void __launch_bounds__(256) k_zfwd(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
-                                              const __grid_constant__ FftPlan pz, int tx, double scale) {
-  zfwd_body<R>(jobs, d, pz, tx, scale, blockIdx.x, blockIdx.y, blockIdx.z);
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zinv(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
+                                              const __grid_constant__ ZPlan<R> pz, int tx) {
+  zinv_body(jobs, d, pz, tx, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zfwd(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
+                                              const __grid_constant__ ZPlan<R> pz, int tx, double scale) {
+  zfwd_body(jobs, d, pz, tx, scale, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Width of the z tile a precision's kernels use: the FP64 ones take a power of two up to 32 (at or below tx).
+template <typename R>
+int zpass_tile(int tx) {
+  if (sizeof(R) == 4) return tx;
+  int p = 1;
+  while (2 * p <= tx && 2 * p <= kFxMaxTile) p *= 2;
+  return p;
 }
 
 template <typename R>
 void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem) {
+  tx = zpass_tile<R>(tx);
   *grid = (jobs.njobs == 0 || jobs.maxlev == 0) ? dim3(0, 0, 0) : dim3((d.nkx + tx - 1) / tx, jobs.maxlev, jobs.njobs);
   *smem = sizeof(cpx_t<R>) * (size_t)d.ngz * tx;
 }
 
+// Threads of a z-pass CTA: `threads` (128 or 256), and in FP64 no more than share the tile's radix-8 butterflies evenly
+// over the rounds that many threads need.
 template <typename R>
-void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, cudaStream_t st, int threads) {
+int zpass_threads(const Dims& d, int tx, int threads) {
+  threads = threads == 128 ? 128 : 256;
+  if (sizeof(R) == 4) return threads;
+  const int items = std::max(1, d.ngz / 8) * zpass_tile<R>(tx), rounds = (items + threads - 1) / threads;
+  return std::min(threads, ((items + rounds - 1) / rounds + 31) / 32 * 32);
+}
+
+template <typename R>
+void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, cudaStream_t st, int threads) {
   dim3 grid;
   size_t sm;
   zpass_shape(jobs, d, tx, &grid, &sm);
   if (grid.x == 0) return;
-  k_zinv<R><<<grid, threads == 128 ? 128 : 256, sm, st>>>(jobs, d, pz, tx);
+  k_zinv<R><<<grid, zpass_threads<R>(d, tx, threads), sm, st>>>(jobs, d, pz, zpass_tile<R>(tx));
 }
 
 template <typename R>
-void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, double scale, cudaStream_t st,
+void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, double scale, cudaStream_t st,
                  int threads) {
   dim3 grid;
   size_t sm;
   zpass_shape(jobs, d, tx, &grid, &sm);
   if (grid.x == 0) return;
-  k_zfwd<R><<<grid, threads == 128 ? 128 : 256, sm, st>>>(jobs, d, pz, tx, scale);
+  k_zfwd<R><<<grid, zpass_threads<R>(d, tx, threads), sm, st>>>(jobs, d, pz, zpass_tile<R>(tx), scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -1510,19 +1663,19 @@ __device__ __forceinline__ int batch_member(const Batch<D>& b, int blk) {
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 5) k_zinv_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zinv_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
   const int m = batch_member(b, blockIdx.x);
   const ZDesc<R>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m], gxy = D.gx * D.gy;
-  zinv_body<R>(D.jobs, D.d, D.p, D.tx, q % D.gx, (q % gxy) / D.gx, q / gxy);
+  zinv_body(D.jobs, D.d, D.p, D.tx, q % D.gx, (q % gxy) / D.gx, q / gxy);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 5) k_zfwd_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zfwd_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
   const int m = batch_member(b, blockIdx.x);
   const ZDesc<R>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m], gxy = D.gx * D.gy;
-  zfwd_body<R>(D.jobs, D.d, D.p, D.tx, D.scale, q % D.gx, (q % gxy) / D.gx, q / gxy);
+  zfwd_body(D.jobs, D.d, D.p, D.tx, D.scale, q % D.gx, (q % gxy) / D.gx, q / gxy);
 }
 
 template <typename R>
@@ -1682,10 +1835,10 @@ cudaError_t configure_kernels() {
   return cudaSuccess;
 }
 
-template void launch_zinv<double>(const ZJobs<double>&, const Dims&, const FftPlan&, int, cudaStream_t, int);
-template void launch_zinv<float>(const ZJobs<float>&, const Dims&, const FftPlan&, int, cudaStream_t, int);
-template void launch_zfwd<double>(const ZJobs<double>&, const Dims&, const FftPlan&, int, double, cudaStream_t, int);
-template void launch_zfwd<float>(const ZJobs<float>&, const Dims&, const FftPlan&, int, double, cudaStream_t, int);
+template void launch_zinv<double>(const ZJobs<double>&, const Dims&, const ZPlan<double>&, int, cudaStream_t, int);
+template void launch_zinv<float>(const ZJobs<float>&, const Dims&, const ZPlan<float>&, int, cudaStream_t, int);
+template void launch_zfwd<double>(const ZJobs<double>&, const Dims&, const ZPlan<double>&, int, double, cudaStream_t, int);
+template void launch_zfwd<float>(const ZJobs<float>&, const Dims&, const ZPlan<float>&, int, double, cudaStream_t, int);
 template void launch_xprod<double>(const ProdArgs<double>&, const Dims&, const FftPlan&, const FftPlan&, const double2*,
                                    cudaStream_t);
 template void launch_xprod<float>(const ProdArgs<float>&, const Dims&, const FftPlan&, const FftPlan&, const double2*,
@@ -1693,6 +1846,8 @@ template void launch_xprod<float>(const ProdArgs<float>&, const Dims&, const Fft
 template void launch_xmask<double>(const MaskArgs<double>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
 template void launch_xmask<float>(const MaskArgs<float>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
 template void zpass_shape<double>(const ZJobs<double>&, const Dims&, int, dim3*, size_t*);
+template int zpass_tile<double>(int);
+template int zpass_tile<float>(int);
 template void zpass_shape<float>(const ZJobs<float>&, const Dims&, int, dim3*, size_t*);
 template void xprod_shape<double>(const ProdArgs<double>&, const Dims&, dim3*, size_t*);
 template void xprod_shape<float>(const ProdArgs<float>&, const Dims&, dim3*, size_t*);

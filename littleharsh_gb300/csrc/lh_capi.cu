@@ -81,10 +81,10 @@ struct lh_handle {
   double* tabs = nullptr;  // lu_u, lu_v, u11 (rewritten when dt changes)
   DevScalars* sc = nullptr;
   PlanStore pz, ph, pf;  // z (Ngalz), x half length (Ngalx/2), x full length (Ngalx)
-  FxPlan qz{};           // z in fixed point
+  FxPlan qz{}, qx{};     // z and x in fixed point
   double2* rtw = nullptr;
   PlanStore pz2, ph2, pf2;  // the same for the middle band (bands only)
-  FxPlan qz2{};
+  FxPlan qz2{}, qx2{};
   double2* rtw2 = nullptr;
   Dims dmid{};              // the middle band's plane geometry (bands only)
   int tx = 8, chunk = 16;
@@ -223,14 +223,35 @@ int build_fx(lh_handle* h, FxPlan* P, int n) {
   FxTables t;
   if (!fx_build(n, P, &t)) return fail(h, LH_EFFT, "transform length %d is too long", n);
   if (t.tw.empty()) t.tw.push_back(int4{0, 0, 0, 0});
-  short *a, *b, *c, *e;
+  short *a, *b, *c, *e, *f;
   int4* w;
   int rc;
   if ((rc = upload(h, &a, t.pos_sample)) || (rc = upload(h, &b, t.pos_freq)) || (rc = upload(h, &c, t.sample_pos)) ||
-      (rc = upload(h, &e, t.freq_pos)) || (rc = upload(h, &w, t.tw)))
+      (rc = upload(h, &e, t.freq_pos)) || (rc = upload(h, &f, t.turn)) || (rc = upload(h, &w, t.tw)))
     return rc;
-  P->pos_sample = a; P->pos_freq = b; P->sample_pos = c; P->freq_pos = e; P->tw = w;
+  P->pos_sample = a; P->pos_freq = b; P->sample_pos = c; P->freq_pos = e; P->turn = f; P->tw = w;
   return LH_OK;
+}
+
+// Levels per CTA of the FP64 product pass: the chunk with the least estimated time, (CTAs / CTAs resident at once, at least one wave)
+// x (levels + 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (FP64 product pass,
+// chunks of 2 / 4 / 8 / 16 levels: 48 x 48 x 66 0.11 / 0.15 / 0.25 / 0.45 ms a step, 96 x 96 x 130 0.51 / 0.46 / 0.46 /
+// 0.58, 162 x 108 x 124 0.96 / 0.82 / 0.76 / 0.95); on large ones long chunks save the repeated level (576 x 576 x 450,
+// 8 / 16 / 32 / 64: 38.6 / 37.3 / 36.9 / 37.3).  The mixed form keeps 16 or 32 (with this rule 96 x 96 x 130 takes 1 %
+// longer).
+int default_chunk(const lh_handle* h) {
+  const Dims& d = h->d;
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  const double resident = (double)sms * xprod_ctas_per_sm(d);
+  int best = 2;
+  double least = 1e300;
+  for (int c : {2, 4, 8, 16, 32}) {
+    const double ctas = (double)d.ngz * ((d.nyu - 2 + c - 1) / c);
+    const double t = std::max(1.0, ctas / resident) * (c + 1.3);
+    if (t < least) { least = t; best = c; }
+  }
+  return best;
 }
 
 size_t field_elems(const lh_handle* h, char grid) {
@@ -350,13 +371,13 @@ int build_dt_tables(lh_handle* h) {
 struct BandLaunch {
   const Dims* d;
   const FftPlan *pz, *ph, *pf;
-  const FxPlan* qz;
+  const FxPlan *qz, *qx;
   const double2* rtw;
   int c_lo, c_hi, f_lo, f_hi;
 };
 int band_launches(const lh_handle* h, BandLaunch* out) {
   const Dims& d = h->d;
-  const BandLaunch fine{&d, &h->pz.plan, &h->ph.plan, &h->pf.plan, &h->qz, h->rtw, 0, 0, 0, 0};
+  const BandLaunch fine{&d, &h->pz.plan, &h->ph.plan, &h->pf.plan, &h->qz, &h->qx, h->rtw, 0, 0, 0, 0};
   if (!d.banded) {
     out[0] = fine;
     out[0].c_lo = 1; out[0].c_hi = d.nyu - 2; out[0].f_lo = 1; out[0].f_hi = d.nyv - 2;
@@ -364,10 +385,16 @@ int band_launches(const lh_handle* h, BandLaunch* out) {
   }
   out[0] = fine;
   out[0].c_lo = 1; out[0].c_hi = d.Nu1; out[0].f_lo = 1; out[0].f_hi = d.Nv1;
-  out[1] = BandLaunch{&h->dmid, &h->pz2.plan, &h->ph2.plan, &h->pf2.plan, &h->qz2, h->rtw2, d.Nu1 + 1, d.Nu2, d.Nv1 + 1, d.Nv2};
+  out[1] = BandLaunch{&h->dmid, &h->pz2.plan, &h->ph2.plan, &h->pf2.plan, &h->qz2, &h->qx2, h->rtw2, d.Nu1 + 1, d.Nu2, d.Nv1 + 1, d.Nv2};
   out[2] = fine;
   out[2].c_lo = d.Nu2 + 1; out[2].c_hi = d.nyu - 2; out[2].f_lo = d.Nv2 + 1; out[2].f_hi = d.nyv - 2;
   return 3;
+}
+
+template <typename R>
+XPlan<R> xplan(const lh_handle* h, const BandLaunch& B) {
+  if constexpr (sizeof(R) == 4) return XPlan<R>{*B.ph, *B.pf, B.rtw};
+  else return XPlan<R>{*B.qx, h->t.wcq, h->t.wfq};
 }
 
 // The nonlinear term's plane work for one band: z-inverse of the levels the band's products need, products,
@@ -376,8 +403,8 @@ template <typename R>
 struct NlBand {
   const Dims* d;
   const ZPlan<R>* pz;
-  const FftPlan *ph, *pf;
-  const double2* rtw;
+  XPlan<R> px;
+  double norm;  // of the z-forward: 1/Ngalz, and in FP64 also the product pass's 1/Ngalx
   ZJobs<R> zi, zf;
   ProdArgs<R> xp;
 };
@@ -392,7 +419,8 @@ int nl_bands(const lh_handle* h, NlBand<R>* out) {
     const BandLaunch& B = bl[b];
     const Dims& db = *B.d;
     NlBand<R>& o = out[b];
-    o.d = B.d; o.pz = &zplan<R>(*B.pz, *B.qz); o.ph = B.ph; o.pf = B.pf; o.rtw = B.rtw;
+    o.d = B.d; o.pz = &zplan<R>(*B.pz, *B.qz); o.px = xplan<R>(h, B);
+    o.norm = sizeof(R) == 4 ? 1.0 / db.ngz : 1.0 / ((double)db.ngz * db.ngx);
     const int L0 = std::min(B.c_lo, B.f_lo + 1), L1 = std::max(B.c_hi, B.f_hi + 1);
     {
       const int ul = std::max(1, L0 - 1), uh = std::min(d.nyu - 2, L1);
@@ -453,11 +481,11 @@ void enqueue_nonlinear(lh_handle* h, cudaStream_t st, bool zinv, bool xprod, boo
       mark(h, K_ZINV);
     }
     if (xprod) {
-      launch_xprod<R>(B.xp, *B.d, *B.ph, *B.pf, B.rtw, st);
+      launch_xprod<R>(B.xp, *B.d, B.px, st);
       mark(h, K_XPROD);
     }
     if (zfwd) {
-      launch_zfwd<R>(B.zf, *B.d, *B.pz, h->tx, 1.0 / B.d->ngz, st, h->zthreads);
+      launch_zfwd<R>(B.zf, *B.d, *B.pz, h->tx, B.norm, st, h->zthreads);
       mark(h, K_ZFWD);
     }
   }
@@ -804,7 +832,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
   int rc;
   // FFT plans: z of length ngz, x through a complex transform of ngx/2
   if ((rc = build_plan(h, h->pz, d.ngz, d.nz / 2)) || (rc = build_plan(h, h->ph, d.ngx / 2, 0)) ||
-      (rc = build_plan(h, h->pf, d.ngx, 0)) || (rc = build_fx(h, &h->qz, d.ngz)))
+      (rc = build_plan(h, h->pf, d.ngx, 0)) || (rc = build_fx(h, &h->qz, d.ngz)) || (rc = build_fx(h, &h->qx, d.ngx)))
     return bail(rc);
   if (d.banded) {
     // the middle band's planes: their own transform lengths and mode counts, the same storage
@@ -813,7 +841,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
     c.ngx = d.ngx2; c.ngz = d.ngz2; c.nkx = d.nkx2; c.nz = d.nz2;
     c.mp = c.nkx * c.ngz;
     if ((rc = build_plan(h, h->pz2, c.ngz, c.nz / 2)) || (rc = build_plan(h, h->ph2, c.ngx / 2, 0)) ||
-        (rc = build_plan(h, h->pf2, c.ngx, 0)) || (rc = build_fx(h, &h->qz2, c.ngz)))
+        (rc = build_plan(h, h->pf2, c.ngx, 0)) || (rc = build_fx(h, &h->qz2, c.ngz)) || (rc = build_fx(h, &h->qx2, c.ngx)))
       return bail(rc);
     std::vector<double2> rt(c.ngx / 2 + 1);
     for (int k = 0; k <= c.ngx / 2; ++k) {
@@ -849,6 +877,12 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
       return bail(rc);
     h->t.kx = pkx; h->t.kz = pkz; h->t.k2x = pk2x; h->t.k2z = pk2z; h->t.d2u = pd2u; h->t.d2v = pd2v;
     h->t.cu = pcu; h->t.cv = pcv; h->t.wc = pwc; h->t.wf = pwf; h->t.dyc = pdyc; h->t.dyvw = pdyvw;
+    std::vector<int4> wcq, wfq;
+    for (double w : wc) wcq.push_back(fx_weight(w));
+    for (double w : wf) wfq.push_back(fx_weight(w));
+    int4 *pwcq, *pwfq;
+    if ((rc = upload(h, &pwcq, wcq)) || (rc = upload(h, &pwfq, wfq))) return bail(rc);
+    h->t.wcq = pwcq; h->t.wfq = pwfq;
     // the same values rounded to float (to nearest, as a device conversion would round them)
     auto rounded = [](const std::vector<double>& v) { return std::vector<float>(v.begin(), v.end()); };
     float *pkxf, *pkzf, *pcuf, *pcvf;
@@ -990,7 +1024,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
   // z tile width: narrow tiles keep several CTAs per SM so that one CTA's loads overlap another's
   // butterflies (measured on configuration 2: FP64 best at 4, mixed at 8)
   h->tx = h->precision == LH_PREC_MIXED ? 8 : 4;
-  h->chunk = d.nyu > 256 ? 32 : 16;
+  h->chunk = h->precision == LH_PREC_MIXED ? (d.nyu > 256 ? 32 : 16) : default_chunk(h);
   // launch-shape overrides for tuning sweeps: LH_TX (z tile width, 1..64), LH_CHUNK (levels per x-pass CTA)
   if (const char* v = std::getenv("LH_TX")) { const int x = std::atoi(v); if (x >= 1 && x <= 64) h->tx = x; }
   if (const char* v = std::getenv("LH_CHUNK")) { const int x = std::atoi(v); if (x >= 1 && x <= 4096) h->chunk = x; }
@@ -1316,14 +1350,14 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
             xprod_shape<R>(xa, *B.d, &g, &sm);
             if (g.x == 0) continue;
             XDesc<R> D{};
-            D.a = xa; D.d = *B.d; D.ph = *B.ph; D.pf = *B.pf; D.rtw = B.rtw; D.gx = g.x; D.gy = g.y;
+            D.a = xa; D.d = *B.d; D.p = B.px; D.gx = g.x; D.gy = g.y;
             xd.push_back(D);
           } else {
             const ZJobs<R>& J = part == 0 ? B.zi : B.zf;
             zpass_shape<R>(J, *B.d, h->tx, &g, &sm);
             if (g.x == 0) continue;
             ZDesc<R> D{};
-            D.jobs = J; D.d = *B.d; D.p = *B.pz; D.scale = 1.0 / B.d->ngz; D.tx = zpass_tile<R>(h->tx);
+            D.jobs = J; D.d = *B.d; D.p = *B.pz; D.scale = B.norm; D.tx = zpass_tile<R>(h->tx);
             D.gx = g.x; D.gy = g.y; D.gz = g.z;
             zd.push_back(D);
           }
@@ -1810,7 +1844,7 @@ int lh_cfl_dt(lh_handle* h, double cfl, double* dt_out) {
       a.dxi = db.ngx / h->Lx; a.dzi = db.ngz / h->Lz;
       a.sc = h->sc; a.want_cfl = 1; a.chunk = h->chunk; a.split = h->xsplit; a.threads = h->xthreads;
       a.c_lo = B.c_lo; a.c_hi = B.c_hi; a.f_lo = B.c_lo; a.f_hi = B.c_lo - 1;  // centres only
-      launch_xprod<R>(a, db, *B.ph, *B.pf, B.rtw, h->st);
+      launch_xprod<R>(a, db, xplan<R>(h, B), h->st);
     }
   };
   if (h->precision == LH_PREC_MIXED) run(0.0f);

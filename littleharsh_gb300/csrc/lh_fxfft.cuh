@@ -65,6 +65,7 @@ struct FxPlan {
   const short* pos_freq;     // position of frequency k
   const short* sample_pos;   // sample at a position
   const short* freq_pos;     // frequency at a position
+  const short* turn;         // pos_sample[freq_pos[.]]: from the place of an output to that of an input
   const int4* tw;            // two int4 per twiddle: (w_r, w_r + w_i), (w_i - w_r, -), each high and low word
 };
 
@@ -240,13 +241,13 @@ FX_HD int fx_exp(unsigned hi) { return (int)((hi >> 20) & 2047u); }
 // 2^kFxBits, so their moduli are below 2^(kFxBits + 1/2).
 FX_HD int fx_scale(int e) { return kFxBits - ((e ? e : 1) - 1022); }
 
-// An upper bound of |x| for a scaled value, in units of 2^38.
+// An upper bound of |x| for a scaled value, in units of 2^42: 2^15 of them (two parts of the longest line) fit 32 bits.
 FX_HD unsigned fx_mag(i64 x) {
   const int h = (int)(x >> 32);
-  return ((unsigned)(h ^ (h >> 31)) >> 6) + 1u;
+  return ((unsigned)(h ^ (h >> 31)) >> 10) + 1u;
 }
 
-// Bits that an inverse line is shifted right by over its passes: its sum of moduli, at most sum * 2^38 for the sum of
+// Bits that an inverse line is shifted right by over its passes: its sum of moduli, at most sum * 2^42 for the sum of
 // fx_mag, comes down to 2^(kFxBits + 1), which no partial sum can exceed; never more than the plan's own shifts,
 // which hold for every line.
 FX_HD int fx_inv_shift(unsigned sum, int most) {
@@ -256,7 +257,7 @@ FX_HD int fx_inv_shift(unsigned sum, int most) {
 #else
   while (bits < 32 && (sum >> bits)) ++bits;
 #endif
-  const int g = bits - (kFxBits + 1 - 38);
+  const int g = bits - (kFxBits + 1 - 42);
   return g < 0 ? 0 : (g < most ? g : most);
 }
 
@@ -332,6 +333,17 @@ __device__ __forceinline__ void fx_pass(fx2* buf, int nb, const FxPlan& P, const
     case 8: { constexpr int RAD = 8; CALL; break; } \
     default: { constexpr int RAD = 9; CALL; break; } \
   }
+
+// All passes of nb vectors of shared memory, vector v at buf[v * n]: samples at their pos_sample places, frequency k comes
+// out at pos_freq[k].  sum: the sums of fx_mag of inverse lines, NULL for forward ones.  A barrier follows each pass.
+static __device__ __noinline__ void fx_fft(fx2* buf, int nb, const FxPlan& P, const unsigned* sum) {
+  auto shift = [&](const FxPass& ps, int v) { return fx_pass_shift(ps, sum ? fx_inv_shift(sum[v], P.shift) : P.shift); };
+  for (int i = 0; i < P.npass; ++i) {
+    const FxPass& ps = P.ps[i];
+    FX_RADIX(ps.rad, (fx_pass<RAD>(buf, nb, P, ps, [&](int v) { return shift(ps, v); })));
+    __syncthreads();
+  }
+}
 
 // 16 bytes from global to shared memory, asynchronously
 __device__ __forceinline__ void fx_copy(fx2* dst, const double2* src) {
@@ -419,6 +431,7 @@ __device__ __forceinline__ void fx_tile(const FxCol& C, const FxPlan& P, In in, 
 struct FxIn {
   int e, add, least;  // add: S << 20; least: high words up to this one scale to nothing
   bool far;           // exponents beyond the conversion's range: by integer shifts
+  __device__ __forceinline__ FxIn() {}
   __device__ __forceinline__ explicit FxIn(int e_) : e(e_) {
     const int S = fx_scale(e);
     add = (int)((unsigned)S << 20);
@@ -453,7 +466,12 @@ __device__ __forceinline__ unsigned fx_hi(double2 v) {
   return max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
 }
 // a shifted left (s >= 0) or right (s < 0)
-__device__ __forceinline__ i64 fx_shift(i64 a, int s) { return s >= 0 ? fx_shl(a, min(s, 63)) : a >> min(-s, 63); }
+__device__ __forceinline__ i64 fx_shift(i64 a, int s) { return s >= 0 ? fx_shl(a, s) : a >> -s; }
+// magnitude bits of the high word
+__device__ __forceinline__ unsigned fx_bits(i64 a) {
+  const int h = (int)(a >> 32);
+  return (unsigned)(h ^ (h >> 31));
+}
 
 #endif
 
@@ -462,7 +480,7 @@ __device__ __forceinline__ i64 fx_shift(i64 a, int s) { return s >= 0 ? fx_shl(a
 // ---------------------------------------------------------------------------
 
 struct FxTables {
-  std::vector<short> pos_sample, pos_freq, sample_pos, freq_pos;
+  std::vector<short> pos_sample, pos_freq, sample_pos, freq_pos, turn;
   std::vector<int4> tw;
 };
 
@@ -474,6 +492,15 @@ inline void fx_word(long double v, int* h, int* l) {
   *l = (int)q;
 }
 
+// An interpolation weight as (high, low word of m 2^62, k), w = m 2^k with |m| < 2: k = 0 but for weights beyond [-1, 1].
+inline int4 fx_weight(double w) {
+  int k = 0;
+  while (std::fabs(w) > 1.0 && k < 1000) { w *= 0.5; ++k; }
+  int4 r{0, 0, k, 0};
+  fx_word(w, &r.x, &r.y);
+  return r;
+}
+
 inline unsigned fx_div_mult(unsigned d) { return d > 1 ? 0xFFFFFFFFu / d + 1u : 0u; }
 
 // Fills the plan and its tables for a length of factors 2 and 3; false for another one.
@@ -481,7 +508,7 @@ inline bool fx_build(int n, FxPlan* plan, FxTables* tab) {
   int P = 1, Q = 1, m = n, a = 0, b = 0;
   while (m % 2 == 0) { m /= 2; P *= 2; ++a; }
   while (m % 3 == 0) { m /= 3; Q *= 3; ++b; }
-  if (m != 1 || n > 32767) return false;
+  if (m != 1 || n > 16384) return false;
   int rad[2][kFxMaxPass], np[2] = {0, 0};
   if (a == 1) rad[0][np[0]++] = 2;
   else {
@@ -562,6 +589,8 @@ inline bool fx_build(int n, FxPlan* plan, FxTables* tab) {
       mm *= r;
     }
   }
+  tab->turn.resize(n);
+  for (int i = 0; i < n; ++i) tab->turn[i] = tab->pos_sample[tab->freq_pos[i]];
   plan->npass = np[0] + np[1];
   if (plan->npass) {
     const FxPass& l = plan->ps[plan->npass - 1];

@@ -74,6 +74,8 @@ struct Tables {
   const double* cv;    // [nyv] ddthetavi*dthdyv
   const double* wc;    // [nyu] weight of face j in the centre-j interpolation of v
   const double* wf;    // [nyv] weight of centre j+1 in the face-j interpolation of u, w
+  const int4* wcq;     // [nyu] wc in fixed point (XPlan)
+  const int4* wfq;     // [nyv] wf
   const double* dyc;   // [nyu] 1/(yv(j)-yv(j-1)) at centres, for the CFL number
   const double* dyvw;  // [nn+2] yv(j)-yv(j-1), j = 1..nn+1 at index j (flow rate)
   const double* lu_u;  // [3 kRK][3][nyu] Helmholtz LU (a1, 1/diag, scaled a3), u grid, long columns
@@ -173,9 +175,18 @@ struct ProdArgs {
   const double2 *us, *ws;
   int nps;
 };
+// What the product pass transforms with: FP32 half- and full-length plans and the half-length form's twiddles, or the
+// fixed-point plan and interpolation weights of FP64.
+template <typename R> struct XPlan {
+  FftPlan ph, pf;
+  const double2* rtw;
+};
+template <> struct XPlan<double> {
+  FxPlan pf;
+  const int4 *wc, *wf;  // wc, wf of the product arguments as (high, low word, k): m 2^k with 62 fractional bits of m
+};
 template <typename R>
-void launch_xprod(const ProdArgs<R>& a, const Dims& d, const FftPlan& ph, const FftPlan& pf, const double2* rtw,
-                  cudaStream_t st);
+void launch_xprod(const ProdArgs<R>& a, const Dims& d, const XPlan<R>& p, cudaStream_t st);
 
 template <typename R>
 struct MaskArgs {
@@ -262,8 +273,7 @@ template <typename R>
 struct XDesc {                  // x pass with the products
   ProdArgs<R> a;
   Dims d;
-  FftPlan ph, pf;
-  const double2* rtw;
+  XPlan<R> p;
   int gx, gy;
 };
 template <typename R>
@@ -331,6 +341,8 @@ template <typename R>
 void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem);
 template <typename R>
 int zpass_tile(int tx);
+// FP64 product-pass CTAs (of up to 256 threads) resident on an SM, from their threads, registers and shared memory.
+int xprod_ctas_per_sm(const Dims& d);
 template <typename R>
 void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem);
 template <typename R>

@@ -429,10 +429,13 @@ __device__ void x_forward_pairs(int np2, cpx_t<R>* F, cpx_t<R>* const* rows, con
   __syncthreads();
 }
 
-template <typename R>
-__device__ __forceinline__ void xprod_body(const ProdArgs<R>& a, const Dims& d, const FftPlan& ph, const FftPlan& pf,
-                                           const double2* __restrict__ rtw, int bx, int by) {
+// FP32 (the mixed form)
+__device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims& d, const XPlan<float>& plan, int bx,
+                                           int by) {
+  using R = float;
   using T2 = cpx_t<R>;
+  const FftPlan &ph = plan.ph, &pf = plan.pf;
+  const double2* __restrict__ rtw = plan.rtw;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ngx = d.ngx, h = ngx / 2, hp = h + 1;
   // 3 vectors of ngx, 2 with a.split (also holds the half-length v transform)
@@ -484,35 +487,27 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<R>& a, const Dims& d, 
     // with a.split and both kinds, the face pair goes through the buffer after the centre pairs' transform
     const bool later = a.split && cprod && fprod;
     const int fslot = (cprod && !later) ? 2 : 0;
-    // mixed form: the level means at centre jj and face jj-1 (the FP64 form transforms u and w whole)
+    // the level means at centre jj and face jj-1
     R Uc = (R)0, Wc = (R)0, Uf = (R)0, Wf = (R)0;
-    if constexpr (sizeof(R) == 4) {
-      if (a.mean_split) {
-        const R Um = (R)a.us[(size_t)(jj - 1) * a.nps].x, Wm = (R)a.ws[(size_t)(jj - 1) * a.nps].x;
-        Uc = (R)a.us[(size_t)jj * a.nps].x;
-        Wc = (R)a.ws[(size_t)jj * a.nps].x;
-        Uf = Um + wfj * (Uc - Um);
-        Wf = Wm + wfj * (Wc - Wm);
-      }
+    if (a.mean_split) {
+      const R Um = (R)a.us[(size_t)(jj - 1) * a.nps].x, Wm = (R)a.ws[(size_t)(jj - 1) * a.nps].x;
+      Uc = (R)a.us[(size_t)jj * a.nps].x;
+      Wc = (R)a.ws[(size_t)jj * a.nps].x;
+      Uf = Um + wfj * (Uc - Um);
+      Wf = Wm + wfj * (Wc - Wm);
     }
     auto face_pair = [&](int x, R u, R w, int px) {
       const R uf = up[x] + wfj * (u - up[x]);
       const R wf = wp[x] + wfj * (w - wp[x]);
-      if constexpr (sizeof(R) == 4) F[sxi<R>(fslot * ngx + px)] = T2{(Uf + uf) * vp[x], (Wf + wf) * vp[x]};
-      else F[sxi<R>(fslot * ngx + px)] = T2{uf * vp[x], wf * vp[x]};
+      F[sxi<R>(fslot * ngx + px)] = T2{(Uf + uf) * vp[x], (Wf + wf) * vp[x]};
     };
     for (int x = threadIdx.x; x < ngx; x += blockDim.x) {
       const R u = uc[x], w = wc[x];
       const int px = pf.perm[x];
       if (cprod) {
         const R v = vp[x] + wcj * (vc[x] - vp[x]);
-        if constexpr (sizeof(R) == 4) {
-          F[sxi<R>(px)] = T2{u * ((Uc + Uc) + u), u * (Wc + w) + Uc * w};
-          F[sxi<R>(ngx + px)] = T2{w * ((Wc + Wc) + w), v * v};
-        } else {
-          F[sxi<R>(px)] = T2{u * u, u * w};
-          F[sxi<R>(ngx + px)] = T2{w * w, v * v};
-        }
+        F[sxi<R>(px)] = T2{u * ((Uc + Uc) + u), u * (Wc + w) + Uc * w};
+        F[sxi<R>(ngx + px)] = T2{w * ((Wc + Wc) + w), v * v};
         if (a.want_cfl) {
           const double cv = fabs((double)u) * a.dxi + fabs((double)v) * dyi + fabs((double)w) * a.dzi;
           cmax = fmax(cmax, cv);
@@ -560,11 +555,312 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<R>& a, const Dims& d, 
   }
 }
 
+// FP64: the rows in 64-bit fixed point (lh_fxfft.cuh), two levels at a time.
+//
+// Three inverse lines of ngx: (u, w) of level j, (v of j, v of j + 1), (u, w) of j + 1, each two real rows in one complex
+// line.  They come out in 64-bit integers with one scale per line, are shifted to the full range by what their largest
+// value leaves (found by an OR over the magnitudes), interpolated and multiplied as integers, and the products go
+// forward two to a line: (uu, uw), (ww, vv), (uv, vw), each pair on the coarser of its two scales.  The FP64 the rows
+// come from and go to is the kernel's only floating point, but for the CFL number.
+//
+// Bound by instruction issue on the integer pipes (390 instructions a point of a transform, 53 % issue; transforms about
+// half of them), no longer by the FP64 pipe.  80 registers (three CTAs of 256 threads).  A step of the 576 x 576 x 450
+// grid: 140.0 -> 36.9 ms; 96 x 96 x 130 1.81 -> 0.46, 48 x 48 x 66 0.65 -> 0.11 ms.  Its memory traffic alone is 3 ms.
+//
+// Shared memory: two buffers of three lines that exchange their parts every two levels (the raw FP64 rows and the
+// products in one, the inverse lines in the other: while the last products are transformed, the next rows are copied in
+// where the inverse lines were), and u, w, v of the previous level.
+
+struct FxProd {                // per iteration, twice (an iteration clears the next one's)
+  unsigned e[3], sum[3], bits[6];
+};
+
+__device__ __forceinline__ void fx_reduce_max(unsigned m, unsigned* dst) {
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(dst, m);
+}
+__device__ __forceinline__ void fx_reduce_add(unsigned m, unsigned* dst) {
+  m = __reduce_add_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicAdd(dst, m);
+}
+__device__ __forceinline__ void fx_reduce_or(unsigned m, unsigned* dst) {
+  m = __reduce_or_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicOr(dst, m);
+}
+
+// Levels an iteration takes: two where the buffers of six lines fit (all lengths to 1936), else one.
+__host__ __device__ __forceinline__ int xprod_levels(int ngx) { return ngx <= 1936 ? 2 : 1; }
+// Levels of a CTA: whole iterations, so that every level's v has the same partner whatever the chunk.
+__host__ __device__ __forceinline__ int xprod_chunk(int chunk, int ngx) { return xprod_levels(ngx) == 2 ? (chunk + 1) & ~1 : chunk; }
+
+__device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims& d, const XPlan<double>& plan, int bx,
+                                           int by) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ FxProd red[2];
+  __shared__ double cflred[8];
+  const FxPlan& P = plan.pf;
+  const int n = d.ngx, nkx = d.nkx, tid = threadIdx.x, bd = blockDim.x;
+  const int lp = xprod_levels(n), nl = lp + 1;  // levels and lines of an iteration
+  fx2* B0 = reinterpret_cast<fx2*>(smraw);      // nl lines
+  fx2* B1 = B0 + nl * n;                        // nl lines
+  i64* pu = reinterpret_cast<i64*>(B1 + nl * n);  // u, w, v of the previous level
+  i64 *pw = pu + n, *pv = pw + n;
+  const int L0 = min(a.c_lo, a.f_lo + 1), L1 = max(a.c_hi, a.f_hi + 1);
+  const int chunk = xprod_chunk(a.chunk, n), c0 = L0 + by * chunk, c1 = min(c0 + chunk - 1, L1);
+  if (c0 > c1) return;
+  const size_t rowoff = (size_t)bx * nkx;
+  for (int i = tid; i < (int)(2 * sizeof(FxProd) / 4); i += bd) reinterpret_cast<unsigned*>(red)[i] = 0;
+
+  // Copies the FP64 rows of line 0 (u, w of level j), line 1 (v of jv, v of jv + 1) and, for two levels, line 2 (u, w of
+  // j + 1) into raw: row r of line l at raw[(2 l + r) nkx].  A row that does not exist is zero.
+  auto fetch = [&](fx2* raw, int j, bool two, int jv, int v_lo, int v_hi) {
+    const int rows = two ? 6 : 4;
+    for (int t = tid; t < rows * nkx; t += bd) {
+      const int q = t / nkx, k = t - q * nkx;
+      const double2* src = nullptr;
+      if (q == 2 || q == 3) {
+        const int f = jv + (q - 2);
+        if (f >= v_lo && f <= v_hi) src = a.mv + (size_t)f * d.mp;
+      } else {
+        const int f = q < 2 ? j : j + 1;
+        src = ((q & 1) ? a.mw : a.mu) + (size_t)f * d.mp;
+      }
+      if (src) fx_copy(raw + t, src + rowoff + k);
+      else raw[t] = fx2{0, 0};
+    }
+  };
+
+  // From the fetched rows to nv lines of integers, transformed, in Z.
+  auto inverse = [&](const fx2* raw, fx2* Z, int nv, FxProd& R, FxProd& next) {
+    const double2* rd = reinterpret_cast<const double2*>(raw);
+    fx_copy_wait();
+    __syncthreads();
+    unsigned m[3] = {0, 0, 0};
+    for (int t = tid; t < 2 * nv * nkx; t += bd) {
+      const unsigned h = fx_hi(rd[t]);
+      const int q = t / (2 * nkx);
+      m[0] = max(m[0], q == 0 ? h : 0u);
+      m[1] = max(m[1], q == 1 ? h : 0u);
+      m[2] = max(m[2], q == 2 ? h : 0u);
+    }
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+      if (v < nv) fx_reduce_max(m[v], &R.e[v]);
+    for (int i = tid; i < (int)(sizeof(FxProd) / 4); i += bd) reinterpret_cast<unsigned*>(&next)[i] = 0;
+    __syncthreads();
+    unsigned sum[3] = {0, 0, 0};
+    for (int v = 0; v < nv; ++v) {
+      const FxIn in((int)(R.e[v] >> 20) + 1);  // one bit of room: a line's values are sums of two rows'
+      const double2 *ra = rd + 2 * v * nkx, *rb = ra + nkx;
+      fx2* z = Z + v * n;
+      unsigned s = 0;
+      for (int k = tid; k < nkx; k += bd) {
+        const double2 A = ra[k], B = rb[k];
+        const i64 ax = in(A.x), ay = in(A.y), bx2 = in(B.x), by2 = in(B.y);
+        // a + i b at k, its mirror at n - k; the kx = 0 values are real.  Parts exchanged: an inverse transform
+        if (k == 0) {
+          z[P.pos_sample[0]] = fx2{bx2, ax};
+          s += fx_mag(ax) + fx_mag(bx2);
+        } else {
+          const fx2 p = fx2{ay + bx2, ax - by2}, q = fx2{bx2 - ay, ax + by2};
+          z[P.pos_sample[k]] = p;
+          z[P.pos_sample[n - k]] = q;
+          s += fx_mag(p.x) + fx_mag(p.y) + fx_mag(q.x) + fx_mag(q.y);
+        }
+      }
+      for (int k = nkx + tid; k <= n - nkx; k += bd) z[P.pos_sample[k]] = fx2{0, 0};
+      sum[0] += v == 0 ? s : 0u;
+      sum[1] += v == 1 ? s : 0u;
+      sum[2] += v == 2 ? s : 0u;
+    }
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+      if (v < nv) fx_reduce_add(sum[v], &R.sum[v]);
+    __syncthreads();
+    fx_fft(Z, nv, P, R.sum);
+    // magnitude bits of the real (u, v of the lower level) and the imaginary rows (w, v of the upper one)
+    for (int v = 0; v < nv; ++v) {
+      unsigned o0 = 0, o1 = 0;
+      for (int x = tid; x < n; x += bd) {
+        const fx2 z = Z[v * n + x];
+        o0 |= fx_bits(z.y);
+        o1 |= fx_bits(z.x);
+      }
+      fx_reduce_or(o0, &R.bits[2 * v]);
+      fx_reduce_or(o1, &R.bits[2 * v + 1]);
+    }
+    __syncthreads();
+  };
+  // scale of a line, and left shift and scale of its rows brought below 2^60
+  auto line_scale = [&](const FxProd& R, int v) {
+    return fx_scale((int)(R.e[v] >> 20) + 1) - fx_inv_shift(R.sum[v], P.shift);
+  };
+  auto room = [&](const FxProd& R, int row) { return __clz((int)R.bits[row]) - 4; };
+  auto lost = [&](const FxProd& R, int v) { return R.e[v] >= 0x7ff00000u; };
+
+  constexpr int kNone = 1 << 14;  // scale of a row of zeros: finer than any other
+  int Spu = kNone, Spw = kNone, Spv = kNone;  // scales of the previous level's rows
+  bool badp = false, badpv = false;
+  double cmax = 0.0;
+  int it = 0;
+  fx2 *raw = B0, *Z = B1;
+  const int v_top = d.nyv - 2;
+  const int j0 = c0 - 1;
+  if (j0 >= 1) {  // the previous level; its v in the pair it has in the chunk below
+    const bool paired = lp == 2 && j0 - 1 >= L0;
+    const int jv = paired ? j0 - 1 : j0;
+    fetch(raw, j0, false, jv, max(jv, 1), paired ? min(v_top, j0) : min(v_top, jv));
+    __syncthreads();  // red is cleared
+    inverse(raw, Z, 2, red[0], red[1]);
+    const FxProd& R = red[0];
+    const int su = room(R, 0), sw = room(R, 1), sv = room(R, paired ? 3 : 2);
+    for (int x = tid; x < n; x += bd) {
+      const fx2 z = Z[x], zv = Z[n + x];
+      pu[x] = fx_shift(z.y, su);
+      pw[x] = fx_shift(z.x, sw);
+      pv[x] = fx_shift(paired ? zv.x : zv.y, sv);
+    }
+    Spu = line_scale(R, 0) + su;
+    Spw = line_scale(R, 0) + sw;
+    Spv = line_scale(R, 1) + sv;
+    badp = lost(R, 0);
+    badpv = lost(R, 1);
+    it = 1;
+  } else {
+    for (int x = tid; x < 3 * n; x += bd) pu[x] = 0;
+  }
+  __syncthreads();
+  fetch(raw, c0, lp == 2 && c0 < c1, c0, 1, min(v_top, lp == 2 && c0 < c1 ? c0 + 1 : c0));
+  for (int j = c0; j <= c1; j += lp, ++it) {
+    const bool two = lp == 2 && j < c1;
+    FxProd& R = red[it & 1];
+    inverse(raw, Z, two ? 3 : 2, R, red[(it + 1) & 1]);
+    for (int q = 0; q < (two ? 2 : 1); ++q) {
+      const int jj = j + q;
+      const bool cprod = jj >= a.c_lo && jj <= a.c_hi;
+      const bool fprod = jj - 1 >= a.f_lo && jj - 1 <= a.f_hi;  // face jj-1 interior and in this launch
+      const bool vface = jj <= v_top;
+      const int vu = q == 0 ? 0 : 2;
+      const int su = room(R, 2 * vu), sw = room(R, 2 * vu + 1), sv = room(R, 2 + q);
+      const int Su = line_scale(R, vu) + su, Sw = line_scale(R, vu) + sw, Sv = vface ? line_scale(R, 1) + sv : kNone;
+      const bool bad = lost(R, vu), badv = lost(R, 1);
+      // v at the centre, u and w at the face below, each on the coarser scale of its two levels
+      const int4 wc = plan.wc[jj], wf = fprod ? plan.wf[jj - 1] : int4{0, 0, 0, 0};
+      const int Svc = min(Spv, Sv) - (wc.z ? wc.z + 1 : 0);
+      const int Suf = min(Spu, Su) - (wf.z ? wf.z + 1 : 0), Swf = min(Spw, Sw) - (wf.z ? wf.z + 1 : 0);
+      const int dvp = min(Spv - Svc, 63), dvc = min(Sv - Svc, 63), dup = min(Spu - Suf, 63), duc = min(Su - Suf, 63),
+                dwp = min(Spw - Swf, 63), dwc = min(Sw - Swf, 63);
+      // the products' scales and what brings each on its pair's
+      const int Suu = 2 * Su - 61, Suw = Su + Sw - 61, Sww = 2 * Sw - 61, Svv = 2 * Svc - 61;
+      const int Suv = Suf + Spv - 61, Svw = Swf + Spv - 61;
+      const int S0 = min(Suu, Suw), S1 = min(Sww, Svv), S2 = min(Suv, Svw);
+      const int d00 = min(Suu - S0, 63), d01 = min(Suw - S0, 63), d10 = min(Sww - S1, 63), d11 = min(Svv - S1, 63),
+                d20 = min(Suv - S2, 63), d21 = min(Svw - S2, 63);
+      fx2* F = raw;
+      int np = 0;                        // lines transformed forward at once
+      const int f0 = 0, f1 = cprod ? 2 : 0;
+      const bool split = nl < 3 && cprod && fprod;  // the face pair after the centre pairs
+      auto face = [&](int x, i64 u, i64 w, int slot) {
+        const i64 up = pu[x] >> dup, wp = pw[x] >> dwp, v = pv[x];
+        const i64 uf = up + fx_shl(fx_mul<1, 1>((u >> duc) - up, wf.x, wf.y), wf.z);
+        const i64 wv = wp + fx_shl(fx_mul<1, 1>((w >> dwc) - wp, wf.x, wf.y), wf.z);
+        F[slot * n + P.turn[x]] = fx2{fx_mulvar(uf, v) >> d20, fx_mulvar(wv, v) >> d21};
+      };
+      for (int x = tid; x < n; x += bd) {
+        const fx2 z = Z[vu * n + x], zv = Z[n + x];
+        const i64 u = fx_shift(z.y, su), w = fx_shift(z.x, sw);
+        const i64 v = vface ? fx_shift(q == 0 ? zv.y : zv.x, sv) : 0;
+        if (cprod) {
+          const i64 vp = pv[x] >> dvp;
+          const i64 vc = vp + fx_shl(fx_mul<1, 1>((v >> dvc) - vp, wc.x, wc.y), wc.z);
+          if (a.want_cfl) {
+            if (!bad && !badv && !badpv)
+              cmax = fmax(cmax, fabs(fx_to(u, Su)) * a.dxi + fabs(fx_to(vc, Svc)) * a.dyc[jj] + fabs(fx_to(w, Sw)) * a.dzi);
+          } else {
+            const int px = P.turn[x];
+            F[px] = fx2{fx_mulvar(u, u) >> d00, fx_mulvar(u, w) >> d01};
+            F[n + px] = fx2{fx_mulvar(w, w) >> d10, fx_mulvar(vc, vc) >> d11};
+          }
+        }
+        if (fprod && !split && !a.want_cfl) face(x, u, w, f1);
+        if (!split) {
+          pu[x] = u;
+          pw[x] = w;
+          pv[x] = v;
+        }
+      }
+      __syncthreads();
+      if (q == (two ? 1 : 0) && !split && j + lp <= c1) {  // the lines in Z are done with: the next rows take their place
+        const int jn = j + lp;
+        const bool tn = lp == 2 && jn < c1;
+        fetch(Z, jn, tn, jn, 1, min(v_top, tn ? jn + 1 : jn));
+      }
+      auto forward = [&](int lines, int first) {  // pairs first.. of this level
+        fx_fft(F, lines, P, nullptr);
+        for (int t = tid; t < lines * nkx; t += bd) {
+          const int p = t / nkx, k = t - p * nkx, pair = first + p;
+          const fx2 zk = F[p * n + P.pos_freq[k]], zc = F[p * n + P.pos_freq[k ? n - k : 0]];
+          const bool centre = cprod && pair < 2;
+          const int S = (centre ? (pair == 0 ? S0 : S1) : S2) - P.shift;
+          const bool nan = centre ? (bad || (pair == 1 && (badv || badpv))) : (bad || badp || badpv);
+          const FxOut out(nan ? 2047 : 0, S);
+          const size_t o = (size_t)(centre ? jj : jj - 1) * d.mp + rowoff + k;
+          const int r0 = centre ? 2 * pair : 4;
+          const i64 xk = zk.x >> 1, yk = zk.y >> 1, xc = zc.x >> 1, yc = zc.y >> 1;
+          double2 A = double2{out(xk + xc), out(yk - yc)}, B = double2{out(yk + yc), out(xc - xk)};
+          if (nan) A = B = double2{__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll)};
+          a.out[r0][o] = A;
+          a.out[r0 + 1][o] = B;
+        }
+        __syncthreads();
+      };
+      if (!a.want_cfl) {
+        np = (cprod ? 2 : 0) + (fprod && !split ? 1 : 0);
+        if (np) forward(np, f0);
+        if (split) {
+          for (int x = tid; x < n; x += bd) {
+            const fx2 z = Z[vu * n + x], zv = Z[n + x];
+            const i64 u = fx_shift(z.y, su), w = fx_shift(z.x, sw);
+            face(x, u, w, 0);
+            pu[x] = u;
+            pw[x] = w;
+            pv[x] = vface ? fx_shift(q == 0 ? zv.y : zv.x, sv) : 0;
+          }
+          __syncthreads();
+          forward(1, 2);
+        }
+      }
+      if (split && j + lp <= c1) {
+        const int jn = j + lp;
+        fetch(Z, jn, false, jn, 1, min(v_top, jn));
+      }
+      Spu = Su;
+      Spw = Sw;
+      Spv = Sv;
+      badp = bad;
+      badpv = badv;
+    }
+    fx2* t = raw;
+    raw = Z;
+    Z = t;
+  }
+  if (a.want_cfl) {
+    for (int o = 16; o > 0; o >>= 1) cmax = fmax(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+    if ((tid & 31) == 0) cflred[tid >> 5] = cmax;
+    __syncthreads();
+    if (tid == 0) {
+      double m = 0.0;
+      for (int w = 0; w < (bd >> 5); ++w) m = fmax(m, cflred[w]);
+      atomicMax(&a.sc->cflbits, (unsigned long long)__double_as_longlong(m));
+    }
+  }
+}
+
 template <typename R>
-__global__ void __launch_bounds__(256) k_xprod(const __grid_constant__ ProdArgs<R> a, const __grid_constant__ Dims d,
-                                               const __grid_constant__ FftPlan ph, const __grid_constant__ FftPlan pf,
-                                               const double2* __restrict__ rtw) {
-  xprod_body<R>(a, d, ph, pf, rtw, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 6 : 3) k_xprod(const __grid_constant__ ProdArgs<R> a,
+                                                                      const __grid_constant__ Dims d,
+                                                                      const __grid_constant__ XPlan<R> p) {
+  xprod_body(a, d, p, blockIdx.x, blockIdx.y);
 }
 
 // ---- the FP32 product pass on two z rows per CTA --------------------------------------------------------
@@ -782,9 +1078,16 @@ __device__ __forceinline__ void xprod2_body(const ProdArgs<float>& a, const Dims
 }
 
 __global__ void __launch_bounds__(256) k_xprod2(const __grid_constant__ ProdArgs<float> a,
-                                                const __grid_constant__ Dims d, const __grid_constant__ FftPlan ph,
-                                                const __grid_constant__ FftPlan pf, const double2* __restrict__ rtw) {
-  xprod2_body(a, d, ph, pf, rtw, blockIdx.x, blockIdx.y);
+                                                const __grid_constant__ Dims d, const __grid_constant__ XPlan<float> p) {
+  xprod2_body(a, d, p.ph, p.pf, p.rtw, blockIdx.x, blockIdx.y);
+}
+
+// Threads of a product-pass CTA: `threads` (128 or 256), and in FP64 no more than its three lines have radix-8
+// butterflies.
+template <typename R>
+int xprod_threads(const Dims& d, int threads) {
+  threads = threads == 128 ? 128 : 256;
+  return sizeof(R) == 4 ? threads : std::min(threads, (3 * d.ngx / 8 + 31) / 32 * 32);
 }
 
 template <typename R>
@@ -796,24 +1099,36 @@ void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem) 
     *smem = sizeof(float4) * sx_elems<float>(3 * (size_t)d.ngx) + sizeof(float2) * 6 * (size_t)d.ngx;
     return;
   }
-  *grid = nlev <= 0 ? dim3(0, 0, 0) : dim3(d.ngz, (nlev + a.chunk - 1) / a.chunk);
-  *smem = sizeof(cpx_t<R>) * sx_elems<R>((a.split ? 2 : 3) * (size_t)d.ngx) + sizeof(R) * 6 * (size_t)d.ngx;
+  const int chunk = sizeof(R) == 8 ? xprod_chunk(a.chunk, d.ngx) : a.chunk;
+  *grid = nlev <= 0 ? dim3(0, 0, 0) : dim3(d.ngz, (nlev + chunk - 1) / chunk);
+  if (sizeof(R) == 8) *smem = (2 * (xprod_levels(d.ngx) + 1) * sizeof(fx2) + 3 * sizeof(i64)) * (size_t)d.ngx;
+  else *smem = sizeof(cpx_t<R>) * sx_elems<R>((a.split ? 2 : 3) * (size_t)d.ngx) + sizeof(R) * 6 * (size_t)d.ngx;
+}
+
+int xprod_ctas_per_sm(const Dims& d) {
+  ProdArgs<double> a{};
+  a.chunk = 2;
+  dim3 grid;
+  size_t smem;
+  xprod_shape(a, d, &grid, &smem);
+  const int threads = xprod_threads<double>(d, 256);
+  const int by_regs = 65536 / (80 * threads), by_smem = (int)(233472 / (smem + 1024 + 256));
+  return std::max(1, std::min({32, 2048 / threads, by_regs, by_smem}));
 }
 
 template <typename R>
-void launch_xprod(const ProdArgs<R>& a, const Dims& d, const FftPlan& ph, const FftPlan& pf, const double2* rtw,
-                  cudaStream_t st) {
+void launch_xprod(const ProdArgs<R>& a, const Dims& d, const XPlan<R>& p, cudaStream_t st) {
   dim3 grid;
   size_t sm;
   xprod_shape(a, d, &grid, &sm);
   if (grid.x == 0) return;
   if constexpr (sizeof(R) == 4) {
     if (a.rows == 2) {
-      k_xprod2<<<grid, a.threads == 128 ? 128 : 256, sm, st>>>(a, d, ph, pf, rtw);
+      k_xprod2<<<grid, a.threads == 128 ? 128 : 256, sm, st>>>(a, d, p);
       return;
     }
   }
-  k_xprod<R><<<grid, a.threads == 128 ? 128 : 256, sm, st>>>(a, d, ph, pf, rtw);
+  k_xprod<R><<<grid, xprod_threads<R>(d, a.threads), sm, st>>>(a, d, p);
 }
 
 // Canopy forcing on one mixed row of one processed plane: x-inverse, solid
@@ -1679,11 +1994,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zfwd_batch(cons
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 6 : 5) k_xprod_batch(const __grid_constant__ Batch<XDesc<R>> b) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 6 : 3) k_xprod_batch(const __grid_constant__ Batch<XDesc<R>> b) {
   const int m = batch_member(b, blockIdx.x);
   const XDesc<R>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m];
-  xprod_body<R>(D.a, D.d, D.ph, D.pf, D.rtw, q % D.gx, q / D.gx);
+  xprod_body(D.a, D.d, D.p, q % D.gx, q / D.gx);
 }
 
 template <typename R>
@@ -1839,10 +2154,8 @@ template void launch_zinv<double>(const ZJobs<double>&, const Dims&, const ZPlan
 template void launch_zinv<float>(const ZJobs<float>&, const Dims&, const ZPlan<float>&, int, cudaStream_t, int);
 template void launch_zfwd<double>(const ZJobs<double>&, const Dims&, const ZPlan<double>&, int, double, cudaStream_t, int);
 template void launch_zfwd<float>(const ZJobs<float>&, const Dims&, const ZPlan<float>&, int, double, cudaStream_t, int);
-template void launch_xprod<double>(const ProdArgs<double>&, const Dims&, const FftPlan&, const FftPlan&, const double2*,
-                                   cudaStream_t);
-template void launch_xprod<float>(const ProdArgs<float>&, const Dims&, const FftPlan&, const FftPlan&, const double2*,
-                                  cudaStream_t);
+template void launch_xprod<double>(const ProdArgs<double>&, const Dims&, const XPlan<double>&, cudaStream_t);
+template void launch_xprod<float>(const ProdArgs<float>&, const Dims&, const XPlan<float>&, cudaStream_t);
 template void launch_xmask<double>(const MaskArgs<double>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
 template void launch_xmask<float>(const MaskArgs<float>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
 template void zpass_shape<double>(const ZJobs<double>&, const Dims&, int, dim3*, size_t*);

@@ -1,5 +1,5 @@
-"""The FP64 transforms in 64-bit fixed point: their error against extended precision on the CPU, and the step's z passes
-at the lengths where their passes differ, on the GPU."""
+"""The FP64 transforms in 64-bit fixed point: their error against extended precision on the CPU, and the step's
+passes at the lengths where they differ, on the GPU."""
 import ctypes as C
 import os
 import subprocess
@@ -7,7 +7,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from tests.helpers import SMOOTH, projected_ic, rel_l2
+from tests.helpers import SMALL, SMOOTH, projected_ic, rel_l2
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "littleharsh_gb300", "csrc")
@@ -98,12 +98,17 @@ def test_scale_of_a_line_does_not_matter(host, scale):
 Z_LENGTHS = [6, 8, 9, 16, 18, 27, 32, 54, 64, 81, 108, 128, 162]
 
 
+# x lengths (even): the same, and one beyond two levels per iteration of the product pass
+X_LENGTHS = [6, 8, 16, 18, 32, 54, 64, 128, 162, 486, 1944]
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("ngz", Z_LENGTHS)
-def test_z_lengths_against_the_oracle(oracle_mod, ngz):
-    """Right-hand sides and nonlinear term of the first substage, to the tolerance of the other substage comparisons."""
+@pytest.mark.parametrize("cfg", [dict(SMOOTH, ngalz=n) for n in Z_LENGTHS] + [dict(SMOOTH, ngalx=n, ngalz=12) for n in X_LENGTHS],
+                         ids=[f"z{n}" for n in Z_LENGTHS] + [f"x{n}" for n in X_LENGTHS])
+def test_lengths_against_the_oracle(oracle_mod, cfg):
+    """Right-hand sides and nonlinear term of the first substage, to the tolerance of the other substage comparisons, and
+    the CFL time step."""
     import littleharsh_gb300 as lh
-    cfg = dict(SMOOTH, ngalz=ngz)
     o = oracle_mod.Oracle(**cfg)
     f = projected_ic(o, seed=2)
     dt = o.cfl_dt(0.5)
@@ -116,3 +121,28 @@ def test_z_lengths_against_the_oracle(oracle_mod, ngz):
     s.substage(1, 1)
     for a, b in zip(s.get_nonlinear() + s.get_rhs(), list(o.get_nonlinear()) + list(o.get_rhs())):
         assert rel_l2(a, b) < 1e-11
+    assert abs(s.cfl_dt(0.5) - o.cfl_dt(0.5)) < 1e-12 * dt
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("banded", [False, True], ids=["one", "bands"])
+def test_chunks_of_levels_keep_results(monkeypatch, banded):
+    """Chunks of one, three and any number of levels start at whole pairs of levels: bit for bit the same step."""
+    import littleharsh_gb300 as lh
+    from littleharsh_gb300.initial import initial_field
+    cfg = dict(SMALL, ngalx2=18, ngalz2=18) if banded else SMALL
+    ref = None
+    for chunk in ("64", "1", "3", "6"):
+        monkeypatch.setenv("LH_CHUNK", chunk)
+        s = lh.Solver(lh.Config(**cfg))
+        g = s.grid
+        s.set_fields(*initial_field(g["yu"], g["yv"], s.nz, s.nkx, s.nyp, seed=9, kmax=4))
+        s.project()
+        s.set_time(0.0, 1e-3, 0.0)
+        s.step(2)
+        f = s.get_fields()
+        assert all(np.all(np.isfinite(x)) for x in f)
+        if ref is not None:
+            for a, b in zip(f, ref):
+                np.testing.assert_array_equal(a, b)
+        ref = f

@@ -856,10 +856,13 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
   }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 6 : 3) k_xprod(const __grid_constant__ ProdArgs<R> a,
-                                                                      const __grid_constant__ Dims d,
-                                                                      const __grid_constant__ XPlan<R> p) {
+__global__ void __launch_bounds__(256) k_xprod(const __grid_constant__ ProdArgs<float> a, const __grid_constant__ Dims d,
+                                               const __grid_constant__ XPlan<float> p) {
+  xprod_body(a, d, p, blockIdx.x, blockIdx.y);
+}
+
+__global__ void __launch_bounds__(256, 3) k_xprod_fx(const __grid_constant__ ProdArgs<double> a, const __grid_constant__ Dims d,
+                                                     const __grid_constant__ XPlan<double> p) {
   xprod_body(a, d, p, blockIdx.x, blockIdx.y);
 }
 
@@ -1128,7 +1131,8 @@ void launch_xprod(const ProdArgs<R>& a, const Dims& d, const XPlan<R>& p, cudaSt
       return;
     }
   }
-  k_xprod<R><<<grid, xprod_threads<R>(d, a.threads), sm, st>>>(a, d, p);
+  if constexpr (sizeof(R) == 4) k_xprod<<<grid, xprod_threads<R>(d, a.threads), sm, st>>>(a, d, p);
+  else k_xprod_fx<<<grid, xprod_threads<R>(d, a.threads), sm, st>>>(a, d, p);
 }
 
 // Canopy forcing on one mixed row of one processed plane: x-inverse, solid
@@ -2138,7 +2142,7 @@ cudaError_t configure_kernels() {
   if (e != cudaSuccess) return e;
   const cudaError_t r[18] = {allow_smem(k_xcond, optin), allow_smem(k_zinv<double>, optin), allow_smem(k_zinv<float>, optin),
                              allow_smem(k_zfwd<double>, optin), allow_smem(k_zfwd<float>, optin),
-                             allow_smem(k_xprod<double>, optin), allow_smem(k_xprod<float>, optin), allow_smem(k_xprod2, optin),
+                             allow_smem(k_xprod_fx, optin), allow_smem(k_xprod, optin), allow_smem(k_xprod2, optin),
                              allow_smem(k_xmask<double>, optin), allow_smem(k_xmask<float>, optin),
                              allow_smem(k_zinv_batch<double>, optin), allow_smem(k_zinv_batch<float>, optin),
                              allow_smem(k_zfwd_batch<double>, optin), allow_smem(k_zfwd_batch<float>, optin),

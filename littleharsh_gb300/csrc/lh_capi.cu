@@ -233,25 +233,35 @@ int build_fx(lh_handle* h, FxPlan* P, int n) {
   return LH_OK;
 }
 
-// Levels per CTA of the FP64 product pass: the chunk with the least estimated time, (CTAs / CTAs resident at once, at least one wave)
-// x (levels + 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (FP64 product pass,
-// chunks of 2 / 4 / 8 / 16 levels: 48 x 48 x 66 0.11 / 0.15 / 0.25 / 0.45 ms a step, 96 x 96 x 130 0.51 / 0.46 / 0.46 /
-// 0.58, 162 x 108 x 124 0.96 / 0.82 / 0.76 / 0.95); on large ones long chunks save the repeated level (576 x 576 x 450,
-// 8 / 16 / 32 / 64: 38.6 / 37.3 / 36.9 / 37.3).  The mixed form keeps 16 or 32 (with this rule 96 x 96 x 130 takes 1 %
-// longer).
-int default_chunk(const lh_handle* h) {
+// The product pass's default launch shape.
+//
+// Mixed form: two z rows per CTA where Ngalz is even, with 128 threads while a stage of its three transforms has at most
+// 256 butterflies (3/4 Ngalx; with 256 threads most would idle), else 256.  Against one row and 256 threads, ms a step:
+// 96 x 96 x 130 0.42 -> 0.21, 288 x 288 x 226 3.08 -> 1.91, 576 x 576 x 450 17.4 -> 15.2 (128 threads there 15.9).
+//
+// Levels per CTA: the chunk with the least estimated time, (CTAs / CTAs resident at once, at least one wave) x (levels +
+// 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (FP64, chunks of 2 / 4 / 8 / 16
+// levels: 48 x 48 x 66 0.11 / 0.15 / 0.25 / 0.45 ms a step, 96 x 96 x 130 0.51 / 0.46 / 0.46 / 0.58, 162 x 108 x 124
+// 0.96 / 0.82 / 0.76 / 0.95; mixed, two rows: 48 x 48 x 66 0.07 / 0.10, 96 x 96 x 130 0.20 / 0.22 / 0.23); on large ones
+// long chunks save the repeated level (576 x 576 x 450, 8 / 16 / 32 / 64: 38.6 / 37.3 / 36.9 / 37.3, mixed 15.2 / 15.1 /
+// 15.2 / -).
+void default_xprod_shape(lh_handle* h) {
   const Dims& d = h->d;
+  const bool mixed = h->precision == LH_PREC_MIXED;
+  if (mixed && d.ngz % 2 == 0) {
+    h->xrows = 2;
+    h->xthreads = 3 * d.ngx / 4 <= 256 ? 128 : 256;
+  }
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-  const double resident = (double)sms * xprod_ctas_per_sm(d);
-  int best = 2;
+  const double resident = (double)sms * (mixed ? xprod_ctas_per_sm<float>(d, h->xrows, h->xthreads)
+                                               : xprod_ctas_per_sm<double>(d, 1, h->xthreads));
   double least = 1e300;
   for (int c : {2, 4, 8, 16, 32}) {
-    const double ctas = (double)d.ngz * ((d.nyu - 2 + c - 1) / c);
+    const double ctas = (double)(d.ngz / h->xrows) * ((d.nyu - 2 + c - 1) / c);
     const double t = std::max(1.0, ctas / resident) * (c + 1.3);
-    if (t < least) { least = t; best = c; }
+    if (t < least) { least = t; h->chunk = c; }
   }
-  return best;
 }
 
 size_t field_elems(const lh_handle* h, char grid) {
@@ -1024,7 +1034,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
   // z tile width: narrow tiles keep several CTAs per SM so that one CTA's loads overlap another's
   // butterflies (measured on configuration 2: FP64 best at 4, mixed at 8)
   h->tx = h->precision == LH_PREC_MIXED ? 8 : 4;
-  h->chunk = h->precision == LH_PREC_MIXED ? (d.nyu > 256 ? 32 : 16) : default_chunk(h);
+  default_xprod_shape(h);
   // launch-shape overrides for tuning sweeps: LH_TX (z tile width, 1..64), LH_CHUNK (levels per x-pass CTA)
   if (const char* v = std::getenv("LH_TX")) { const int x = std::atoi(v); if (x >= 1 && x <= 64) h->tx = x; }
   if (const char* v = std::getenv("LH_CHUNK")) { const int x = std::atoi(v); if (x >= 1 && x <= 4096) h->chunk = x; }

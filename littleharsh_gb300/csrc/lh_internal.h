@@ -341,8 +341,10 @@ template <typename R>
 void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem);
 template <typename R>
 int zpass_tile(int tx);
-// FP64 product-pass CTAs (of up to 256 threads) resident on an SM, from their threads, registers and shared memory.
-int xprod_ctas_per_sm(const Dims& d);
+// Product-pass CTAs of `rows` z rows and at most `threads` threads resident on an SM, from their threads, registers and
+// shared memory.
+template <typename R>
+int xprod_ctas_per_sm(const Dims& d, int rows, int threads);
 template <typename R>
 void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem);
 template <typename R>

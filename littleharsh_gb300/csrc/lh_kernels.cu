@@ -1108,14 +1108,17 @@ void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem) 
   else *smem = sizeof(cpx_t<R>) * sx_elems<R>((a.split ? 2 : 3) * (size_t)d.ngx) + sizeof(R) * 6 * (size_t)d.ngx;
 }
 
-int xprod_ctas_per_sm(const Dims& d) {
-  ProdArgs<double> a{};
+template <typename R>
+int xprod_ctas_per_sm(const Dims& d, int rows, int threads) {
+  ProdArgs<R> a{};
   a.chunk = 2;
+  a.rows = rows;
   dim3 grid;
   size_t smem;
   xprod_shape(a, d, &grid, &smem);
-  const int threads = xprod_threads<double>(d, 256);
-  const int by_regs = 65536 / (80 * threads), by_smem = (int)(233472 / (smem + 1024 + 256));
+  threads = xprod_threads<R>(d, threads);
+  const int regs = sizeof(R) == 8 ? 80 : (rows == 2 ? 48 : 40);  // registers a thread of the three kernels
+  const int by_regs = 65536 / (regs * threads), by_smem = (int)(233472 / (smem + 1024 + 256));
   return std::max(1, std::min({32, 2048 / threads, by_regs, by_smem}));
 }
 
@@ -2165,6 +2168,8 @@ template void launch_xmask<float>(const MaskArgs<float>&, const Dims&, const Fft
 template void zpass_shape<double>(const ZJobs<double>&, const Dims&, int, dim3*, size_t*);
 template int zpass_tile<double>(int);
 template int zpass_tile<float>(int);
+template int xprod_ctas_per_sm<double>(const Dims&, int, int);
+template int xprod_ctas_per_sm<float>(const Dims&, int, int);
 template void zpass_shape<float>(const ZJobs<float>&, const Dims&, int, dim3*, size_t*);
 template void xprod_shape<double>(const ProdArgs<double>&, const Dims&, dim3*, size_t*);
 template void xprod_shape<float>(const ProdArgs<float>&, const Dims&, dim3*, size_t*);

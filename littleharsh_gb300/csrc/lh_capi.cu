@@ -1424,11 +1424,12 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
       std::vector<FDesc> fd;
       std::vector<PDesc> pd;
       std::vector<int> bv, bfl, bp;
+      std::vector<size_t> sv, sp;
       for (lh_handle* h : hs) {
         VDesc V{};
         V.r1 = h->r1; V.r2 = h->r2; V.r3 = h->r3; V.u1 = h->u1; V.u2 = h->u2; V.u3 = h->u3;
-        V.d = h->d; V.t = h->t; V.k = k; V.gx = (h->d.np + 127) / 128; V.gy = 3;
-        vd.push_back(V); bv.push_back(V.gx * V.gy);
+        V.d = h->d; V.t = h->t; V.k = k; V.gx = vsolve_ctas(h->d); V.gy = 3;
+        vd.push_back(V); bv.push_back(V.gx * V.gy); sv.push_back(vsolve_smem(h->d));
         if (h->prm.flag_ctpress == 0) {
           FDesc F{};
           F.u1 = h->u1; F.sc = h->sc; F.d = h->d; F.t = h->t; F.k = k; F.Qx1 = h->Qx1[k];
@@ -1437,12 +1438,12 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
         PDesc P{};
         P.u1 = h->u1; P.u2 = h->u2; P.u3 = h->u3; P.p = h->p; P.psi = h->psi; P.d = h->d; P.t = h->t;
         psolve_scalars(h, k, &P.dtirk, &P.dtrk);
-        P.gwb = h->gw[0][0]; P.gwt = h->gw[2][1]; P.sc = h->sc; P.gx = (h->d.np + 127) / 128;
-        pd.push_back(P); bp.push_back(P.gx);
+        P.gwb = h->gw[0][0]; P.gwt = h->gw[2][1]; P.sc = h->sc; P.gx = psolve_ctas(h->d);
+        pd.push_back(P); bp.push_back(P.gx); sp.push_back(psolve_smem(h->d));
       }
-      add_slot(slots, K_VSOLVE, vd, bv, std::vector<size_t>(vd.size(), 0));
+      add_slot(slots, K_VSOLVE, vd, bv, sv);
       add_slot(slots, K_FLOWRATE, fd, bfl, std::vector<size_t>(fd.size(), 0));
-      add_slot(slots, K_PSOLVE, pd, bp, std::vector<size_t>(pd.size(), 0));
+      add_slot(slots, K_PSOLVE, pd, bp, sp);
     }
   }
 }
@@ -1456,9 +1457,9 @@ void launch_slot(const Slot& sl, cudaStream_t st) {
     case K_XPROD: launch_xprod_batch<R>(*(const Batch<XDesc<R>>*)p, sl.smem, st); break;
     case K_IB_XMASK: launch_xmask_batch<R>(*(const Batch<MDesc<R>>*)p, sl.smem, st); break;
     case K_ASSEMBLE: launch_assemble_batch(*(const Batch<ADesc>*)p, sizeof(R) == 4, st); break;
-    case K_VSOLVE: launch_vsolve_batch(*(const Batch<VDesc>*)p, st); break;
+    case K_VSOLVE: launch_vsolve_batch(*(const Batch<VDesc>*)p, sl.smem, st); break;
     case K_FLOWRATE: launch_flowrate_batch(*(const Batch<FDesc>*)p, st); break;
-    default: launch_psolve_batch(*(const Batch<PDesc>*)p, st); break;
+    default: launch_psolve_batch(*(const Batch<PDesc>*)p, sl.smem, st); break;
   }
 }
 

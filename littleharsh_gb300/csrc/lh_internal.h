@@ -224,6 +224,11 @@ void launch_build_dg(double* dg2, double* dg3, const double* rows, const Dims& d
 void launch_psolve(double2* u1, double2* u2, double2* u3, double2* p, double2* psi, const Dims& d,
                    const Tables& t, double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc,
                    cudaStream_t st);
+// CTAs of a velocity (per component) or pressure solve, and their dynamic shared memory
+int vsolve_ctas(const Dims& d);
+int psolve_ctas(const Dims& d);
+size_t vsolve_smem(const Dims& d);
+size_t psolve_smem(const Dims& d);
 void launch_divergence(const double2* u1, const double2* u2, const double2* u3, double2* div, const Dims& d,
                        const Tables& t, cudaStream_t st);
 void launch_absmax(const double2* x, size_t n, DevScalars* sc, cudaStream_t st);
@@ -332,9 +337,9 @@ void launch_xprod_batch(const Batch<XDesc<R>>& b, size_t smem, cudaStream_t st);
 template <typename R>
 void launch_xmask_batch(const Batch<MDesc<R>>& b, size_t smem, cudaStream_t st);
 void launch_assemble_batch(const Batch<ADesc>& b, bool fp32_products, cudaStream_t st);
-void launch_vsolve_batch(const Batch<VDesc>& b, cudaStream_t st);
+void launch_vsolve_batch(const Batch<VDesc>& b, size_t smem, cudaStream_t st);
 void launch_flowrate_batch(const Batch<FDesc>& b, cudaStream_t st);
-void launch_psolve_batch(const Batch<PDesc>& b, cudaStream_t st);
+void launch_psolve_batch(const Batch<PDesc>& b, size_t smem, cudaStream_t st);
 // Grid and dynamic shared memory of the single launches (what the batched ones reproduce per member; a zero
 // grid means no launch).
 template <typename R>

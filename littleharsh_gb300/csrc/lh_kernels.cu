@@ -1341,98 +1341,202 @@ void launch_assemble(const AsmArgs& a, const Dims& d, const Tables& t, cudaStrea
   else k_assemble<double2><<<grid, 256, 0, st>>>(a, d, t);
 }
 
-// Thomas sweeps of one column over levels lo..hi with an LU indexed by level
-// (LUsolU/LUsolV, tridLU_3D_IB.f90:106-116,179-189); levels are prefetched
-// four at a time.
-__device__ __forceinline__ void thomas_column(double2* __restrict__ R, double2* __restrict__ U, size_t np, int col,
+// The column solves take two threads per column, one for the real parts and one for the imaginary ones (neighbouring
+// lanes: the accesses stay as coalesced as with one thread and 16 bytes).  A sweep is a chain of FP64 instructions, and a
+// warp's FP64 instruction takes 64 clocks of its quarter of the SM whatever else runs there.  Two forms:
+//  * many columns: each thread walks its levels, the loads of the next ones issued ahead; every quarter has several warps
+//    and the FP64 pipe or memory is the bound;
+//  * few columns: a CTA keeps 16 columns' values of all levels in shared memory.  Its warps form right-hand sides and
+//    corrections for different levels at once, and only the recurrences, two FP64 instructions a level up and one down,
+//    are left to one warp.
+// Both do the arithmetic of one thread walking a column, operation by operation.
+constexpr int kColThreads = 128;
+constexpr int kColBatch = 2;     // levels whose loads are in flight together (twice that with the batch ahead)
+constexpr int kTileThreads = 256;
+constexpr int kTileParts = 32;   // parts (half columns) of a tile
+constexpr int kTileBatch = 8;    // levels whose loads a warp of a tile has in flight
+
+// Whether a grid's solves keep tiles of columns in shared memory: while its tiles are about as many as the chip holds at
+// once (two CTAs an SM in the pressure solve, five of the three components' CTAs in the velocity solve).  Beyond that
+// the tiles queue, and a thread per part has parallelism enough.  Three launches, ms, tiles against threads:
+// pressure 48 x 48 x 66 (34 tiles) 0.08 / 0.16, 96 x 96 x 130 (132) 0.15 / 0.32, 144 x 144 x 154 (294) 0.24 / 0.37,
+// 192 x 192 x 226 (520) 0.65 / 0.60; velocity 0.05 / 0.07, 0.08 / 0.13, 0.18 / 0.17, 0.45 / 0.32.
+__host__ __device__ __forceinline__ bool column_fits(const Dims& d) { return d.nyu <= 400; }  // 205 KB
+__host__ __device__ __forceinline__ bool psolve_tiled(const Dims& d) { return column_fits(d) && d.np <= 16 * 304; }
+__host__ __device__ __forceinline__ bool vsolve_tiled(const Dims& d) { return column_fits(d) && 3 * d.np <= 16 * 760; }
+static int column_ctas(const Dims& d, bool tiled) {
+  return tiled ? (2 * d.np + kTileParts - 1) / kTileParts : (2 * d.np + kColThreads - 1) / kColThreads;
+}
+int vsolve_ctas(const Dims& d) { return column_ctas(d, vsolve_tiled(d)); }
+int psolve_ctas(const Dims& d) { return column_ctas(d, psolve_tiled(d)); }
+size_t vsolve_smem(const Dims& d) { return vsolve_tiled(d) ? sizeof(double) * (size_t)d.nyu * (kTileParts + 6) : 0; }
+size_t psolve_smem(const Dims& d) { return sizeof(double) * (psolve_tiled(d) ? (size_t)d.nyp * (2 * kTileParts + 1) : (size_t)d.nyv); }
+
+// Thomas sweeps of one column's real or imaginary part over levels lo..hi with an LU indexed by level
+// (LUsolU/LUsolV, tridLU_3D_IB.f90:106-116,179-189): R, U at the part's value of level 0, levels np2 apart.
+__device__ __forceinline__ void thomas_column(double* __restrict__ R, double* __restrict__ U, size_t np2,
                                               const double* __restrict__ a1, const double* __restrict__ a2,
                                               const double* __restrict__ a3, int lo, int hi) {
-  double2 x = R[(size_t)lo * np + col];
-  x = double2{x.x * a2[lo], x.y * a2[lo]};
-  R[(size_t)lo * np + col] = x;
-  int jj = lo + 1;
-  for (; jj + 3 <= hi; jj += 4) {
-    double2 v[4];
+  constexpr int NB = 2 * kColBatch;
+  double v[NB], w[NB];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = R[(size_t)(jj + q) * np + col];
+  for (int q = 0; q < NB; ++q) v[q] = R[(size_t)min(lo + q, hi) * np2];
+  double x = 0.0;
+  for (int j = lo; j <= hi; j += NB) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const double b1 = a1[jj + q], b2 = a2[jj + q];
-      x = double2{(v[q].x - b1 * x.x) * b2, (v[q].y - b1 * x.y) * b2};
-      R[(size_t)(jj + q) * np + col] = x;
+    for (int q = 0; q < NB; ++q) w[q] = R[(size_t)min(j + NB + q, hi) * np2];  // the next levels
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      if (j + q > hi) break;
+      x = j + q == lo ? v[q] * a2[lo] : (v[q] - a1[j + q] * x) * a2[j + q];
+      R[(size_t)(j + q) * np2] = x;
     }
-  }
-  for (; jj <= hi; ++jj) {
-    const double2 v = R[(size_t)jj * np + col];
-    x = double2{(v.x - a1[jj] * x.x) * a2[jj], (v.y - a1[jj] * x.y) * a2[jj]};
-    R[(size_t)jj * np + col] = x;
-  }
-  U[(size_t)hi * np + col] = x;
-  jj = hi - 1;
-  for (; jj - 3 >= lo; jj -= 4) {
-    double2 v[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = R[(size_t)(jj - q) * np + col];
+    for (int q = 0; q < NB; ++q) v[q] = w[q];
+  }
+  U[(size_t)hi * np2] = x;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const double b3 = a3[jj - q];
-      x = double2{v[q].x - b3 * x.x, v[q].y - b3 * x.y};
-      U[(size_t)(jj - q) * np + col] = x;
+  for (int q = 0; q < NB; ++q) v[q] = R[(size_t)max(hi - 1 - q, lo) * np2];
+  for (int j = hi - 1; j >= lo; j -= NB) {
+#pragma unroll
+    for (int q = 0; q < NB; ++q) w[q] = R[(size_t)max(j - NB - q, lo) * np2];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      if (j - q < lo) break;
+      x = v[q] - a3[j - q] * x;
+      U[(size_t)(j - q) * np2] = x;
     }
-  }
-  for (; jj >= lo; --jj) {
-    const double2 v = R[(size_t)jj * np + col];
-    x = double2{v.x - a3[jj] * x.x, v.y - a3[jj] * x.y};
-    U[(size_t)jj * np + col] = x;
+#pragma unroll
+    for (int q = 0; q < NB; ++q) v[q] = w[q];
   }
 }
 
-// Velocity solves: one thread per (component, column).  Long columns use the
+// The Thomas sweeps of a tile of columns.  A level's coefficients are those of the column's segment; zeros on the levels
+// between a short column's wall bands and below a segment's first level let the segments fall apart by themselves.
+__device__ __forceinline__ void vsolve_tile(const double* __restrict__ R, double* __restrict__ U, const Dims& d, const Tables& t,
+                                            int k, int comp, int bx) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int ny = comp == 1 ? d.nyv : d.nyu, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  double* X = reinterpret_cast<double*>(smraw);  // [ny][32]
+  double* M = X + (size_t)ny * kTileParts;       // a1, a2, a3 per level: long columns, then short ones
+  const int part = bx * kTileParts + lane, col = part >> 1;
+  const bool in = col < d.np;
+  const bool lng = !in || is_long(d, col % d.nkx, col / d.nkx);
+  const size_t np2 = 2 * (size_t)d.np;
+  const int e1 = comp == 1 ? d.Nv1 + 1 : d.Nu1 + 1, s3 = comp == 1 ? d.Nv2 : d.Nu2;
+  const double* ll = (comp == 1 ? t.lu_v : t.lu_u) + (size_t)k * 3 * ny;
+  const double* l1 = (comp == 1 ? t.lu_v1 : t.lu_u1) + (size_t)k * 3 * ny;
+  const double* l3 = (comp == 1 ? t.lu_v3 : t.lu_u3) + (size_t)k * 3 * ny;
+  for (int j = threadIdx.x; j < ny; j += blockDim.x) {
+    M[j] = j == 0 ? 0.0 : ll[j];
+    M[ny + j] = ll[ny + j];
+    M[2 * ny + j] = j == ny - 1 ? 0.0 : ll[2 * ny + j];
+    if (d.banded) {
+      const double* l = j <= e1 ? l1 : l3;
+      const bool mid = j > e1 && j < s3;
+      M[3 * ny + j] = mid || j == 0 || j == s3 ? 0.0 : l[j];
+      M[4 * ny + j] = mid ? 0.0 : l[ny + j];
+      M[5 * ny + j] = mid || j == e1 || j == ny - 1 ? 0.0 : l[2 * ny + j];
+    }
+  }
+  if (in) {
+    for (int j0 = warp; j0 < ny; j0 += kTileBatch * warps) {
+      double r[kTileBatch];
+#pragma unroll
+      for (int q = 0; q < kTileBatch; ++q) r[q] = R[(size_t)min(j0 + q * warps, ny - 1) * np2 + part];
+#pragma unroll
+      for (int q = 0; q < kTileBatch; ++q)
+        if (j0 + q * warps < ny) X[(j0 + q * warps) * kTileParts + lane] = r[q];
+    }
+  }
+  __syncthreads();
+  if (warp == 0 && in) {
+    const double *a1 = lng ? M : M + 3 * ny, *a2 = a1 + ny, *a3 = a2 + ny;
+    double *c = X + lane, x = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < ny; ++j) {
+      x = (c[j * kTileParts] - a1[j] * x) * a2[j];
+      c[j * kTileParts] = x;
+    }
+#pragma unroll 8
+    for (int j = ny - 2; j >= 0; --j) {
+      x = c[j * kTileParts] - a3[j] * x;
+      c[j * kTileParts] = x;
+    }
+  }
+  __syncthreads();
+  if (in) {
+#pragma unroll 4
+    for (int j = warp; j < ny; j += warps) U[(size_t)j * np2 + part] = X[j * kTileParts + lane];
+  }
+}
+
+// Velocity solves: two threads per (component, column).  Long columns use the
 // LU of the whole channel; short columns solve their two wall bands with those
 // bands' LUs and are zero in between.
 __device__ __forceinline__ void vsolve_body(double2* r1, double2* r2, double2* r3, double2* u1, double2* u2, double2* u3,
                                             const Dims& d, const Tables& t, int k, int bx, int by) {
-  const int col = bx * blockDim.x + threadIdx.x;
+  if (vsolve_tiled(d)) {
+    vsolve_tile(reinterpret_cast<double*>(by == 0 ? r1 : (by == 1 ? r2 : r3)),
+                reinterpret_cast<double*>(by == 0 ? u1 : (by == 1 ? u2 : u3)), d, t, k, by, bx);
+    return;
+  }
+  const int part = bx * blockDim.x + threadIdx.x, col = part >> 1;
   if (col >= d.np) return;
   const int comp = by;
   const int ny = comp == 1 ? d.nyv : d.nyu;
-  double2* R = comp == 0 ? r1 : (comp == 1 ? r2 : r3);
-  double2* U = comp == 0 ? u1 : (comp == 1 ? u2 : u3);
-  const size_t np = d.np;
+  double* R = reinterpret_cast<double*>(comp == 0 ? r1 : (comp == 1 ? r2 : r3)) + part;
+  double* U = reinterpret_cast<double*>(comp == 0 ? u1 : (comp == 1 ? u2 : u3)) + part;
+  const size_t np2 = 2 * (size_t)d.np;
   const int i = col % d.nkx, kk = col / d.nkx;
   if (is_long(d, i, kk)) {
     const double* lu = comp == 1 ? t.lu_v + (size_t)k * 3 * d.nyv : t.lu_u + (size_t)k * 3 * d.nyu;
-    thomas_column(R, U, np, col, lu, lu + ny, lu + 2 * ny, 0, ny - 1);
+    thomas_column(R, U, np2, lu, lu + ny, lu + 2 * ny, 0, ny - 1);
     return;
   }
   const double* l1 = (comp == 1 ? t.lu_v1 : t.lu_u1) + (size_t)k * 3 * ny;
   const double* l3 = (comp == 1 ? t.lu_v3 : t.lu_u3) + (size_t)k * 3 * ny;
   const int e1 = comp == 1 ? d.Nv1 + 1 : d.Nu1 + 1, s3 = comp == 1 ? d.Nv2 : d.Nu2;
-  thomas_column(R, U, np, col, l1, l1 + ny, l1 + 2 * ny, 0, e1);
-  thomas_column(R, U, np, col, l3, l3 + ny, l3 + 2 * ny, s3, ny - 1);
-  for (int jj = e1 + 1; jj < s3; ++jj) U[(size_t)jj * np + col] = double2{0.0, 0.0};
+  thomas_column(R, U, np2, l1, l1 + ny, l1 + 2 * ny, 0, e1);
+  thomas_column(R, U, np2, l3, l3 + ny, l3 + 2 * ny, s3, ny - 1);
+  for (int jj = e1 + 1; jj < s3; ++jj) U[(size_t)jj * np2] = 0.0;
 }
 
-__global__ void __launch_bounds__(128) k_vsolve(double2* r1, double2* r2, double2* r3, double2* u1, double2* u2,
-                                                double2* u3, const __grid_constant__ Dims d,
-                                                const __grid_constant__ Tables t, int k) {
+__global__ void __launch_bounds__(kTileThreads) k_vsolve(double2* r1, double2* r2, double2* r3, double2* u1, double2* u2,
+                                                        double2* u3, const __grid_constant__ Dims d,
+                                                        const __grid_constant__ Tables t, int k) {
   vsolve_body(r1, r2, r3, u1, u2, u3, d, t, k, blockIdx.x, blockIdx.y);
 }
 
 void launch_vsolve(double2* r1, double2* r2, double2* r3, double2* u1, double2* u2, double2* u3, const Dims& d,
                    const Tables& t, int k, cudaStream_t st) {
-  dim3 grid((d.np + 127) / 128, 3);
-  k_vsolve<<<grid, 128, 0, st>>>(r1, r2, r3, u1, u2, u3, d, t, k);
+  k_vsolve<<<dim3(vsolve_ctas(d), 3), vsolve_tiled(d) ? kTileThreads : kColThreads, vsolve_smem(d), st>>>(r1, r2, r3, u1, u2, u3, d, t, k);
 }
 
-// flowrate_corr on mode (0,0): the flow-rate sum runs in the reference's
-// order on one thread; the correction is spread over the block.
+// flowrate_corr on mode (0,0) (one CTA of kFlowThreads): the levels are read by all threads, the flow-rate sum then runs
+// in the reference's order on one (its rounding is what the pressure gradient's last digits come from), and the
+// correction is spread over the threads again.  12 -> 8 us a launch at 130 levels, 60 -> 20 us at 450.
+constexpr int kFlowThreads = 256;
 __device__ __forceinline__ void flowrate_body(double2* u1, DevScalars* sc, const Dims& d, const Tables& t, int k,
                                               double Qx1) {
+  __shared__ double w[kFlowThreads], v[kFlowThreads];
   __shared__ double gsh;
+  double Q = 0.0;
+  for (int j0 = 1; j0 <= d.nn + 1; j0 += kFlowThreads) {
+    const int j = j0 + threadIdx.x;
+    if (j <= d.nn + 1) {
+      w[threadIdx.x] = t.dyvw[j];
+      v[threadIdx.x] = u1[(size_t)(j - d.ju0) * d.np].x;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int n = min(kFlowThreads, d.nn + 2 - j0);
+#pragma unroll 8
+      for (int q = 0; q < n; ++q) Q = Q + w[q] * v[q];
+    }
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
-    double Q = 0.0;
-    for (int j = 1; j <= d.nn + 1; ++j) Q = Q + t.dyvw[j] * u1[(size_t)(j - d.ju0) * d.np].x;
     const double g = (sc->QxT - Q) / Qx1;
     sc->Qx = Q;
     sc->mpgx = sc->mpgx + g;
@@ -1441,7 +1545,7 @@ __device__ __forceinline__ void flowrate_body(double2* u1, DevScalars* sc, const
   __syncthreads();
   const double g = gsh;
   const double* u11 = t.u11 + (size_t)k * (d.nn + 3);
-  for (int j = threadIdx.x; j <= d.nn + 2; j += blockDim.x) {
+  for (int j = threadIdx.x; j <= d.nn + 2; j += kFlowThreads) {
     double2* u = u1 + (size_t)(j - d.ju0) * d.np;
     u->x = u->x + g * u11[j];
   }
@@ -1453,7 +1557,7 @@ __global__ void k_flowrate(double2* u1, DevScalars* sc, const __grid_constant__ 
 }
 
 void launch_flowrate(double2* u1, DevScalars* sc, const Dims& d, const Tables& t, int k, double Qx1, cudaStream_t st) {
-  k_flowrate<<<1, 256, 0, st>>>(u1, sc, d, t, k, Qx1);
+  k_flowrate<<<1, kFlowThreads, 0, st>>>(u1, sc, d, t, k, Qx1);
 }
 
 // LU_buildP + LU_decP (tridLU_3D_IB.f90:497-571,643-684), one thread per
@@ -1500,144 +1604,316 @@ void launch_build_dg(double* dg2, double* dg3, const double* rows, const Dims& d
   k_build_dg<<<(d.np + 127) / 128, 128, 0, st>>>(dg2, dg3, rows, d, t, pin);
 }
 
-// solveP + v_corr over the p levels lo..hi of one column (a long column's all,
-// or one wall band of a short one).  The divergence is formed on the fly in
-// the forward sweep; the backward sweep adds psi to p and corrects u, w on the
-// same levels and v on the faces between them.
 // bit pattern test for a NaN or an infinity (integer work only, off the FP64 pipe)
 __device__ __forceinline__ bool nonfinite(double x) {
   return ((unsigned long long)__double_as_longlong(x) & 0x7ff0000000000000ull) == 0x7ff0000000000000ull;
 }
 
-__device__ __forceinline__ void psolve_segment(double2* __restrict__ u1, double2* __restrict__ u2,
-                                               double2* __restrict__ u3, double2* __restrict__ p,
-                                               double2* __restrict__ psi, const Dims& d, const Tables& t, int col,
-                                               double kx, double kz, double dtirk, double dtrk, int lo, int hi,
-                                               bool pin00, bool& bad) {
-  // levels are loaded four at a time ahead of the recurrences (the arithmetic and its order are those of
-  // one level at a time)
-  const size_t np = d.np;
-  const double* __restrict__ dg2 = t.dg2;
-  const double* __restrict__ dg3 = t.dg3;
-  double2 x = double2{0.0, 0.0};
-  double2 vlo = u2[(size_t)lo * np + col];  // v on face jp, carried from the level below
-  auto fwd = [&](int jp, const double2& a, const double2& w, const double2& v1, const double2& v0, double b2) {
-    const double c = t.cu[jp + 1];
-    const double2 dv = double2{(-kx * a.y - kz * w.y) + c * (v1.x - v0.x), (kx * a.x + kz * w.x) + c * (v1.y - v0.y)};
-    double2 ps = double2{dtirk * dv.x, dtirk * dv.y};
-    if (pin00 && jp == lo) ps = double2{0.0, 0.0};
-    if (jp == lo) x = double2{ps.x * b2, ps.y * b2};
-    else {
-      const double b1 = t.dg1[jp];
-      x = double2{(ps.x - b1 * x.x) * b2, (ps.y - b1 * x.y) * b2};
+// solveP + v_corr over the p levels lo..hi of one column's real or imaginary part (a long column's all, or one wall band
+// of a short one).  The divergence is formed on the fly in the forward sweep; the backward sweep adds psi to p and
+// corrects u, w on the same levels and v on the faces between them.
+//
+// A launch of the 288 x 288 x 226 grid: 0.37 -> 0.27 ms against one thread per column, of 96 x 96 x 130, by tiles,
+// 195 -> 50 us; of 576 x 576 x 450 1.89 ms both ways (1.4 ms of it FP64 issue).
+// u, v, w, p, psi point at the part's value of level 0, ou, ow at the other part of u and w; kx, kz (and kxd, kzd, times
+// dt (a + b)) are negated for the real part: i (kx u + kz w) takes the other part.
+struct ColumnPart {
+  double *u, *v, *w, *p, *psi;
+  const double *ou, *ow, *dg2, *dg3;
+  double kx, kz, kxd, kzd;
+  size_t np, np2;
+};
+// The divergence of level j, from the other part's u and w there and the part's own v on the faces above and below.
+__device__ __forceinline__ double column_div(const ColumnPart& c, double ou, double ow, double cu, double dv) {
+  return fma(cu, dv, fma(c.kx, ou, c.kz * ow));
+}
+// One level of the forward sweep, (dtirk div - b1 x) b2.  Which of the two products is fused into the difference is part
+// of the results: every fourth level from the lower wall and all of a short column's upper band round the right-hand side
+// on its own (`alone`), the others round b1 x.  That is what the compiler made of the sweep when it ran in batches of
+// four, and established runs of the mixed form depend on it: its FP32 transforms turn a last bit of the FP64 state into
+// 1e-8.
+__device__ __forceinline__ double column_up(bool alone, double dtirk, double div, double b1, double b2, double x) {
+  if (alone) return __dmul_rn(fma(-b1, x, __dmul_rn(dtirk, div)), b2);
+  return __dmul_rn(fma(dtirk, div, -__dmul_rn(b1, x)), b2);
+}
+
+__device__ __forceinline__ void psolve_segment(const ColumnPart& c, const Tables& t, const double* F, double dtirk, int lo,
+                                               int hi, bool pin00, bool alone, bool& bad) {
+  constexpr int NB = kColBatch;
+  static_assert(NB == 2, "the forward sweep takes two batches per four levels");
+  const size_t np = c.np, np2 = c.np2;
+  double x = 0.0;
+  {
+    double vlo = c.v[(size_t)lo * np2];  // v on face jp, carried from the level below
+    double A[NB], W[NB], V[NB], B[NB], A2[NB], W2[NB], V2[NB], B2[NB];
+    auto get = [&](int jp, double* a, double* w, double* v, double* b) {
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        const size_t j = (size_t)min(jp + q, hi);
+        a[q] = c.ou[(j + 1) * np2];
+        w[q] = c.ow[(j + 1) * np2];
+        v[q] = c.v[(j + 1) * np2];
+        b[q] = c.dg2[j * np];
+      }
+    };
+    auto div = [&](int j, double a, double w, double v) {
+      const double r = column_div(c, a, w, __ldg(t.cu + j + 1), v - vlo);
+      vlo = v;
+      return pin00 && j == lo ? 0.0 : r;
+    };
+    auto put = [&](int j, double y) {
+      x = y;
+      c.psi[(size_t)j * np2] = x;
+    };
+    const int end = lo + (hi - lo + 1) / 4 * 4;  // of the whole fours
+    get(lo, A, W, V, B);
+    int jp = lo;
+    for (; jp < end; jp += 4) {
+      get(jp + 2, A2, W2, V2, B2);
+      {
+        const double r = div(jp, A[0], W[0], V[0]);
+        const double b1 = __ldg(t.dg1 + jp);
+        put(jp, jp == lo ? __dmul_rn(__dmul_rn(dtirk, r), B[0]) : column_up(true, dtirk, r, b1, B[0], x));
+      }
+      put(jp + 1, column_up(alone, dtirk, div(jp + 1, A[1], W[1], V[1]), __ldg(t.dg1 + jp + 1), B[1], x));
+      if (jp + 4 <= hi) get(jp + 4, A, W, V, B);
+      put(jp + 2, column_up(alone, dtirk, div(jp + 2, A2[0], W2[0], V2[0]), __ldg(t.dg1 + jp + 2), B2[0], x));
+      put(jp + 3, column_up(alone, dtirk, div(jp + 3, A2[1], W2[1], V2[1]), __ldg(t.dg1 + jp + 3), B2[1], x));
     }
-    psi[(size_t)jp * np + col] = x;
+    for (; jp <= hi; ++jp) {
+      get(jp, A, W, V, B);
+      const double r = div(jp, A[0], W[0], V[0]);
+      const double b1 = __ldg(t.dg1 + jp);
+      put(jp, jp == lo ? __dmul_rn(__dmul_rn(dtirk, r), B[0]) : column_up(alone || jp == end, dtirk, r, b1, B[0], x));
+    }
+  }
+  const unsigned pair = 3u << (threadIdx.x & 30);  // the lanes of the column's two parts
+  double S[NB], G[NB], P[NB], A[NB], W[NB], V[NB], S2[NB], G2[NB], P2[NB], A2[NB], W2[NB], V2[NB];
+  auto get = [&](int jp, double* s, double* g, double* p, double* a, double* w, double* v) {
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const size_t j = (size_t)max(jp - q, lo);
+      s[q] = c.psi[j * np2];
+      g[q] = c.dg3[j * np];
+      p[q] = c.p[j * np2];
+      a[q] = c.u[(j + 1) * np2];
+      w[q] = c.w[(j + 1) * np2];
+      v[q] = c.v[(j + 1) * np2];
+    }
   };
-  int jp = lo;
-  for (; jp + 3 <= hi; jp += 4) {
-    double2 A[4], W[4], V[4];
-    double B2[4];
+  double xn = x;  // psi(hi)
+  get(hi, S, G, P, A, W, V);
+  for (int jp = hi; jp >= lo; jp -= NB) {
+    if (jp - NB >= lo) get(jp - NB, S2, G2, P2, A2, W2, V2);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const size_t cu = (size_t)(jp + q + 1) * np + col;
-      A[q] = u1[cu];
-      W[q] = u3[cu];
-      V[q] = u2[cu];
-      B2[q] = dg2[(size_t)(jp + q) * np + col];
+    for (int q = 0; q < NB; ++q) {
+      const int j = jp - q;
+      if (j < lo) break;
+      const double xc = j == hi ? xn : fma(-G[q], xn, S[q]);
+      const double other = __shfl_xor_sync(pair, xc, 1);
+      const double pn = P[q] + xc;
+      // a NaN or infinity anywhere in the fields reaches the divergence of its column, hence psi and p
+      bad = bad || nonfinite(pn);
+      c.p[(size_t)j * np2] = pn;
+      c.u[(size_t)(j + 1) * np2] = fma(-c.kxd, other, A[q]);
+      c.w[(size_t)(j + 1) * np2] = fma(-c.kzd, other, W[q]);
+      if (j < hi) c.v[(size_t)(j + 1) * np2] = fma(-F[j + 1], xn - xc, V[q]);
+      xn = xc;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) fwd(jp + q, A[q], W[q], V[q], q == 0 ? vlo : V[q - 1], B2[q]);
-    vlo = V[3];
-  }
-  for (; jp <= hi; ++jp) {
-    const size_t cu = (size_t)(jp + 1) * np + col;
-    const double2 v1 = u2[cu];
-    fwd(jp, u1[cu], u3[cu], v1, vlo, dg2[(size_t)jp * np + col]);
-    vlo = v1;
-  }
-  const double kxd = dtrk * kx, kzd = dtrk * kz;
-  double2 xn = x;  // psi(hi)
-  auto bwd = [&](int jq, const double2& v, double b3, const double2& pp, const double2& a, const double2& w,
-                 const double2& vv) {
-    const double2 xc = jq == hi ? xn : double2{v.x - b3 * xn.x, v.y - b3 * xn.y};
-    const size_t cp = (size_t)jq * np + col, cu = (size_t)(jq + 1) * np + col;
-    const double2 pn = double2{pp.x + xc.x, pp.y + xc.y};
-    // a NaN or infinity anywhere in the fields reaches the divergence of its column, hence psi and p
-    bad = bad || nonfinite(pn.x) || nonfinite(pn.y);
-    p[cp] = pn;
-    u1[cu] = double2{a.x - (-kxd * xc.y), a.y - (kxd * xc.x)};
-    u3[cu] = double2{w.x - (-kzd * xc.y), w.y - (kzd * xc.x)};
-    if (jq < hi) {
-      const double f = dtrk * t.cv[jq + 1];
-      u2[cu] = double2{vv.x - f * (xn.x - xc.x), vv.y - f * (xn.y - xc.y)};
-    }
-    xn = xc;
-  };
-  jp = hi;
-  for (; jp - 3 >= lo; jp -= 4) {
-    double2 Ps[4], P[4], A[4], W[4], V[4];
-    double B3[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int jq = jp - q;
-      const size_t cp = (size_t)jq * np + col, cu = (size_t)(jq + 1) * np + col;
-      Ps[q] = psi[cp];
-      B3[q] = dg3[cp];
-      P[q] = p[cp];
-      A[q] = u1[cu];
-      W[q] = u3[cu];
-      V[q] = u2[cu];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) bwd(jp - q, Ps[q], B3[q], P[q], A[q], W[q], V[q]);
-  }
-  for (; jp >= lo; --jp) {
-    const size_t cp = (size_t)jp * np + col, cu = (size_t)(jp + 1) * np + col;
-    bwd(jp, psi[cp], dg3[cp], p[cp], u1[cu], u3[cu], u2[cu]);
+    for (int q = 0; q < NB; ++q) { S[q] = S2[q]; G[q] = G2[q]; P[q] = P2[q]; A[q] = A2[q]; W[q] = W2[q]; V[q] = V2[q]; }
   }
 }
 
-__device__ __forceinline__ void psolve_body(double2* u1, double2* u2, double2* u3, double2* p, double2* psi, const Dims& d,
-                                            const Tables& t, double dtirk, double dtrk, double gwb, double gwt,
-                                            DevScalars* sc, int bx) {
-  const int col = bx * blockDim.x + threadIdx.x;
-  if (col >= d.np) return;
-  const size_t np = d.np;
-  const int i = col % d.nkx, kk = col / d.nkx;
-  const double kx = t.kx[i], kz = t.kz[kk];
-  bool bad = false;
-  if (is_long(d, i, kk)) {
-    psolve_segment(u1, u2, u3, p, psi, d, t, col, kx, kz, dtirk, dtrk, 0, d.nyp - 1, col == 0, bad);
-  } else {
-    psolve_segment(u1, u2, u3, p, psi, d, t, col, kx, kz, dtirk, dtrk, 0, d.Nu1 - 1, false, bad);
-    psolve_segment(u1, u2, u3, p, psi, d, t, col, kx, kz, dtirk, dtrk, d.Nu2, d.nyp - 1, false, bad);
-    // v on the end rows of the short column's bands (v_corr, littleharsh.f90:904-905)
-    u2[(size_t)(d.Nv1 + 1) * np + col] = double2{0.0, 0.0};
-    u2[(size_t)d.Nv2 * np + col] = double2{0.0, 0.0};
+// The pressure solve and correction of a tile of columns (see psolve_segment); zeros on the levels a short column does not
+// have and below a segment's first level.
+__device__ __forceinline__ void psolve_tile(const ColumnPart& c, const Dims& d, const Tables& t, double dtirk, double dtrk,
+                                            double gwb, double gwt, bool in, int col, bool lng, bool& bad) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int n = d.nyp, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  double* X = reinterpret_cast<double*>(smraw);    // [nyp][32]
+  double* B2 = X + (size_t)n * kTileParts;         // dg2 per level and column: [nyp][16]
+  double* G = B2 + (size_t)n * (kTileParts / 2);   // dg3
+  double* D1 = G + (size_t)n * (kTileParts / 2);   // dg1 per level
+  const size_t np = c.np, np2 = c.np2;
+  auto has = [&](int j) { return lng || j < d.Nu1 || j >= d.Nu2; };
+  constexpr int NB = kTileBatch;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) D1[j] = j == 0 ? 0.0 : t.dg1[j];
+  if (in) {
+    for (int j0 = warp; j0 < n; j0 += NB * warps) {
+      double A[NB], W[NB], V0[NB], V1[NB], B[NB], D[NB];
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        const size_t j = (size_t)min(j0 + q * warps, n - 1);
+        A[q] = c.ou[(j + 1) * np2];
+        W[q] = c.ow[(j + 1) * np2];
+        V0[q] = c.v[j * np2];
+        V1[q] = c.v[(j + 1) * np2];
+        B[q] = __ldg(c.dg2 + j * np);
+        D[q] = __ldg(c.dg3 + j * np);
+      }
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        const int j = j0 + q * warps;
+        if (j >= n) break;
+        const double dv = column_div(c, A[q], W[q], __ldg(t.cu + j + 1), V1[q] - V0[q]);
+        const bool none = !has(j), last = j == n - 1 || (!lng && j < d.Nu2 && j >= d.Nu1 - 1);
+        X[j * kTileParts + lane] = (col == 0 && j == 0) || none ? 0.0 : dv;
+        if (!(lane & 1)) {
+          B2[j * (kTileParts / 2) + (lane >> 1)] = none ? 0.0 : B[q];
+          G[j * (kTileParts / 2) + (lane >> 1)] = last ? 0.0 : D[q];
+        }
+      }
+    }
   }
-  u2[col] = double2{0.0, 0.0};
-  u2[(size_t)(d.nyv - 1) * np + col] = double2{0.0, 0.0};
-  {
-    const double2 a = u1[np + col], w = u3[np + col];
-    u1[col] = double2{-gwb * a.x, -gwb * a.y};
-    u3[col] = double2{-gwb * w.x, -gwb * w.y};
-    const double2 at = u1[(size_t)(d.nyu - 2) * np + col], wt = u3[(size_t)(d.nyu - 2) * np + col];
-    u1[(size_t)(d.nyu - 1) * np + col] = double2{-gwt * at.x, -gwt * at.y};
-    u3[(size_t)(d.nyu - 1) * np + col] = double2{-gwt * wt.x, -gwt * wt.y};
+  __syncthreads();
+  if (warp == 0 && in) {
+    double *x = X + lane, y = 0.0;
+    const double *b = B2 + (lane >> 1), *g = G + (lane >> 1);
+    auto up = [&](int j, bool alone) {
+      const double r = x[j * kTileParts], bj = b[j * (kTileParts / 2)];
+      y = column_up(alone, dtirk, r, D1[j], bj, y);
+      x[j * kTileParts] = y;
+    };
+    if (!d.banded) {
+      int j = 0;
+#pragma unroll 2
+      for (; j + 3 < n; j += 4) {
+        up(j, true);
+        up(j + 1, false);
+        up(j + 2, false);
+        up(j + 3, false);
+      }
+      for (; j < n; ++j) up(j, (j & 3) == 0);
+    } else {
+      // b = 0 on the levels between a short column's bands leaves y = 0, as the upper segment's first level wants it
+      for (int j = 0; j < n; ++j) {
+        up(j, (!lng && j >= d.Nu2) || (j & 3) == 0);
+      }
+    }
+#pragma unroll 8
+    for (int j = n - 2; j >= 0; --j) {
+      y = fma(-g[j * (kTileParts / 2)], y, x[j * kTileParts]);
+      x[j * kTileParts] = y;
+    }
+  }
+  __syncthreads();
+  if (!in) return;
+  for (int j0 = warp; j0 < n; j0 += NB * warps) {
+    double P[NB], A[NB], W[NB], V[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const size_t j = (size_t)min(j0 + q * warps, n - 1);
+      P[q] = c.p[j * np2];
+      A[q] = c.u[(j + 1) * np2];
+      W[q] = c.w[(j + 1) * np2];
+      V[q] = c.v[(j + 1) * np2];
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const int j = j0 + q * warps;
+      if (j >= n) break;
+      if (!has(j)) continue;
+      const size_t f = (size_t)(j + 1) * np2;
+      const double x = X[j * kTileParts + lane], o = X[j * kTileParts + (lane ^ 1)];
+      const double pn = P[q] + x, u = fma(-c.kxd, o, A[q]), w = fma(-c.kzd, o, W[q]);
+      bad = bad || nonfinite(pn);
+      c.p[(size_t)j * np2] = pn;
+      c.u[f] = u;
+      c.w[f] = w;
+      if (j == 0) { c.u[0] = -gwb * u; c.w[0] = -gwb * w; }
+      if (j == n - 1) { c.u[f + np2] = -gwt * u; c.w[f + np2] = -gwt * w; }
+      if (j < n - 1 && has(j + 1)) c.v[f] = fma(-__dmul_rn(dtrk, __ldg(t.cv + j + 1)), X[(j + 1) * kTileParts + lane] - x, V[q]);
+    }
+  }
+  if (warp == 0) {  // walls, and the end rows of the short column's bands (v_corr, littleharsh.f90:904-905)
+    c.v[0] = 0.0;
+    c.v[(size_t)(d.nyv - 1) * np2] = 0.0;
+    if (!lng) {
+      c.v[(size_t)(d.Nv1 + 1) * np2] = 0.0;
+      c.v[(size_t)d.Nv2 * np2] = 0.0;
+    }
+  }
+}
+
+__device__ __forceinline__ ColumnPart column_part(double2* u1, double2* u2, double2* u3, double2* p, double2* psi, const Dims& d,
+                                                  const Tables& t, double dtrk, int part) {
+  const int col = part >> 1;
+  const double sign = (part & 1) ? 1.0 : -1.0;
+  ColumnPart c;
+  c.np = d.np; c.np2 = 2 * (size_t)d.np;
+  c.u = reinterpret_cast<double*>(u1) + part;
+  c.v = reinterpret_cast<double*>(u2) + part;
+  c.w = reinterpret_cast<double*>(u3) + part;
+  c.p = reinterpret_cast<double*>(p) + part;
+  c.psi = reinterpret_cast<double*>(psi) + part;
+  c.ou = reinterpret_cast<double*>(u1) + (part ^ 1);
+  c.ow = reinterpret_cast<double*>(u3) + (part ^ 1);
+  c.dg2 = t.dg2 + col;
+  c.dg3 = t.dg3 + col;
+  c.kx = sign * t.kx[col % d.nkx];
+  c.kz = sign * t.kz[col / d.nkx];
+  c.kxd = dtrk * c.kx;
+  c.kzd = dtrk * c.kz;
+  return c;
+}
+
+template <bool TILE>
+__device__ __forceinline__ void psolve_body(double2* u1, double2* u2, double2* u3, double2* p, double2* psi, const Dims& d,
+                                            const Tables& t, double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc,
+                                            int bx) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  bool bad = false;
+  if constexpr (TILE) {
+    const int part = bx * kTileParts + (threadIdx.x & 31);
+    const bool in = (part >> 1) < d.np;
+    const ColumnPart c = column_part(u1, u2, u3, p, psi, d, t, dtrk, in ? part : 0);
+    const int col = in ? part >> 1 : 0;
+    psolve_tile(c, d, t, dtirk, dtrk, gwb, gwt, in, col, is_long(d, col % d.nkx, col / d.nkx), bad);
+  } else {
+    double* F = reinterpret_cast<double*>(smraw);  // dtrk cv per face
+    for (int j = threadIdx.x; j < d.nyv; j += blockDim.x) F[j] = dtrk * t.cv[j];
+    __syncthreads();
+    const int part = bx * blockDim.x + threadIdx.x, col = part >> 1;
+    if (col >= d.np) return;
+    const ColumnPart c = column_part(u1, u2, u3, p, psi, d, t, dtrk, part);
+    if (is_long(d, col % d.nkx, col / d.nkx)) {
+      psolve_segment(c, t, F, dtirk, 0, d.nyp - 1, col == 0, false, bad);
+    } else {
+      psolve_segment(c, t, F, dtirk, 0, d.Nu1 - 1, false, false, bad);
+      psolve_segment(c, t, F, dtirk, d.Nu2, d.nyp - 1, false, true, bad);
+      // v on the end rows of the short column's bands (v_corr, littleharsh.f90:904-905)
+      c.v[(size_t)(d.Nv1 + 1) * c.np2] = 0.0;
+      c.v[(size_t)d.Nv2 * c.np2] = 0.0;
+    }
+    c.v[0] = 0.0;
+    c.v[(size_t)(d.nyv - 1) * c.np2] = 0.0;
+    c.u[0] = -gwb * c.u[c.np2];
+    c.w[0] = -gwb * c.w[c.np2];
+    c.u[(size_t)(d.nyu - 1) * c.np2] = -gwt * c.u[(size_t)(d.nyu - 2) * c.np2];
+    c.w[(size_t)(d.nyu - 1) * c.np2] = -gwt * c.w[(size_t)(d.nyu - 2) * c.np2];
   }
   if (bad && sc) atomicOr(&sc->err, kErrNonFinite);
 }
 
-__global__ void __launch_bounds__(128, 4) k_psolve(double2* u1, double2* u2, double2* u3, double2* p, double2* psi,
-                                                   const __grid_constant__ Dims d, const __grid_constant__ Tables t,
-                                                   double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc) {
-  psolve_body(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc, blockIdx.x);
+__global__ void __launch_bounds__(kColThreads) k_psolve(double2* u1, double2* u2, double2* u3, double2* p, double2* psi,
+                                                        const __grid_constant__ Dims d, const __grid_constant__ Tables t,
+                                                        double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc) {
+  psolve_body<false>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc, blockIdx.x);
+}
+__global__ void __launch_bounds__(kTileThreads, 2) k_psolve_tile(double2* u1, double2* u2, double2* u3, double2* p, double2* psi,
+                                                                 const __grid_constant__ Dims d, const __grid_constant__ Tables t,
+                                                                 double dtirk, double dtrk, double gwb, double gwt,
+                                                                 DevScalars* sc) {
+  psolve_body<true>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc, blockIdx.x);
 }
 
 void launch_psolve(double2* u1, double2* u2, double2* u3, double2* p, double2* psi, const Dims& d, const Tables& t,
                    double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc, cudaStream_t st) {
-  dim3 grid((d.np + 127) / 128);
-  k_psolve<<<grid, 128, 0, st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
+  if (psolve_tiled(d))
+    k_psolve_tile<<<psolve_ctas(d), kTileThreads, psolve_smem(d), st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
+  else
+    k_psolve<<<psolve_ctas(d), kColThreads, psolve_smem(d), st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
 }
 
 __global__ void k_divergence(const double2* u1, const double2* u2, const double2* u3, double2* div, Dims d, Tables t) {
@@ -2024,7 +2300,7 @@ __global__ void __launch_bounds__(256, 3) k_assemble_batch(const __grid_constant
   assemble_body<P>(D.a, D.d, D.t, q % D.gx, q / D.gx);
 }
 
-__global__ void __launch_bounds__(128) k_vsolve_batch(const __grid_constant__ Batch<VDesc> b) {
+__global__ void __launch_bounds__(kTileThreads, 5) k_vsolve_batch(const __grid_constant__ Batch<VDesc> b) {
   const int m = batch_member(b, blockIdx.x);
   const VDesc& D = b.desc[m];
   const int q = blockIdx.x - b.start[m];
@@ -2036,10 +2312,11 @@ __global__ void k_flowrate_batch(const __grid_constant__ Batch<FDesc> b) {
   flowrate_body(D.u1, D.sc, D.d, D.t, D.k, D.Qx1);
 }
 
-__global__ void __launch_bounds__(128, 4) k_psolve_batch(const __grid_constant__ Batch<PDesc> b) {
+template <bool TILE>
+__global__ void __launch_bounds__(TILE ? kTileThreads : kColThreads) k_psolve_batch(const __grid_constant__ Batch<PDesc> b) {
   const int m = batch_member(b, blockIdx.x);
   const PDesc& D = b.desc[m];
-  psolve_body(D.u1, D.u2, D.u3, D.p, D.psi, D.d, D.t, D.dtirk, D.dtrk, D.gwb, D.gwt, D.sc, blockIdx.x - b.start[m]);
+  psolve_body<TILE>(D.u1, D.u2, D.u3, D.p, D.psi, D.d, D.t, D.dtirk, D.dtrk, D.gwb, D.gwt, D.sc, blockIdx.x - b.start[m]);
 }
 
 template <typename R>
@@ -2063,14 +2340,17 @@ void launch_assemble_batch(const Batch<ADesc>& b, bool fp32_products, cudaStream
   if (fp32_products) k_assemble_batch<float2><<<b.start[b.n], 256, 0, st>>>(b);
   else k_assemble_batch<double2><<<b.start[b.n], 256, 0, st>>>(b);
 }
-void launch_vsolve_batch(const Batch<VDesc>& b, cudaStream_t st) {
-  if (b.n > 0 && b.start[b.n] > 0) k_vsolve_batch<<<b.start[b.n], 128, 0, st>>>(b);
+void launch_vsolve_batch(const Batch<VDesc>& b, size_t smem, cudaStream_t st) {
+  if (b.n > 0 && b.start[b.n] > 0) k_vsolve_batch<<<b.start[b.n], smem ? kTileThreads : kColThreads, smem, st>>>(b);
 }
 void launch_flowrate_batch(const Batch<FDesc>& b, cudaStream_t st) {
-  if (b.n > 0 && b.start[b.n] > 0) k_flowrate_batch<<<b.start[b.n], 256, 0, st>>>(b);
+  if (b.n > 0 && b.start[b.n] > 0) k_flowrate_batch<<<b.start[b.n], kFlowThreads, 0, st>>>(b);
 }
-void launch_psolve_batch(const Batch<PDesc>& b, cudaStream_t st) {
-  if (b.n > 0 && b.start[b.n] > 0) k_psolve_batch<<<b.start[b.n], 128, 0, st>>>(b);
+void launch_psolve_batch(const Batch<PDesc>& b, size_t smem, cudaStream_t st) {
+  if (b.n <= 0 || b.start[b.n] <= 0) return;
+  // members of one shared-memory size are of one form
+  if (psolve_tiled(b.desc[0].d)) k_psolve_batch<true><<<b.start[b.n], kTileThreads, smem, st>>>(b);
+  else k_psolve_batch<false><<<b.start[b.n], kColThreads, smem, st>>>(b);
 }
 
 // FP64 FMA throughput probe: every thread runs eight independent dependent
@@ -2143,7 +2423,8 @@ cudaError_t configure_kernels() {
   int optin = 0;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  const cudaError_t r[18] = {allow_smem(k_xcond, optin), allow_smem(k_zinv<double>, optin), allow_smem(k_zinv<float>, optin),
+  const cudaError_t r[22] = {allow_smem(k_vsolve, optin), allow_smem(k_psolve_tile, optin), allow_smem(k_vsolve_batch, optin),
+                             allow_smem(k_psolve_batch<true>, optin), allow_smem(k_xcond, optin), allow_smem(k_zinv<double>, optin), allow_smem(k_zinv<float>, optin),
                              allow_smem(k_zfwd<double>, optin), allow_smem(k_zfwd<float>, optin),
                              allow_smem(k_xprod_fx, optin), allow_smem(k_xprod, optin), allow_smem(k_xprod2, optin),
                              allow_smem(k_xmask<double>, optin), allow_smem(k_xmask<float>, optin),

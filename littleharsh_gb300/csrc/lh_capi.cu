@@ -223,13 +223,13 @@ int build_fx(lh_handle* h, FxPlan* P, int n) {
   FxTables t;
   if (!fx_build(n, P, &t)) return fail(h, LH_EFFT, "transform length %d is too long", n);
   if (t.tw.empty()) t.tw.push_back(int4{0, 0, 0, 0});
-  short *a, *b, *c, *e, *f;
+  short *a, *b, *e, *f;
   int4* w;
   int rc;
-  if ((rc = upload(h, &a, t.pos_sample)) || (rc = upload(h, &b, t.pos_freq)) || (rc = upload(h, &c, t.sample_pos)) ||
-      (rc = upload(h, &e, t.freq_pos)) || (rc = upload(h, &f, t.turn)) || (rc = upload(h, &w, t.tw)))
+  if ((rc = upload(h, &a, t.pos_sample)) || (rc = upload(h, &b, t.pos_freq)) || (rc = upload(h, &e, t.freq_pos)) ||
+      (rc = upload(h, &f, t.turn)) || (rc = upload(h, &w, t.tw)))
     return rc;
-  P->pos_sample = a; P->pos_freq = b; P->sample_pos = c; P->freq_pos = e; P->turn = f; P->tw = w;
+  P->pos_sample = a; P->pos_freq = b; P->freq_pos = e; P->turn = f; P->tw = w;
   return LH_OK;
 }
 

@@ -63,7 +63,6 @@ struct FxPlan {
   FxPass ps[kFxMaxPass];
   const short* pos_sample;   // position of sample s
   const short* pos_freq;     // position of frequency k
-  const short* sample_pos;   // sample at a position
   const short* freq_pos;     // frequency at a position
   const short* turn;         // pos_sample[freq_pos[.]]: from the place of an output to that of an input
   const int4* tw;            // two int4 per twiddle: (w_r, w_r + w_i), (w_i - w_r, -), each high and low word
@@ -107,13 +106,11 @@ FX_HD i64 fx_mul(i64 a, int bh, int bl) {
   return fx_shl((i64)h * bh + t, POST);
 }
 
-// a b / 2^61 for |a|, |b| < 2^60
-FX_HD i64 fx_mulvar(i64 a, i64 b) {
-  const i64 s = fx_shl(a, 3);
-  const int h = (int)(s >> 32), l = (int)((unsigned)s >> 1);  // unsigned halves of the low word: h may be 2^31 - 1
-  const int bl = (int)b, bh = fx_high(b);
-  const int t = fx_mhi(h, bl) + 2 * fx_mhi(l, bh) + 1;
-  return (i64)h * bh + t;
+// a b / 2^64 for |a|, |b| < 2^62
+FX_HD i64 fx_prod(i64 a, i64 b) {
+  const int al = (int)a, ah = fx_high(a), bl = (int)b, bh = fx_high(b);
+  const int t = fx_mhi(ah, bl) + fx_mhi(al, bh) + 1;
+  return (i64)ah * bh + t;
 }
 
 FX_HD fx2 fx_add(fx2 a, fx2 b) { return fx2{a.x + b.x, a.y + b.y}; }
@@ -465,8 +462,6 @@ struct FxOut {
 __device__ __forceinline__ unsigned fx_hi(double2 v) {
   return max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
 }
-// a shifted left (s >= 0) or right (s < 0)
-__device__ __forceinline__ i64 fx_shift(i64 a, int s) { return s >= 0 ? fx_shl(a, s) : a >> -s; }
 // magnitude bits of the high word
 __device__ __forceinline__ unsigned fx_bits(i64 a) {
   const int h = (int)(a >> 32);
@@ -480,7 +475,7 @@ __device__ __forceinline__ unsigned fx_bits(i64 a) {
 // ---------------------------------------------------------------------------
 
 struct FxTables {
-  std::vector<short> pos_sample, pos_freq, sample_pos, freq_pos, turn;
+  std::vector<short> pos_sample, pos_freq, freq_pos, turn;
   std::vector<int4> tw;
 };
 
@@ -540,12 +535,11 @@ inline bool fx_build(int n, FxPlan* plan, FxTables* tab) {
     return 0;
   };
   const int qi = inverse(Q % P, P), pi = inverse(P % Q, Q);
-  tab->pos_sample.resize(n); tab->pos_freq.resize(n); tab->sample_pos.resize(n); tab->freq_pos.resize(n);
+  tab->pos_sample.resize(n); tab->pos_freq.resize(n); tab->freq_pos.resize(n);
   for (int s = 0; s < n; ++s) {
     const int n1 = (int)((long long)s * qi % P), n2 = (int)((long long)s * pi % Q);
     const int ps = place(0, n1, P) * Q + place(1, n2, Q), pf = (s % P) * Q + s % Q;
     tab->pos_sample[s] = (short)ps;
-    tab->sample_pos[ps] = (short)s;
     tab->pos_freq[s] = (short)pf;
     tab->freq_pos[pf] = (short)s;
   }

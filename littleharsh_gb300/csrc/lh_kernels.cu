@@ -560,12 +560,13 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
 // Three inverse lines of ngx: (u, w) of level j, (v of j, v of j + 1), (u, w) of j + 1, each two real rows in one complex
 // line.  They come out in 64-bit integers with one scale per line, are shifted to the full range by what their largest
 // value leaves (found by an OR over the magnitudes), interpolated and multiplied as integers, and the products go
-// forward two to a line: (uu, uw), (ww, vv), (uv, vw), each pair on the coarser of its two scales.  The FP64 the rows
-// come from and go to is the kernel's only floating point, but for the CFL number.
+// forward two to a line: (uu, uw), (ww, vv), (uv, vw), each pair on one scale.  They start a bit below a line's range, so
+// that the sums which separate a pair's spectra fit.  The FP64 the rows come from and go to is the kernel's only floating
+// point, but for the CFL number.
 //
-// Bound by instruction issue on the integer pipes (390 instructions a point of a transform, 53 % issue; transforms about
-// half of them), no longer by the FP64 pipe.  80 registers (three CTAs of 256 threads).  A step of the 576 x 576 x 450
-// grid: 140.0 -> 36.9 ms; 96 x 96 x 130 1.81 -> 0.46, 48 x 48 x 66 0.65 -> 0.11 ms.  Its memory traffic alone is 3 ms.
+// Bound by instruction issue on the integer pipes (340 instructions a point of a transform, 190 of them the transforms';
+// 51 % issue), no longer by the FP64 pipe.  A step of the 576 x 576 x 450 grid: 140.0 -> 34.0 ms; 288 x 288 x 226 17.8 ->
+// 4.1, 96 x 96 x 130 1.81 -> 0.44, 48 x 48 x 66 0.65 -> 0.10 ms.  Its memory traffic alone is 3 ms.
 //
 // Shared memory: two buffers of three lines that exchange their parts every two levels (the raw FP64 rows and the
 // products in one, the inverse lines in the other: while the last products are transformed, the next rows are copied in
@@ -593,6 +594,8 @@ __host__ __device__ __forceinline__ int xprod_levels(int ngx) { return ngx <= 19
 // Levels of a CTA: whole iterations, so that every level's v has the same partner whatever the chunk.
 __host__ __device__ __forceinline__ int xprod_chunk(int chunk, int ngx) { return xprod_levels(ngx) == 2 ? (chunk + 1) & ~1 : chunk; }
 
+// TWO: two levels an iteration (xprod_levels).
+template <bool TWO>
 __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims& d, const XPlan<double>& plan, int bx,
                                            int by) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -600,7 +603,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
   __shared__ double cflred[8];
   const FxPlan& P = plan.pf;
   const int n = d.ngx, nkx = d.nkx, tid = threadIdx.x, bd = blockDim.x;
-  const int lp = xprod_levels(n), nl = lp + 1;  // levels and lines of an iteration
+  constexpr int lp = TWO ? 2 : 1, nl = lp + 1;  // levels and lines of an iteration
   fx2* B0 = reinterpret_cast<fx2*>(smraw);      // nl lines
   fx2* B1 = B0 + nl * n;                        // nl lines
   i64* pu = reinterpret_cast<i64*>(B1 + nl * n);  // u, w, v of the previous level
@@ -615,18 +618,16 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
   // j + 1) into raw: row r of line l at raw[(2 l + r) nkx].  A row that does not exist is zero.
   auto fetch = [&](fx2* raw, int j, bool two, int jv, int v_lo, int v_hi) {
     const int rows = two ? 6 : 4;
-    for (int t = tid; t < rows * nkx; t += bd) {
-      const int q = t / nkx, k = t - q * nkx;
-      const double2* src = nullptr;
-      if (q == 2 || q == 3) {
-        const int f = jv + (q - 2);
-        if (f >= v_lo && f <= v_hi) src = a.mv + (size_t)f * d.mp;
-      } else {
-        const int f = q < 2 ? j : j + 1;
-        src = ((q & 1) ? a.mw : a.mu) + (size_t)f * d.mp;
+#pragma unroll 1
+    for (int q = 0; q < rows; ++q) {
+      const bool v = q == 2 || q == 3;
+      const int f = v ? jv + q - 2 : (q < 2 ? j : j + 1);
+      const double2* src = (v ? a.mv : ((q & 1) ? a.mw : a.mu)) + (size_t)f * d.mp + rowoff;
+      const bool none = v && (f < v_lo || f > v_hi);
+      for (int k = tid; k < nkx; k += bd) {
+        if (none) raw[q * nkx + k] = fx2{0, 0};
+        else fx_copy(raw + q * nkx + k, src + k);
       }
-      if (src) fx_copy(raw + t, src + rowoff + k);
-      else raw[t] = fx2{0, 0};
     }
   };
 
@@ -635,20 +636,15 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
     const double2* rd = reinterpret_cast<const double2*>(raw);
     fx_copy_wait();
     __syncthreads();
-    unsigned m[3] = {0, 0, 0};
-    for (int t = tid; t < 2 * nv * nkx; t += bd) {
-      const unsigned h = fx_hi(rd[t]);
-      const int q = t / (2 * nkx);
-      m[0] = max(m[0], q == 0 ? h : 0u);
-      m[1] = max(m[1], q == 1 ? h : 0u);
-      m[2] = max(m[2], q == 2 ? h : 0u);
+#pragma unroll 1
+    for (int v = 0; v < nv; ++v) {
+      unsigned m = 0;
+      for (int k = tid; k < 2 * nkx; k += bd) m = max(m, fx_hi(rd[2 * v * nkx + k]));
+      fx_reduce_max(m, &R.e[v]);
     }
-#pragma unroll
-    for (int v = 0; v < 3; ++v)
-      if (v < nv) fx_reduce_max(m[v], &R.e[v]);
     for (int i = tid; i < (int)(sizeof(FxProd) / 4); i += bd) reinterpret_cast<unsigned*>(&next)[i] = 0;
     __syncthreads();
-    unsigned sum[3] = {0, 0, 0};
+#pragma unroll 1
     for (int v = 0; v < nv; ++v) {
       const FxIn in((int)(R.e[v] >> 20) + 1);  // one bit of room: a line's values are sums of two rows'
       const double2 *ra = rd + 2 * v * nkx, *rb = ra + nkx;
@@ -669,16 +665,12 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
         }
       }
       for (int k = nkx + tid; k <= n - nkx; k += bd) z[P.pos_sample[k]] = fx2{0, 0};
-      sum[0] += v == 0 ? s : 0u;
-      sum[1] += v == 1 ? s : 0u;
-      sum[2] += v == 2 ? s : 0u;
+      fx_reduce_add(s, &R.sum[v]);
     }
-#pragma unroll
-    for (int v = 0; v < 3; ++v)
-      if (v < nv) fx_reduce_add(sum[v], &R.sum[v]);
     __syncthreads();
     fx_fft(Z, nv, P, R.sum);
     // magnitude bits of the real (u, v of the lower level) and the imaginary rows (w, v of the upper one)
+#pragma unroll 1
     for (int v = 0; v < nv; ++v) {
       unsigned o0 = 0, o1 = 0;
       for (int x = tid; x < n; x += bd) {
@@ -690,16 +682,25 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
       fx_reduce_or(o1, &R.bits[2 * v + 1]);
     }
     __syncthreads();
+    // a line that kept more than 61 bits (many modes of one size) comes down by two
+    bool over = false;
+    for (int v = 0; v < nv; ++v) {
+      if (!(R.bits[2 * v] >> 29 | R.bits[2 * v + 1] >> 29)) continue;
+      for (int x = tid; x < n; x += bd) Z[v * n + x] = fx2{Z[v * n + x].x >> 2, Z[v * n + x].y >> 2};
+      over = true;
+    }
+    if (over) __syncthreads();
   };
-  // scale of a line, and left shift and scale of its rows brought below 2^60
+  // scale of a line, and the left shift that brings a row of it below 2^61
+  auto over = [&](const FxProd& R, int v) { return (R.bits[2 * v] >> 29 | R.bits[2 * v + 1] >> 29) ? 2 : 0; };
   auto line_scale = [&](const FxProd& R, int v) {
-    return fx_scale((int)(R.e[v] >> 20) + 1) - fx_inv_shift(R.sum[v], P.shift);
+    return fx_scale((int)(R.e[v] >> 20) + 1) - fx_inv_shift(R.sum[v], P.shift) - over(R, v);
   };
-  auto room = [&](const FxProd& R, int row) { return __clz((int)R.bits[row]) - 4; };
+  auto room = [&](const FxProd& R, int row) { return __clz((int)(R.bits[row] >> over(R, row >> 1))) - 3; };
   auto lost = [&](const FxProd& R, int v) { return R.e[v] >= 0x7ff00000u; };
 
   constexpr int kNone = 1 << 14;  // scale of a row of zeros: finer than any other
-  int Spu = kNone, Spw = kNone, Spv = kNone;  // scales of the previous level's rows
+  int Sp = kNone, Spv = kNone;        // scales of the previous level's u and w, and of its v
   bool badp = false, badpv = false;
   double cmax = 0.0;
   int it = 0;
@@ -713,15 +714,14 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
     __syncthreads();  // red is cleared
     inverse(raw, Z, 2, red[0], red[1]);
     const FxProd& R = red[0];
-    const int su = room(R, 0), sw = room(R, 1), sv = room(R, paired ? 3 : 2);
+    const int s0 = min(room(R, 0), room(R, 1)), sv = room(R, paired ? 3 : 2);
     for (int x = tid; x < n; x += bd) {
       const fx2 z = Z[x], zv = Z[n + x];
-      pu[x] = fx_shift(z.y, su);
-      pw[x] = fx_shift(z.x, sw);
-      pv[x] = fx_shift(paired ? zv.x : zv.y, sv);
+      pu[x] = fx_shl(z.y, s0);
+      pw[x] = fx_shl(z.x, s0);
+      pv[x] = fx_shl(paired ? zv.x : zv.y, sv);
     }
-    Spu = line_scale(R, 0) + su;
-    Spw = line_scale(R, 0) + sw;
+    Sp = line_scale(R, 0) + s0;
     Spv = line_scale(R, 1) + sv;
     badp = lost(R, 0);
     badpv = lost(R, 1);
@@ -735,51 +735,55 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
     const bool two = lp == 2 && j < c1;
     FxProd& R = red[it & 1];
     inverse(raw, Z, two ? 3 : 2, R, red[(it + 1) & 1]);
+#pragma unroll 1
     for (int q = 0; q < (two ? 2 : 1); ++q) {
       const int jj = j + q;
       const bool cprod = jj >= a.c_lo && jj <= a.c_hi;
       const bool fprod = jj - 1 >= a.f_lo && jj - 1 <= a.f_hi;  // face jj-1 interior and in this launch
       const bool vface = jj <= v_top;
       const int vu = q == 0 ? 0 : 2;
-      const int su = room(R, 2 * vu), sw = room(R, 2 * vu + 1), sv = room(R, 2 + q);
-      const int Su = line_scale(R, vu) + su, Sw = line_scale(R, vu) + sw, Sv = vface ? line_scale(R, 1) + sv : kNone;
+      // u and w share their line's scale, as far left as the larger allows: (uu, uw) and (uv, vw) are pairs of one scale.
+      // (ww, vv) is a pair of its own: w by its own size, on the coarser of its scale and v's
+      const int S = line_scale(R, vu), rw = room(R, 2 * vu + 1), s0 = min(room(R, 2 * vu), rw), sv = room(R, 2 + q);
+      const int Sc = S + s0, Sv = vface ? line_scale(R, 1) + sv : kNone;
       const bool bad = lost(R, vu), badv = lost(R, 1);
-      // v at the centre, u and w at the face below, each on the coarser scale of its two levels
       const int4 wc = plan.wc[jj], wf = fprod ? plan.wf[jj - 1] : int4{0, 0, 0, 0};
-      const int Svc = min(Spv, Sv) - (wc.z ? wc.z + 1 : 0);
-      const int Suf = min(Spu, Su) - (wf.z ? wf.z + 1 : 0), Swf = min(Spw, Sw) - (wf.z ? wf.z + 1 : 0);
-      const int dvp = min(Spv - Svc, 63), dvc = min(Sv - Svc, 63), dup = min(Spu - Suf, 63), duc = min(Su - Suf, 63),
-                dwp = min(Spw - Swf, 63), dwc = min(Sw - Swf, 63);
-      // the products' scales and what brings each on its pair's
-      const int Suu = 2 * Su - 61, Suw = Su + Sw - 61, Sww = 2 * Sw - 61, Svv = 2 * Svc - 61;
-      const int Suv = Suf + Spv - 61, Svw = Swf + Spv - 61;
-      const int S0 = min(Suu, Suw), S1 = min(Sww, Svv), S2 = min(Suv, Svw);
-      const int d00 = min(Suu - S0, 63), d01 = min(Suw - S0, 63), d10 = min(Sww - S1, 63), d11 = min(Svv - S1, 63),
-                d20 = min(Suv - S2, 63), d21 = min(Svw - S2, 63);
+      // interpolated values on the coarser scale of the two levels (weights beyond [-1, 1] want more room)
+      const int T1 = min(S + rw, min(Spv, Sv)) - (wc.z ? wc.z + 1 : 0), Tf = min(Sp, Sc) - (wf.z ? wf.z + 1 : 0);
+      const int dw = min(S + rw - T1, 63), dvp = min(Spv - T1, 63), dvc = min(Sv - T1, 63);
+      const int dp = min(Sp - Tf, 63), dc = min(Sc - Tf, 63);
+      const bool shift1 = (dw | dvp | dvc) != 0, shiftf = (dp | dc) != 0;
+      const int S0 = 2 * Sc - 64, S1 = 2 * T1 - 64, S2 = Tf + Spv - 64;  // the pairs' scales
       fx2* F = raw;
       int np = 0;                        // lines transformed forward at once
       const int f0 = 0, f1 = cprod ? 2 : 0;
-      const bool split = nl < 3 && cprod && fprod;  // the face pair after the centre pairs
+      const bool split = !TWO && cprod && fprod;  // the face pair after the centre pairs
       auto face = [&](int x, i64 u, i64 w, int slot) {
-        const i64 up = pu[x] >> dup, wp = pw[x] >> dwp, v = pv[x];
-        const i64 uf = up + fx_shl(fx_mul<1, 1>((u >> duc) - up, wf.x, wf.y), wf.z);
-        const i64 wv = wp + fx_shl(fx_mul<1, 1>((w >> dwc) - wp, wf.x, wf.y), wf.z);
-        F[slot * n + P.turn[x]] = fx2{fx_mulvar(uf, v) >> d20, fx_mulvar(wv, v) >> d21};
+        i64 up = pu[x], wp = pw[x];
+        if (shiftf) { up >>= dp; wp >>= dp; u >>= dc; w >>= dc; }
+        i64 du = fx_mul<0, 2>(u - up, wf.x, wf.y), dwf = fx_mul<0, 2>(w - wp, wf.x, wf.y);
+        if (wf.z) { du = fx_shl(du, wf.z); dwf = fx_shl(dwf, wf.z); }
+        const i64 v = pv[x];
+        F[slot * n + P.turn[x]] = fx2{fx_prod(up + du, v), fx_prod(wp + dwf, v)};
       };
+#pragma unroll 1
       for (int x = tid; x < n; x += bd) {
         const fx2 z = Z[vu * n + x], zv = Z[n + x];
-        const i64 u = fx_shift(z.y, su), w = fx_shift(z.x, sw);
-        const i64 v = vface ? fx_shift(q == 0 ? zv.y : zv.x, sv) : 0;
+        const i64 u = fx_shl(z.y, s0), w = fx_shl(z.x, s0);
+        const i64 v = vface ? fx_shl(q == 0 ? zv.y : zv.x, sv) : 0;
         if (cprod) {
-          const i64 vp = pv[x] >> dvp;
-          const i64 vc = vp + fx_shl(fx_mul<1, 1>((v >> dvc) - vp, wc.x, wc.y), wc.z);
+          i64 w1 = fx_shl(z.x, rw), vp = pv[x], v1 = v;
+          if (shift1) { w1 >>= dw; vp >>= dvp; v1 >>= dvc; }
+          i64 dv = fx_mul<0, 2>(v1 - vp, wc.x, wc.y);
+          if (wc.z) dv = fx_shl(dv, wc.z);
+          const i64 vc = vp + dv;
           if (a.want_cfl) {
             if (!bad && !badv && !badpv)
-              cmax = fmax(cmax, fabs(fx_to(u, Su)) * a.dxi + fabs(fx_to(vc, Svc)) * a.dyc[jj] + fabs(fx_to(w, Sw)) * a.dzi);
+              cmax = fmax(cmax, fabs(fx_to(u, Sc)) * a.dxi + fabs(fx_to(vc, T1)) * a.dyc[jj] + fabs(fx_to(w, Sc)) * a.dzi);
           } else {
             const int px = P.turn[x];
-            F[px] = fx2{fx_mulvar(u, u) >> d00, fx_mulvar(u, w) >> d01};
-            F[n + px] = fx2{fx_mulvar(w, w) >> d10, fx_mulvar(vc, vc) >> d11};
+            F[px] = fx2{fx_prod(u, u), fx_prod(u, w)};
+            F[n + px] = fx2{fx_prod(w1, w1), fx_prod(vc, vc)};
           }
         }
         if (fprod && !split && !a.want_cfl) face(x, u, w, f1);
@@ -797,20 +801,25 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
       }
       auto forward = [&](int lines, int first) {  // pairs first.. of this level
         fx_fft(F, lines, P, nullptr);
-        for (int t = tid; t < lines * nkx; t += bd) {
-          const int p = t / nkx, k = t - p * nkx, pair = first + p;
-          const fx2 zk = F[p * n + P.pos_freq[k]], zc = F[p * n + P.pos_freq[k ? n - k : 0]];
+#pragma unroll 1
+        for (int p = 0; p < lines; ++p) {
+          const int pair = first + p;
           const bool centre = cprod && pair < 2;
-          const int S = (centre ? (pair == 0 ? S0 : S1) : S2) - P.shift;
+          // a pair's spectra come doubled out of the sums below
+          const int S = (centre ? (pair == 0 ? S0 : S1) : S2) - P.shift + 1;
           const bool nan = centre ? (bad || (pair == 1 && (badv || badpv))) : (bad || badp || badpv);
-          const FxOut out(nan ? 2047 : 0, S);
-          const size_t o = (size_t)(centre ? jj : jj - 1) * d.mp + rowoff + k;
+          const FxOut out(0, S);
+          const size_t o = (size_t)(centre ? jj : jj - 1) * d.mp + rowoff;
           const int r0 = centre ? 2 * pair : 4;
-          const i64 xk = zk.x >> 1, yk = zk.y >> 1, xc = zc.x >> 1, yc = zc.y >> 1;
-          double2 A = double2{out(xk + xc), out(yk - yc)}, B = double2{out(yk + yc), out(xc - xk)};
-          if (nan) A = B = double2{__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll)};
-          a.out[r0][o] = A;
-          a.out[r0 + 1][o] = B;
+          double2 *oa = a.out[r0] + o, *ob = a.out[r0 + 1] + o;
+          const fx2* f = F + p * n;
+          for (int k = tid; k < nkx; k += bd) {
+            const fx2 zk = f[P.pos_freq[k]], zc = f[P.pos_freq[k ? n - k : 0]];
+            double2 A = double2{out(zk.x + zc.x), out(zk.y - zc.y)}, B = double2{out(zk.y + zc.y), out(zc.x - zk.x)};
+            if (nan) A = B = double2{__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll)};
+            oa[k] = A;
+            ob[k] = B;
+          }
         }
         __syncthreads();
       };
@@ -820,11 +829,11 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
         if (split) {
           for (int x = tid; x < n; x += bd) {
             const fx2 z = Z[vu * n + x], zv = Z[n + x];
-            const i64 u = fx_shift(z.y, su), w = fx_shift(z.x, sw);
+            const i64 u = fx_shl(z.y, s0), w = fx_shl(z.x, s0);
             face(x, u, w, 0);
             pu[x] = u;
             pw[x] = w;
-            pv[x] = vface ? fx_shift(q == 0 ? zv.y : zv.x, sv) : 0;
+            pv[x] = vface ? fx_shl(q == 0 ? zv.y : zv.x, sv) : 0;
           }
           __syncthreads();
           forward(1, 2);
@@ -834,8 +843,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
         const int jn = j + lp;
         fetch(Z, jn, false, jn, 1, min(v_top, jn));
       }
-      Spu = Su;
-      Spw = Sw;
+      Sp = Sc;
       Spv = Sv;
       badp = bad;
       badpv = badv;
@@ -861,10 +869,21 @@ __global__ void __launch_bounds__(256) k_xprod(const __grid_constant__ ProdArgs<
   xprod_body(a, d, p, blockIdx.x, blockIdx.y);
 }
 
-__global__ void __launch_bounds__(256, 3) k_xprod_fx(const __grid_constant__ ProdArgs<double> a, const __grid_constant__ Dims d,
-                                                     const __grid_constant__ XPlan<double> p) {
-  xprod_body(a, d, p, blockIdx.x, blockIdx.y);
+// Threads at most, and registers: 80 a thread let an SM hold 24 warps, 96 (no spills) 20.  CTAs of 96 to 192 threads do
+// better with 96 (288 x 288 x 226, 128 threads: 4.1 ms against 4.6), the others with 80 (96 x 96 x 130, 64 threads: 0.44
+// against 0.46; 576 x 576 x 450, 224 threads: 34.0 against 37.2).
+constexpr int kFxThreads = 224;
+template <bool TWO>
+__global__ void __launch_bounds__(kFxThreads, 3) k_xprod_fx(const __grid_constant__ ProdArgs<double> a,
+                                                            const __grid_constant__ Dims d,
+                                                            const __grid_constant__ XPlan<double> p) {
+  xprod_body<TWO>(a, d, p, blockIdx.x, blockIdx.y);
 }
+__global__ void __maxnreg__(96) k_xprod_fx96(const __grid_constant__ ProdArgs<double> a, const __grid_constant__ Dims d,
+                                             const __grid_constant__ XPlan<double> p) {
+  xprod_body<true>(a, d, p, blockIdx.x, blockIdx.y);
+}
+__host__ __device__ constexpr bool xprod_wide(int threads) { return threads >= 96 && threads <= 192; }
 
 // ---- the FP32 product pass on two z rows per CTA --------------------------------------------------------
 // The same work as xprod_body for the rows 2 bx and 2 bx + 1, their transforms run in lockstep (fft_dit2):
@@ -1090,7 +1109,7 @@ __global__ void __launch_bounds__(256) k_xprod2(const __grid_constant__ ProdArgs
 template <typename R>
 int xprod_threads(const Dims& d, int threads) {
   threads = threads == 128 ? 128 : 256;
-  return sizeof(R) == 4 ? threads : std::min(threads, (3 * d.ngx / 8 + 31) / 32 * 32);
+  return sizeof(R) == 4 ? threads : std::min({threads, kFxThreads, (3 * d.ngx / 8 + 31) / 32 * 32});
 }
 
 template <typename R>
@@ -1117,7 +1136,7 @@ int xprod_ctas_per_sm(const Dims& d, int rows, int threads) {
   size_t smem;
   xprod_shape(a, d, &grid, &smem);
   threads = xprod_threads<R>(d, threads);
-  const int regs = sizeof(R) == 8 ? 80 : (rows == 2 ? 48 : 40);  // registers a thread of the three kernels
+  const int regs = sizeof(R) == 8 ? (xprod_wide(threads) ? 96 : 80) : (rows == 2 ? 48 : 40);  // of the kernels
   const int by_regs = 65536 / (regs * threads), by_smem = (int)(233472 / (smem + 1024 + 256));
   return std::max(1, std::min({32, 2048 / threads, by_regs, by_smem}));
 }
@@ -1135,7 +1154,12 @@ void launch_xprod(const ProdArgs<R>& a, const Dims& d, const XPlan<R>& p, cudaSt
     }
   }
   if constexpr (sizeof(R) == 4) k_xprod<<<grid, xprod_threads<R>(d, a.threads), sm, st>>>(a, d, p);
-  else k_xprod_fx<<<grid, xprod_threads<R>(d, a.threads), sm, st>>>(a, d, p);
+  else {
+    const int threads = xprod_threads<R>(d, a.threads);
+    if (xprod_levels(d.ngx) == 1) k_xprod_fx<false><<<grid, threads, sm, st>>>(a, d, p);
+    else if (xprod_wide(threads)) k_xprod_fx96<<<grid, threads, sm, st>>>(a, d, p);
+    else k_xprod_fx<true><<<grid, threads, sm, st>>>(a, d, p);
+  }
 }
 
 // Canopy forcing on one mixed row of one processed plane: x-inverse, solid
@@ -2276,12 +2300,18 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zfwd_batch(cons
   zfwd_body(D.jobs, D.d, D.p, D.tx, D.scale, q % D.gx, (q % gxy) / D.gx, q / gxy);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 6 : 3) k_xprod_batch(const __grid_constant__ Batch<XDesc<R>> b) {
+__global__ void __launch_bounds__(256, 6) k_xprod_batch(const __grid_constant__ Batch<XDesc<float>> b) {
   const int m = batch_member(b, blockIdx.x);
-  const XDesc<R>& D = b.desc[m];
+  const XDesc<float>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m];
   xprod_body(D.a, D.d, D.p, q % D.gx, q / D.gx);
+}
+template <bool TWO>
+__global__ void __launch_bounds__(kFxThreads, 3) k_xprod_fx_batch(const __grid_constant__ Batch<XDesc<double>> b) {
+  const int m = batch_member(b, blockIdx.x);
+  const XDesc<double>& D = b.desc[m];
+  const int q = blockIdx.x - b.start[m];
+  xprod_body<TWO>(D.a, D.d, D.p, q % D.gx, q / D.gx);
 }
 
 template <typename R>
@@ -2329,7 +2359,11 @@ void launch_zfwd_batch(const Batch<ZDesc<R>>& b, size_t smem, cudaStream_t st) {
 }
 template <typename R>
 void launch_xprod_batch(const Batch<XDesc<R>>& b, size_t smem, cudaStream_t st) {
-  if (b.n > 0 && b.start[b.n] > 0) k_xprod_batch<R><<<b.start[b.n], 256, smem, st>>>(b);
+  if (b.n <= 0 || b.start[b.n] <= 0) return;
+  // FP64: members of one shared-memory size are of one x length
+  if constexpr (sizeof(R) == 4) k_xprod_batch<<<b.start[b.n], 256, smem, st>>>(b);
+  else if (xprod_levels(b.desc[0].d.ngx) == 2) k_xprod_fx_batch<true><<<b.start[b.n], xprod_threads<R>(b.desc[0].d, 256), smem, st>>>(b);
+  else k_xprod_fx_batch<false><<<b.start[b.n], xprod_threads<R>(b.desc[0].d, 256), smem, st>>>(b);
 }
 template <typename R>
 void launch_xmask_batch(const Batch<MDesc<R>>& b, size_t smem, cudaStream_t st) {
@@ -2423,14 +2457,14 @@ cudaError_t configure_kernels() {
   int optin = 0;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  const cudaError_t r[22] = {allow_smem(k_vsolve, optin), allow_smem(k_psolve_tile, optin), allow_smem(k_vsolve_batch, optin),
+  const cudaError_t r[25] = {allow_smem(k_vsolve, optin), allow_smem(k_psolve_tile, optin), allow_smem(k_vsolve_batch, optin),
                              allow_smem(k_psolve_batch<true>, optin), allow_smem(k_xcond, optin), allow_smem(k_zinv<double>, optin), allow_smem(k_zinv<float>, optin),
                              allow_smem(k_zfwd<double>, optin), allow_smem(k_zfwd<float>, optin),
-                             allow_smem(k_xprod_fx, optin), allow_smem(k_xprod, optin), allow_smem(k_xprod2, optin),
+                             allow_smem(k_xprod_fx<true>, optin), allow_smem(k_xprod_fx<false>, optin), allow_smem(k_xprod_fx96, optin), allow_smem(k_xprod, optin), allow_smem(k_xprod2, optin),
                              allow_smem(k_xmask<double>, optin), allow_smem(k_xmask<float>, optin),
                              allow_smem(k_zinv_batch<double>, optin), allow_smem(k_zinv_batch<float>, optin),
                              allow_smem(k_zfwd_batch<double>, optin), allow_smem(k_zfwd_batch<float>, optin),
-                             allow_smem(k_xprod_batch<double>, optin), allow_smem(k_xprod_batch<float>, optin),
+                             allow_smem(k_xprod_fx_batch<true>, optin), allow_smem(k_xprod_fx_batch<false>, optin), allow_smem(k_xprod_batch, optin),
                              allow_smem(k_xmask_batch<double>, optin), allow_smem(k_xmask_batch<float>, optin)};
   for (cudaError_t x : r)
     if (x != cudaSuccess) return x;

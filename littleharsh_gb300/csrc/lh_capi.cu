@@ -407,6 +407,12 @@ XPlan<R> xplan(const lh_handle* h, const BandLaunch& B) {
   else return XPlan<R>{*B.qx, h->t.wcq, h->t.wfq};
 }
 
+template <typename R>
+MaskPlan<R> mask_plan(const lh_handle* h) {
+  if constexpr (sizeof(R) == 4) return MaskPlan<R>{h->ph.plan, h->rtw};
+  else return MaskPlan<R>{h->qx};
+}
+
 // The nonlinear term's plane work for one band: z-inverse of the levels the band's products need, products,
 // z-forward of the band's product planes, with the geometry and transforms of the band's planes.
 template <typename R>
@@ -595,7 +601,7 @@ int enqueue_substage(lh_handle* h, int k, int upto) {
     if (ib_args<R>(h, k, &zi, &m, &zf)) {
       launch_zinv<R>(zi, d, zplan<R>(h->pz.plan, h->qz), h->tx, st, h->zthreads);
       mark(h, K_IB_ZINV);
-      launch_xmask<R>(m, d, h->ph.plan, h->rtw, st);
+      launch_xmask<R>(m, d, mask_plan<R>(h), st);
       mark(h, K_IB_XMASK);
       launch_zfwd<R>(zf, d, zplan<R>(h->pz.plan, h->qz), h->tx, 1.0 / d.ngz, st, h->zthreads);
       mark(h, K_IB_ZFWD);
@@ -1407,7 +1413,7 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
         zi.push_back(Di); bi.push_back((int)(g.x * g.y * g.z)); si.push_back(sm);
         xmask_shape<R>(mk, h->d, &g, &sm);
         MDesc<R> Dm{};
-        Dm.a = mk; Dm.d = h->d; Dm.ph = h->ph.plan; Dm.rtw = h->rtw; Dm.gx = g.x; Dm.gy = g.y;
+        Dm.a = mk; Dm.d = h->d; Dm.p = mask_plan<R>(h); Dm.gx = g.x; Dm.gy = g.y;
         md.push_back(Dm); bm.push_back((int)(g.x * g.y)); sm_.push_back(sm);
         zpass_shape<R>(c, h->d, h->tx, &g, &sm);
         ZDesc<R> Df{};

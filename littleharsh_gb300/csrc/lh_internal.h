@@ -197,8 +197,16 @@ struct MaskArgs {
   int nplanes[3];
   double beta;
 };
+// What the canopy forcing transforms rows with: FP32 half-length plan and twiddles, or the fixed-point plan of FP64.
+template <typename R> struct MaskPlan {
+  FftPlan ph;
+  const double2* rtw;
+};
+template <> struct MaskPlan<double> {
+  FxPlan pf;
+};
 template <typename R>
-void launch_xmask(const MaskArgs<R>& a, const Dims& d, const FftPlan& ph, const double2* rtw, cudaStream_t st);
+void launch_xmask(const MaskArgs<R>& a, const Dims& d, const MaskPlan<R>& p, cudaStream_t st);
 
 struct AsmArgs {
   const double2 *u1, *u2, *u3, *p;
@@ -285,8 +293,7 @@ template <typename R>
 struct MDesc {                  // canopy forcing x pass
   MaskArgs<R> a;
   Dims d;
-  FftPlan ph;
-  const double2* rtw;
+  MaskPlan<R> p;
   int gx, gy;
 };
 struct ADesc {                  // right-hand-side assembly

@@ -1164,10 +1164,12 @@ void launch_xprod(const ProdArgs<R>& a, const Dims& d, const XPlan<R>& p, cudaSt
 
 // Canopy forcing on one mixed row of one processed plane: x-inverse, solid
 // points set to 0 (or -beta*Luy on the tip planes), x-forward.
-template <typename R>
-__device__ __forceinline__ void xmask_body(const MaskArgs<R>& a, const Dims& d, const FftPlan& ph,
-                                           const double2* __restrict__ rtw, int bx, int by) {
-  using T2 = cpx_t<R>;
+__device__ __forceinline__ void xmask_body(const MaskArgs<float>& a, const Dims& d, const MaskPlan<float>& p, int bx,
+                                           int by) {
+  using R = float;
+  using T2 = float2;
+  const FftPlan& ph = p.ph;
+  const double2* __restrict__ rtw = p.rtw;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ngx = d.ngx, h = ngx / 2, hp = h + 1;
   T2* F = reinterpret_cast<T2*>(smraw);
@@ -1209,27 +1211,162 @@ __device__ __forceinline__ void xmask_body(const MaskArgs<R>& a, const Dims& d, 
   x_forward_packed<R>(1, F, hp, rows, d, ph, rtw);
 }
 
+// FP64: two z rows of a plane as one complex line in 64-bit fixed point (lh_fxfft.cuh).  The rows come out of the inverse
+// transform on one scale and are masked on one of their own each, two bits below a line's range.  On the tip planes the
+// Laplacian's rows are transformed first and leave their values at the solid points; the field's then fill the others, all
+// on the coarser of the two scales.  A row without solid points takes no part: its partner is paired with zeros.
+//
+// Bound by instruction issue on the integer pipes, on small grids by latency; FP64 butterflies on half-length real rows
+// kept the FP64 pipe busy.  A step of the 576 x 576 x 450 grid: 4.91 -> 1.52 ms; 288 x 288 x 226 0.42 -> 0.18,
+// 96 x 96 x 130 0.113 -> 0.078, 48 x 48 x 66 0.051 -> 0.050.
+struct FxMask {            // line 0: the field, line 1: its Laplacian
+  unsigned e[2], sum[2], bits[4];
+};
+__device__ __forceinline__ void xmask_body(const MaskArgs<double>& a, const Dims& d, const MaskPlan<double>& plan, int bx,
+                                           int by) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ FxMask red;
+  const FxPlan& P = plan.pf;
+  const int n = d.ngx, nkx = d.nkx, tid = threadIdx.x, bd = blockDim.x;
+  fx2 *Z = reinterpret_cast<fx2*>(smraw), *F = Z + n;
+  const int kz = 2 * bx;
+  const bool second = kz + 1 < d.ngz;
+  int pl = by, f = 0;
+  while (f < 2 && pl >= a.nplanes[f]) { pl -= a.nplanes[f]; ++f; }
+  double2* const row = a.mix + (size_t)by * d.mp + (size_t)kz * nkx;
+  const int tip = a.tipslot[f][pl];
+  const uint8_t* const m0 = a.mask[f] + ((size_t)pl * d.ngz + kz) * n;
+  const uint8_t* const m1 = m0 + (second ? n : 0);
+  for (int i = tid; i < (int)(sizeof(FxMask) / 4); i += bd) reinterpret_cast<unsigned*>(&red)[i] = 0;
+  // a row without solid points is unchanged by the forcing: its x round trip only drops the imaginary
+  // part of its kx = 0 value (the real inverse ignores it), so that is all it needs
+  int any0 = 0, any1 = 0;
+  for (int x = tid; x < n; x += bd) {
+    any0 |= m0[x];
+    any1 |= m1[x];
+  }
+  const bool on0 = __syncthreads_or(any0), on1 = __syncthreads_or(any1) && second;
+  if (tid == 0) {
+    if (!on0) row[0].y = 0.0;
+    if (second && !on1) row[nkx].y = 0.0;
+  }
+  if (!on0 && !on1) return;
+
+  // rows ra, ra + nkx times mul to a transformed line in Z
+  auto inverse = [&](const double2* ra, double mul, int v) {
+    auto value = [&](int q, int k) {
+      double2 r = (q == 0 ? on0 : on1) ? ra[q * nkx + k] : double2{0.0, 0.0};
+      if (v) r = double2{mul * r.x, mul * r.y};
+      if (k == 0) r.y = 0.0;
+      return r;
+    };
+    unsigned m = 0;
+    for (int k = tid; k < nkx; k += bd) m = max(m, max(fx_hi(value(0, k)), fx_hi(value(1, k))));
+    fx_reduce_max(m, &red.e[v]);
+    __syncthreads();
+    const FxIn in((int)(red.e[v] >> 20) + 1);  // one bit of room: a line's values are sums of two rows'
+    unsigned s = 0;
+    for (int k = tid; k < nkx; k += bd) {
+      const double2 A = value(0, k), B = value(1, k);
+      const i64 ax = in(A.x), ay = in(A.y), bx2 = in(B.x), by2 = in(B.y);
+      // a + i b at k, its mirror at n - k.  Parts exchanged: an inverse transform
+      const fx2 p = fx2{ay + bx2, ax - by2}, q = fx2{bx2 - ay, ax + by2};
+      Z[P.pos_sample[k]] = p;
+      s += fx_mag(p.x) + fx_mag(p.y);
+      if (k) {
+        Z[P.pos_sample[n - k]] = q;
+        s += fx_mag(q.x) + fx_mag(q.y);
+      }
+    }
+    for (int k = nkx + tid; k <= n - nkx; k += bd) Z[P.pos_sample[k]] = fx2{0, 0};
+    fx_reduce_add(s, &red.sum[v]);
+    __syncthreads();
+    fx_fft(Z, 1, P, &red.sum[v]);
+    unsigned o0 = 0, o1 = 0;
+    for (int x = tid; x < n; x += bd) {
+      const fx2 z = Z[x];
+      o0 |= fx_bits(z.y);
+      o1 |= fx_bits(z.x);
+    }
+    fx_reduce_or(o0, &red.bits[2 * v]);
+    fx_reduce_or(o1, &red.bits[2 * v + 1]);
+    __syncthreads();
+  };
+  // the left shift (right if negative) that brings row q of line v below 2^58, and the row's scale after it
+  auto room = [&](int v, int q) { return __clz((int)red.bits[2 * v + q]) - 6; };
+  auto scale = [&](int v, int q) {
+    return fx_scale((int)(red.e[v] >> 20) + 1) - fx_inv_shift(red.sum[v], P.shift) + room(v, q);
+  };
+  auto shifted = [](i64 x, int s) { return s >= 0 ? fx_shl(x, s) : x >> -s; };
+  auto solid = [&](const uint8_t* m, int x) { return m[P.freq_pos[x]] != 0; };
+
+  if (tip >= 0) {
+    inverse(a.lymix + (size_t)tip * d.mp + (size_t)kz * nkx, -a.beta, 1);
+    const int s0 = room(1, 0), s1 = room(1, 1);
+    for (int x = tid; x < n; x += bd) {
+      const fx2 z = Z[x];
+      F[P.turn[x]] = fx2{solid(m0, x) ? shifted(z.y, s0) : 0, solid(m1, x) ? shifted(z.x, s1) : 0};
+    }
+    __syncthreads();
+  }
+  inverse(row, 1.0, 0);
+  int S0 = scale(0, 0), S1 = scale(0, 1);
+  {
+    const int s0 = room(0, 0), s1 = room(0, 1);
+    int d0 = 0, d1 = 0, l0 = 0, l1 = 0;  // from the field's and the Laplacian's scales to the coarser
+    if (tip >= 0) {
+      const int L0 = scale(1, 0), L1 = scale(1, 1), T0 = min(S0, L0), T1 = min(S1, L1);
+      d0 = min(S0 - T0, 63); d1 = min(S1 - T1, 63); l0 = min(L0 - T0, 63); l1 = min(L1 - T1, 63);
+      S0 = T0; S1 = T1;
+    }
+    for (int x = tid; x < n; x += bd) {
+      const fx2 z = Z[x];
+      const int px = P.turn[x];
+      const fx2 l = tip >= 0 ? F[px] : fx2{0, 0};
+      F[px] = fx2{solid(m0, x) ? l.x >> l0 : shifted(z.y, s0) >> d0, solid(m1, x) ? l.y >> l1 : shifted(z.x, s1) >> d1};
+    }
+  }
+  __syncthreads();
+  fx_fft(F, 1, P, nullptr);
+  const bool nan = max(red.e[0], red.e[1]) >= 0x7ff00000u;
+  const double norm = nan ? __longlong_as_double(0x7ff8000000000000ll) : 1.0 / n;
+  const FxOut out0(0, S0 - P.shift + 1), out1(0, S1 - P.shift + 1);  // the sums below double a spectrum
+  for (int k = tid; k < nkx; k += bd) {
+    const fx2 zk = F[P.pos_freq[k]], zc = F[P.pos_freq[k ? n - k : 0]];
+    if (on0) row[k] = double2{norm * out0(zk.x + zc.x), k ? norm * out0(zk.y - zc.y) : 0.0};
+    if (on1) row[nkx + k] = double2{norm * out1(zk.y + zc.y), k ? norm * out1(zc.x - zk.x) : 0.0};
+  }
+}
+
+// Threads of a CTA: FP32 128; FP64 about one per item of its line's radix-8 passes.
 template <typename R>
-__global__ void __launch_bounds__(128) k_xmask(const __grid_constant__ MaskArgs<R> a, const __grid_constant__ Dims d,
-                                               const __grid_constant__ FftPlan ph, const double2* __restrict__ rtw) {
-  xmask_body<R>(a, d, ph, rtw, blockIdx.x, blockIdx.y);
+__host__ __device__ __forceinline__ int xmask_threads(int ngx) {
+  return sizeof(R) == 4 ? 128 : min(128, (ngx / 8 + 31) / 32 * 32);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 1 : 6) k_xmask(const __grid_constant__ MaskArgs<R> a,
+                                                                       const __grid_constant__ Dims d,
+                                                                       const __grid_constant__ MaskPlan<R> p) {
+  xmask_body(a, d, p, blockIdx.x, blockIdx.y);
 }
 
 template <typename R>
 void xmask_shape(const MaskArgs<R>& a, const Dims& d, dim3* grid, size_t* smem) {
   const int tot = a.nplanes[0] + a.nplanes[1] + a.nplanes[2];
-  *grid = tot == 0 ? dim3(0, 0, 0) : dim3(d.ngz, tot);
+  *grid = tot == 0 ? dim3(0, 0, 0) : dim3(sizeof(R) == 4 ? d.ngz : (d.ngz + 1) / 2, tot);
   const int hp = d.ngx / 2 + 1;
-  *smem = sizeof(cpx_t<R>) * sx_elems<R>(2 * (size_t)hp) + sizeof(R) * 2 * (size_t)d.ngx;
+  *smem = sizeof(R) == 4 ? sizeof(cpx_t<R>) * sx_elems<R>(2 * (size_t)hp) + sizeof(R) * 2 * (size_t)d.ngx
+                         : sizeof(fx2) * 2 * (size_t)d.ngx;
 }
 
 template <typename R>
-void launch_xmask(const MaskArgs<R>& a, const Dims& d, const FftPlan& ph, const double2* rtw, cudaStream_t st) {
+void launch_xmask(const MaskArgs<R>& a, const Dims& d, const MaskPlan<R>& p, cudaStream_t st) {
   dim3 grid;
   size_t sm;
   xmask_shape(a, d, &grid, &sm);
   if (grid.x == 0) return;
-  k_xmask<R><<<grid, 128, sm, st>>>(a, d, ph, rtw);
+  k_xmask<R><<<grid, xmask_threads<R>(d.ngx), sm, st>>>(a, d, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -2315,11 +2452,11 @@ __global__ void __launch_bounds__(kFxThreads, 3) k_xprod_fx_batch(const __grid_c
 }
 
 template <typename R>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 9) k_xmask_batch(const __grid_constant__ Batch<MDesc<R>> b) {
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 6) k_xmask_batch(const __grid_constant__ Batch<MDesc<R>> b) {
   const int m = batch_member(b, blockIdx.x);
   const MDesc<R>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m];
-  xmask_body<R>(D.a, D.d, D.ph, D.rtw, q % D.gx, q / D.gx);
+  xmask_body(D.a, D.d, D.p, q % D.gx, q / D.gx);
 }
 
 template <typename P>
@@ -2367,7 +2504,8 @@ void launch_xprod_batch(const Batch<XDesc<R>>& b, size_t smem, cudaStream_t st) 
 }
 template <typename R>
 void launch_xmask_batch(const Batch<MDesc<R>>& b, size_t smem, cudaStream_t st) {
-  if (b.n > 0 && b.start[b.n] > 0) k_xmask_batch<R><<<b.start[b.n], 128, smem, st>>>(b);
+  // members of one shared-memory size are of one x length
+  if (b.n > 0 && b.start[b.n] > 0) k_xmask_batch<R><<<b.start[b.n], xmask_threads<R>(b.desc[0].d.ngx), smem, st>>>(b);
 }
 void launch_assemble_batch(const Batch<ADesc>& b, bool fp32_products, cudaStream_t st) {
   if (b.n <= 0 || b.start[b.n] <= 0) return;
@@ -2478,8 +2616,8 @@ template void launch_zfwd<double>(const ZJobs<double>&, const Dims&, const ZPlan
 template void launch_zfwd<float>(const ZJobs<float>&, const Dims&, const ZPlan<float>&, int, double, cudaStream_t, int);
 template void launch_xprod<double>(const ProdArgs<double>&, const Dims&, const XPlan<double>&, cudaStream_t);
 template void launch_xprod<float>(const ProdArgs<float>&, const Dims&, const XPlan<float>&, cudaStream_t);
-template void launch_xmask<double>(const MaskArgs<double>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
-template void launch_xmask<float>(const MaskArgs<float>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
+template void launch_xmask<double>(const MaskArgs<double>&, const Dims&, const MaskPlan<double>&, cudaStream_t);
+template void launch_xmask<float>(const MaskArgs<float>&, const Dims&, const MaskPlan<float>&, cudaStream_t);
 template void zpass_shape<double>(const ZJobs<double>&, const Dims&, int, dim3*, size_t*);
 template int zpass_tile<double>(int);
 template int zpass_tile<float>(int);

@@ -124,6 +124,31 @@ def test_lengths_against_the_oracle(oracle_mod, cfg):
     assert abs(s.cfl_dt(0.5) - o.cfl_dt(0.5)) < 1e-12 * dt
 
 
+# canopy rows in pairs: an odd row left over, pairs with one or no solid row, one post, lines of one and of several warps
+CANOPY = [dict(ngalx=16, ngalz=9, ntilex=2, ntilez=1, dstx=1, dstz=1), dict(ngalx=54, ngalz=27, ntilex=3, ntilez=3, dstx=5, dstz=2),
+          dict(ngalx=128, ngalz=16, ntilex=1, ntilez=1, dstx=1, dstz=1), dict(ngalx=486, ngalz=18, ntilex=6, ntilez=2),
+          dict(ngalx=1152, ngalz=12, ntilex=4, ntilez=4)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfg", [dict(SMALL, **c) for c in CANOPY], ids=[f"{c['ngalx']}x{c['ngalz']}" for c in CANOPY])
+def test_canopy_rows_against_the_oracle(oracle_mod, cfg):
+    """Right-hand sides after the canopy forcing of the first substage, to the tolerance of the other substage comparisons."""
+    import littleharsh_gb300 as lh
+    o = oracle_mod.Oracle(**cfg)
+    f = projected_ic(o, seed=3)
+    dt = o.cfl_dt(0.5)
+    o.set_fields(*f)
+    o.set_scalars(0.0, dt, 0.0, o.flowrate())
+    s = lh.Solver(lh.Config(**cfg))
+    s.set_fields(*f)
+    s.set_time(0.0, dt, 0.0)
+    o.substage(1, 2)
+    s.substage(1, 2)
+    for a, b in zip(s.get_rhs(), o.get_rhs()):
+        assert rel_l2(a, b) < 1e-11
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("banded", [False, True], ids=["one", "bands"])
 def test_chunks_of_levels_keep_results(monkeypatch, banded):

@@ -1390,7 +1390,7 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
       for (lh_handle* h : hs) {
         ADesc D{};
         D.a = asm_args<R>(h, k); D.d = h->d; D.t = h->t;
-        D.gx = (h->d.np + 255) / 256; D.gy = h->d.nyu;
+        assemble_shape(h->d, sizeof(R) == 4, &D.gx, &D.gy, &D.levels);
         ad.push_back(D);
         blocks.push_back(D.gx * D.gy);
       }

@@ -222,6 +222,7 @@ struct AsmArgs {
   int k;                     // substage index 0..2 (selects 1/axz)
 };
 void launch_assemble(const AsmArgs& a, const Dims& d, const Tables& t, cudaStream_t st);
+void assemble_shape(const Dims& d, bool fp32_products, int* gx, int* gy, int* levels);
 
 void launch_vsolve(double2* r1, double2* r2, double2* r3, double2* u1, double2* u2, double2* u3,
                    const Dims& d, const Tables& t, int k, cudaStream_t st);
@@ -300,7 +301,7 @@ struct ADesc {                  // right-hand-side assembly
   AsmArgs a;
   Dims d;
   Tables t;
-  int gx, gy;
+  int gx, gy, levels;
 };
 struct VDesc {                  // velocity Thomas sweeps
   double2 *r1, *r2, *r3, *u1, *u2, *u3;

@@ -1376,28 +1376,17 @@ void launch_xmask(const MaskArgs<R>& a, const Dims& d, const MaskPlan<R>& p, cud
 __device__ __forceinline__ double2 ld(const double2* p) { return __ldg(p); }
 __device__ __forceinline__ float2 ld(const float2* p) { return __ldg(p); }
 
-// product spectra q = 0..5 (uu, uw, ww, vv, uv, vw) of the assembly's precision
-template <typename P> __device__ __forceinline__ const P* prod(const AsmArgs& a, int q);
-template <> __device__ __forceinline__ const double2* prod<double2>(const AsmArgs& a, int q) { return a.p64[q]; }
-template <> __device__ __forceinline__ const float2* prod<float2>(const AsmArgs& a, int q) { return a.p32[q]; }
-
-// The nonlinear term from the product spectra: (-kx A.y - kz B.y) + c (D1.x - D0.x) and its imaginary
-// partner (d/dx, d/dz of the in-plane products, d/dy of the face products).  The mixed form's FP32
-// spectra are combined in FP32 and only the result is widened.
-__device__ __forceinline__ double2 nterm(double2 A, double2 B, double2 D1, double2 D0, double kx, double kz, double c) {
-  return double2{(-kx * A.y - kz * B.y) + c * (D1.x - D0.x), (kx * A.x + kz * B.x) + c * (D1.y - D0.y)};
-}
+// The mixed form's nonlinear term from the product spectra: (-kx A.y - kz B.y) + c (D1.x - D0.x) and its imaginary
+// partner (d/dx, d/dz of the in-plane products, d/dy of the face products), combined in FP32 and widened.
 __device__ __forceinline__ double2 nterm(float2 A, float2 B, float2 D1, float2 D0, float fx, float fz, float fc) {
   return double2{(double)((-fx * A.y - fz * B.y) + fc * (D1.x - D0.x)),
                  (double)((fx * A.x + fz * B.x) + fc * (D1.y - D0.y))};
 }
-// the wavenumbers and the y metric in the precision the product spectra are combined in
-template <typename P> __device__ __forceinline__ auto wnum(const double* d, const float* f, int i) {
-  if constexpr (sizeof(P) == sizeof(float2)) return __ldg(f + i);
-  else return d[i];
-}
 
-template <typename P>
+// 64 threads a CTA: with 256, three launches of the 96 x 96 x 130 grid take 0.162 ms instead of 0.144 in the mixed form, a
+// tenth more in FP64 too, and half as much again on 48 x 48 x 66; the largest grids 2 % less in FP64.
+constexpr int kAsmThreads = 64;
+
 __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, const Tables& t, int bx, int by) {
   const int col = bx * blockDim.x + threadIdx.x;
   if (col >= d.np) return;
@@ -1438,13 +1427,13 @@ __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, c
       double rx = a.C1 * L_x + a.C2 * nold.x + (a.d * kf) * pc.y;
       double ry = a.C1 * L_y + a.C2 * nold.y + -(a.d * kf) * pc.x;
       if (f == 0 && col == 0) rx = rx + (-a.d * a.sc->mpgx);
-      const P A = ld(prod<P>(a, f == 0 ? 0 : 1) + c0);
-      const P B = ld(prod<P>(a, f == 0 ? 1 : 2) + c0);
-      const P* D = prod<P>(a, f == 0 ? 4 : 5);
+      const float2 A = ld(a.p32[f == 0 ? 0 : 1] + c0);
+      const float2 B = ld(a.p32[f == 0 ? 1 : 2] + c0);
+      const float2* D = a.p32[f == 0 ? 4 : 5];
       // a short column's product is zero on the middle band's planes (they hold only long modes)
-      const P D1 = (lng || !coarse_v(d, jj)) ? ld(D + f1) : P{0, 0};
-      const P D0 = (lng || !coarse_v(d, jj - 1)) ? ld(D + f0) : P{0, 0};
-      const double2 N = nterm(A, B, D1, D0, wnum<P>(t.kx, t.kxf, i), wnum<P>(t.kz, t.kzf, kk), wnum<P>(t.cu, t.cuf, jj));
+      const float2 D1 = (lng || !coarse_v(d, jj)) ? ld(D + f1) : float2{0, 0};
+      const float2 D0 = (lng || !coarse_v(d, jj - 1)) ? ld(D + f0) : float2{0, 0};
+      const double2 N = nterm(A, B, D1, D0, __ldg(t.kxf + i), __ldg(t.kzf + kk), __ldg(t.cuf + jj));
       const double nr = N.x, ni = N.y;
       (f == 0 ? a.n1 : a.n3)[c0] = double2{nr, ni};
       rx = rx - a.g * nr;
@@ -1473,9 +1462,9 @@ __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, c
       const double2 nold = a.C2 != 0.0 ? a.n2[c0] : double2{0.0, 0.0};
       double rx = a.C1 * L_x + a.C2 * nold.x + C3 * (p1.x - p0.x);
       double ry = a.C1 * L_y + a.C2 * nold.y + C3 * (p1.y - p0.y);
-      const P A = ld(prod<P>(a, 4) + c0), B = ld(prod<P>(a, 5) + c0);
-      const P V1 = ld(prod<P>(a, 3) + c0 + np), V0 = ld(prod<P>(a, 3) + c0);
-      const double2 N = nterm(A, B, V1, V0, wnum<P>(t.kx, t.kxf, i), wnum<P>(t.kz, t.kzf, kk), wnum<P>(t.cv, t.cvf, jj));
+      const float2 A = ld(a.p32[4] + c0), B = ld(a.p32[5] + c0);
+      const float2 V1 = ld(a.p32[3] + c0 + np), V0 = ld(a.p32[3] + c0);
+      const double2 N = nterm(A, B, V1, V0, __ldg(t.kxf + i), __ldg(t.kzf + kk), __ldg(t.cvf + jj));
       const double nr = N.x, ni = N.y;
       a.n2[c0] = double2{nr, ni};
       rx = rx - a.g * nr;
@@ -1490,16 +1479,138 @@ __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, c
   }
 }
 
-template <typename P>
-__global__ void __launch_bounds__(256) k_assemble(const __grid_constant__ AsmArgs a, const __grid_constant__ Dims d,
-                                                  const __grid_constant__ Tables t) {
-  assemble_body<P>(a, d, t, blockIdx.x, blockIdx.y);
+// FP64: several levels of a column a thread.  The kernel is bound by FP64 instructions (a warp's takes 64 clocks of its
+// quarter of the SM; the pipe is 89 % busy, memory a quarter), so what a level's or a column's points share is formed once:
+// the metric times dt C1 by one thread a CTA, the wavenumbers times dt d once a column.  What is left is 12 instructions a
+// real or imaginary part of u1 and u3 and 13 of u2, 77 a point against 87 with a product for each factor.  u0 is added last
+// and not within its factor 1 + dt C1 (k2 + a2): that takes six instructions less (14.8 ms), but its rounding doubles the
+// error of p.  Three launches, before and after: 576 x 576 x 450 18.0 -> 16.1 ms, 288 x 288 x 226 2.28 -> 2.06, 96 x 96 x
+// 130 0.179 -> 0.158, 48 x 48 x 66 0.061 -> 0.038.
+constexpr int kAsmLevels = 4;  // at most
+struct AsmLevel {
+  double um, u0, up, cu;      // dt C1 times the u grid's second derivative, d/dy at centres
+  double vm, v0, vp, cv, pv;  // the same at faces; pv = -dt d cv
+};
+__device__ __forceinline__ void assemble_levels(const AsmArgs& a, const Dims& d, const Tables& t, int levels, int bx,
+                                                int by) {
+  __shared__ AsmLevel level[kAsmLevels];
+  const int j0 = by * levels, j1 = min(j0 + levels, d.nyu);
+  for (int e = threadIdx.x; e < 9 * levels; e += blockDim.x) {
+    const int q = e / 9, i = e - 9 * q, jj = min(j0 + q, i < 4 ? d.nyu - 1 : d.nyv - 1);
+    const double c = i == 3 ? t.cu[jj] : (i >= 7 ? t.cv[jj] : (i < 3 ? t.d2u[3 * jj + i] : t.d2v[3 * jj + i - 4]));
+    const double f = i == 3 || i == 7 ? 1.0 : (i == 8 ? -a.dt * a.d : a.dt * a.C1);
+    reinterpret_cast<double*>(&level[q])[i] = f * c;
+  }
+  __syncthreads();
+  const int np = d.np, col = bx * blockDim.x + threadIdx.x;
+  if (col >= np) return;
+  const int i = col % d.nkx, kk = col / d.nkx;
+  const double kx = t.kx[i], kz = t.kz[kk];
+  const double dtC2 = a.dt * a.C2, dtg = a.dt * a.g, dtd = a.dt * a.d;
+  const double k2 = (a.dt * a.C1) * (t.k2x[i] + t.k2z[kk]), px = dtd * kx, pz = dtd * kz;
+  // 1/axz of LUsolU/LUsolV (tridLU_3D_IB.f90:489,93) for this substage: a multiply instead of a
+  // division, which costs ~10 FP64 instructions on a part with little FP64 throughput
+  const double iaxz = t.iaxz[(size_t)a.k * np + col];
+  const bool lng = is_long(d, i, kk);
+  // the first substage's zeta is 0 (start.f90:413-427): its old nonlinear term is not read, so a term left
+  // from earlier fields (even a non-finite one) does not enter
+  const bool old = a.C2 != 0.0;
+#pragma unroll 1
+  for (int jj = j0; jj < j1; ++jj) {
+    const AsmLevel& L = level[jj - j0];
+    const size_t c0 = (size_t)jj * np + col;
+    // u1 and u3 on centre jj
+    const int lu = lev_u(d, lng, jj);
+    if (lu != 1) {  // the column's end rows, or outside a short column
+      a.r1[c0] = double2{0.0, 0.0};
+      a.r3[c0] = double2{0.0, 0.0};
+      if (lu == 0 || (jj != 0 && jj != d.nyu - 1)) {
+        a.n1[c0] = double2{0.0, 0.0};
+        a.n3[c0] = double2{0.0, 0.0};
+      }
+    } else {
+      const double z = L.u0 + k2;
+      const double2 pc = ld(a.p + c0 - np);
+      // a short column's product is zero on the middle band's planes (they hold only long modes)
+      const bool in1 = lng || !coarse_v(d, jj), in0 = lng || !coarse_v(d, jj - 1);
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        const double2* u = f == 0 ? a.u1 : a.u3;
+        double2* n = f == 0 ? a.n1 : a.n3;
+        const double2 um = ld(u + c0 - np), u0 = ld(u + c0), up = ld(u + c0 + np);
+        const double2 nold = old ? n[c0] : double2{0.0, 0.0};
+        const double2 A = ld(a.p64[f == 0 ? 0 : 1] + c0), B = ld(a.p64[f == 0 ? 1 : 2] + c0);
+        const double2* D = a.p64[f == 0 ? 4 : 5] + c0;
+        const double2 D1 = in1 ? ld(D) : double2{0.0, 0.0}, D0 = in0 ? ld(D - np) : double2{0.0, 0.0};
+        const double pk = f == 0 ? px : pz;
+        double rx = fma(L.um, um.x, fma(z, u0.x, L.up * up.x)), ry = fma(L.um, um.y, fma(z, u0.y, L.up * up.y));
+        rx = fma(pk, pc.y, fma(dtC2, nold.x, rx));
+        ry = fma(-pk, pc.x, fma(dtC2, nold.y, ry));
+        if (f == 0 && col == 0) rx = fma(-dtd, a.sc->mpgx, rx);
+        // d/dx, d/dz of the in-plane products, d/dy of the face product
+        const double nr = fma(L.cu, D1.x - D0.x, -fma(kx, A.y, kz * B.y));
+        const double ni = fma(L.cu, D1.y - D0.y, fma(kx, A.x, kz * B.x));
+        n[c0] = double2{nr, ni};
+        (f == 0 ? a.r1 : a.r3)[c0] = double2{(u0.x + fma(-dtg, nr, rx)) * iaxz, (u0.y + fma(-dtg, ni, ry)) * iaxz};
+        if (jj == a.tipu[0] || jj == a.tipu[1]) {
+          const double a1 = t.d2u[3 * jj], a2 = t.d2u[3 * jj + 1], a3 = t.d2u[3 * jj + 2];
+          a.lytip[(size_t)(2 * f + (jj == a.tipu[0] ? 0 : 1)) * np + col] =
+              double2{a1 * um.x + a2 * u0.x + a3 * up.x, a1 * um.y + a2 * u0.y + a3 * up.y};
+        }
+      }
+    }
+    // u2 on face jj
+    if (jj > d.nyv - 1) continue;
+    const int lv = lev_v(d, lng, jj);
+    if (lv != 1) {
+      a.r2[c0] = double2{0.0, 0.0};
+      if (lv == 0 || (jj != 0 && jj != d.nyv - 1)) a.n2[c0] = double2{0.0, 0.0};
+    } else {
+      const double z = L.v0 + k2;
+      const double2 um = ld(a.u2 + c0 - np), u0 = ld(a.u2 + c0), up = ld(a.u2 + c0 + np);
+      const double2 p0 = ld(a.p + c0 - np), p1 = ld(a.p + c0);
+      const double2 nold = old ? a.n2[c0] : double2{0.0, 0.0};
+      const double2 A = ld(a.p64[4] + c0), B = ld(a.p64[5] + c0), V1 = ld(a.p64[3] + c0 + np), V0 = ld(a.p64[3] + c0);
+      double rx = fma(L.vm, um.x, fma(z, u0.x, L.vp * up.x)), ry = fma(L.vm, um.y, fma(z, u0.y, L.vp * up.y));
+      rx = fma(L.pv, p1.x - p0.x, fma(dtC2, nold.x, rx));
+      ry = fma(L.pv, p1.y - p0.y, fma(dtC2, nold.y, ry));
+      const double nr = fma(L.cv, V1.x - V0.x, -fma(kx, A.y, kz * B.y));
+      const double ni = fma(L.cv, V1.y - V0.y, fma(kx, A.x, kz * B.x));
+      a.n2[c0] = double2{nr, ni};
+      a.r2[c0] = double2{(u0.x + fma(-dtg, nr, rx)) * iaxz, (u0.y + fma(-dtg, ni, ry)) * iaxz};
+      if (jj == a.tipv[0] || jj == a.tipv[1]) {
+        const double a1 = t.d2v[3 * jj], a2 = t.d2v[3 * jj + 1], a3 = t.d2v[3 * jj + 2];
+        a.lytip[(size_t)(4 + (jj == a.tipv[0] ? 0 : 1)) * np + col] =
+            double2{a1 * um.x + a2 * u0.x + a3 * up.x, a1 * um.y + a2 * u0.y + a3 * up.y};
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kAsmThreads) k_assemble(const __grid_constant__ AsmArgs a, const __grid_constant__ Dims d,
+                                                          const __grid_constant__ Tables t) {
+  assemble_body(a, d, t, blockIdx.x, blockIdx.y);
+}
+__global__ void __launch_bounds__(kAsmThreads) k_assemble64(const __grid_constant__ AsmArgs a, const __grid_constant__ Dims d,
+                                                            const __grid_constant__ Tables t, int levels) {
+  assemble_levels(a, d, t, levels, blockIdx.x, blockIdx.y);
+}
+
+// Levels a CTA: more share what a column's points share, fewer leave more CTAs.  Three launches, ms, 1 / 2 / 4 levels:
+// 48 x 48 x 66 (34000 points) 0.039 / 0.045 / 0.068, 96 x 96 x 130 (266000) 0.162 / 0.158 / 0.172, 288 x 288 x 226 (4.2
+// million) 2.18 / 2.09 / 2.06, 576 x 576 x 450 17.1 / 16.4 / 16.1.
+void assemble_shape(const Dims& d, bool fp32_products, int* gx, int* gy, int* levels) {
+  const long long points = (long long)d.np * d.nyu;
+  *gx = (d.np + kAsmThreads - 1) / kAsmThreads;
+  *levels = fp32_products ? 1 : points < 100000 ? 1 : (points < 1000000 ? 2 : kAsmLevels);
+  *gy = (d.nyu + *levels - 1) / *levels;
 }
 
 void launch_assemble(const AsmArgs& a, const Dims& d, const Tables& t, cudaStream_t st) {
-  dim3 grid((d.np + 255) / 256, d.nyu);
-  if (a.p32[0]) k_assemble<float2><<<grid, 256, 0, st>>>(a, d, t);
-  else k_assemble<double2><<<grid, 256, 0, st>>>(a, d, t);
+  int gx, gy, levels;
+  assemble_shape(d, a.p32[0] != nullptr, &gx, &gy, &levels);
+  if (a.p32[0]) k_assemble<<<dim3(gx, gy), kAsmThreads, 0, st>>>(a, d, t);
+  else k_assemble64<<<dim3(gx, gy), kAsmThreads, 0, st>>>(a, d, t, levels);
 }
 
 // The column solves take two threads per column, one for the real parts and one for the imaginary ones (neighbouring
@@ -2459,12 +2570,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 6) k_xmask_batch(co
   xmask_body(D.a, D.d, D.p, q % D.gx, q / D.gx);
 }
 
-template <typename P>
-__global__ void __launch_bounds__(256, 3) k_assemble_batch(const __grid_constant__ Batch<ADesc> b) {
+template <bool FP32>
+__global__ void __launch_bounds__(kAsmThreads, 768 / kAsmThreads) k_assemble_batch(const __grid_constant__ Batch<ADesc> b) {
   const int m = batch_member(b, blockIdx.x);
   const ADesc& D = b.desc[m];
   const int q = blockIdx.x - b.start[m];
-  assemble_body<P>(D.a, D.d, D.t, q % D.gx, q / D.gx);
+  if constexpr (FP32) assemble_body(D.a, D.d, D.t, q % D.gx, q / D.gx);
+  else assemble_levels(D.a, D.d, D.t, D.levels, q % D.gx, q / D.gx);
 }
 
 __global__ void __launch_bounds__(kTileThreads, 5) k_vsolve_batch(const __grid_constant__ Batch<VDesc> b) {
@@ -2509,8 +2621,8 @@ void launch_xmask_batch(const Batch<MDesc<R>>& b, size_t smem, cudaStream_t st) 
 }
 void launch_assemble_batch(const Batch<ADesc>& b, bool fp32_products, cudaStream_t st) {
   if (b.n <= 0 || b.start[b.n] <= 0) return;
-  if (fp32_products) k_assemble_batch<float2><<<b.start[b.n], 256, 0, st>>>(b);
-  else k_assemble_batch<double2><<<b.start[b.n], 256, 0, st>>>(b);
+  if (fp32_products) k_assemble_batch<true><<<b.start[b.n], kAsmThreads, 0, st>>>(b);
+  else k_assemble_batch<false><<<b.start[b.n], kAsmThreads, 0, st>>>(b);
 }
 void launch_vsolve_batch(const Batch<VDesc>& b, size_t smem, cudaStream_t st) {
   if (b.n > 0 && b.start[b.n] > 0) k_vsolve_batch<<<b.start[b.n], smem ? kTileThreads : kColThreads, smem, st>>>(b);

@@ -351,10 +351,10 @@ __device__ void x_inverse(const cpx_t<R>* const* rows, int nr, cpx_t<R>* F, int 
 // Forward real transform of the data already packed in F (z[m] = x[2m] + i
 // x[2m+1] stored at position perm[m]) into nr mixed rows scaled by 1/ngx,
 // kx < nkx kept.
-template <typename R>
-__device__ void x_forward_packed(int nr, cpx_t<R>* F, int hp, cpx_t<R>* const* rows, const Dims& d,
+__device__ void x_forward_packed(int nr, float2* F, int hp, float2* const* rows, const Dims& d,
                                  const FftPlan& ph, const double2* __restrict__ rtw) {
-  using T2 = cpx_t<R>;
+  using R = float;
+  using T2 = float2;
   const int h = d.ngx / 2, nkx = d.nkx;
   const R scale = (R)(1.0 / d.ngx);
   fft_dit<R, -1, false>(F, nr, 1, hp, ph, false);
@@ -381,12 +381,12 @@ __device__ void x_forward_packed(int nr, cpx_t<R>* F, int hp, cpx_t<R>* const* r
 // takes the mixed rows A, B (nkx modes, zero beyond, imaginary part of the
 // kx = 0 mode dropped as the real inverse does) as z = a + i b; the forward
 // splits the transform of z = a + i b into the two half spectra.  This costs
-// fewer FP64 instructions than two half-length real transforms with their
+// fewer instructions than two half-length real transforms with their
 // pre/post twiddle passes.
-template <typename R>
-__device__ void x_inverse_pair(const cpx_t<R>* rowA, const cpx_t<R>* rowB, cpx_t<R>* F, R* outA, R* outB,
+__device__ void x_inverse_pair(const float2* rowA, const float2* rowB, float2* F, float* outA, float* outB,
                                const Dims& d, const FftPlan& pf) {
-  using T2 = cpx_t<R>;
+  using R = float;
+  using T2 = float2;
   const int n = d.ngx, nkx = d.nkx;
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     T2 z = T2{0, 0};
@@ -413,9 +413,9 @@ __device__ void x_inverse_pair(const cpx_t<R>* rowA, const cpx_t<R>* rowB, cpx_t
 
 // Forward transform of np2 packed pairs F[p*n + perm[x]] = a[x] + i b[x]
 // into 2*np2 mixed rows (kx < nkx, scaled by 1/ngx).
-template <typename R>
-__device__ void x_forward_pairs(int np2, cpx_t<R>* F, cpx_t<R>* const* rows, const Dims& d, const FftPlan& pf) {
-  using T2 = cpx_t<R>;
+__device__ void x_forward_pairs(int np2, float2* F, float2* const* rows, const Dims& d, const FftPlan& pf) {
+  using R = float;
+  using T2 = float2;
   const int n = d.ngx, nkx = d.nkx;
   const R sc = (R)(0.5 / n);
   fft_dit<R, -1, false>(F, np2, 1, n, pf, false);
@@ -458,7 +458,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
   double cmax = 0.0;
   // warm-up: previous centre and face
   if (c0 - 1 >= 1) {
-    x_inverse_pair<R>(a.mu + (size_t)(c0 - 1) * d.mp + rowoff, a.mw + (size_t)(c0 - 1) * d.mp + rowoff, F, up, wp, d,
+    x_inverse_pair(a.mu + (size_t)(c0 - 1) * d.mp + rowoff, a.mw + (size_t)(c0 - 1) * d.mp + rowoff, F, up, wp, d,
                       pf);
     const T2* rows[1] = {a.mv + (size_t)(c0 - 1) * d.mp + rowoff};
     R* outs[1] = {vp};
@@ -469,7 +469,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
   }
   for (int jj = c0; jj <= c1; ++jj) {
     const bool vface = jj <= d.nyv - 2;  // face jj interior (else the top wall, v = 0)
-    x_inverse_pair<R>(a.mu + (size_t)jj * d.mp + rowoff, a.mw + (size_t)jj * d.mp + rowoff, F, uc, wc, d, pf);
+    x_inverse_pair(a.mu + (size_t)jj * d.mp + rowoff, a.mw + (size_t)jj * d.mp + rowoff, F, uc, wc, d, pf);
     if (vface) {
       const T2* rows[1] = {a.mv + (size_t)jj * d.mp + rowoff};
       R* outs[1] = {vc};
@@ -529,12 +529,12 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
         ++npair;
       }
       if (later) {
-        x_forward_pairs<R>(2, F, rows, d, pf);
+        x_forward_pairs(2, F, rows, d, pf);
         for (int x = threadIdx.x; x < ngx; x += blockDim.x) face_pair(x, uc[x], wc[x], pf.perm[x]);
         __syncthreads();
-        x_forward_pairs<R>(1, F, rows + 4, d, pf);
+        x_forward_pairs(1, F, rows + 4, d, pf);
       } else {
-        x_forward_pairs<R>(npair, F, rows, d, pf);
+        x_forward_pairs(npair, F, rows, d, pf);
       }
     }
     // current becomes previous
@@ -1208,7 +1208,7 @@ __device__ __forceinline__ void xmask_body(const MaskArgs<float>& a, const Dims&
   }
   __syncthreads();
   T2* rows[1] = {row};
-  x_forward_packed<R>(1, F, hp, rows, d, ph, rtw);
+  x_forward_packed(1, F, hp, rows, d, ph, rtw);
 }
 
 // FP64: two z rows of a plane as one complex line in 64-bit fixed point (lh_fxfft.cuh).  The rows come out of the inverse

@@ -754,6 +754,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
       const int dp = min(Sp - Tf, 63), dc = min(Sc - Tf, 63);
       const bool shift1 = (dw | dvp | dvc) != 0, shiftf = (dp | dc) != 0;
       const int S0 = 2 * Sc - 64, S1 = 2 * T1 - 64, S2 = Tf + Spv - 64;  // the pairs' scales
+      const FxOut outc(0, Sc), out1(0, T1);  // of the CFL number
       fx2* F = raw;
       int np = 0;                        // lines transformed forward at once
       const int f0 = 0, f1 = cprod ? 2 : 0;
@@ -779,7 +780,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims
           const i64 vc = vp + dv;
           if (a.want_cfl) {
             if (!bad && !badv && !badpv)
-              cmax = fmax(cmax, fabs(fx_to(u, Sc)) * a.dxi + fabs(fx_to(vc, T1)) * a.dyc[jj] + fabs(fx_to(w, Sc)) * a.dzi);
+              cmax = fmax(cmax, fabs(outc(u)) * a.dxi + fabs(out1(vc)) * a.dyc[jj] + fabs(outc(w)) * a.dzi);
           } else {
             const int px = P.turn[x];
             F[px] = fx2{fx_prod(u, u), fx_prod(u, w)};

@@ -376,7 +376,8 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
 // addresses and nothing is copied twice.
 //
 // The CTA is warp-specialised, its roles ordered only by mbarriers:
-//   warps 0-3 (producers) fetch halos into a ring of six buffers with 16-byte
+//   warps 0-3 and 9-12 (two groups of producers, every other stage each) fetch
+//     halos into a ring of four buffers with 16-byte
 //     loads into registers and 16-byte shared stores (cp.async with a zero-fill
 //     size measured slower: its copies were not coalesced, about 32 L2 sectors
 //     and 38 shared wavefronts per warp instruction against 16 and 4); each
@@ -400,9 +401,13 @@ constexpr int TC_XR = TX + 2;                // halo x voxels
 constexpr int TC_HALO = TC_ZR * TC_XR;       // voxel rows of one k chunk of a halo
 constexpr int TC_XP = TC_ZR + 1;             // x pitch in 16-byte rows: odd, so a warp's copies spread over all banks
 constexpr int TC_KP = TC_XR * TC_XP;         // k-chunk pitch in 16-byte rows
-constexpr int TC_NBUF = 6;                   // halo ring (4: 218 us, 6: 203 us, 8: 201 us on 130x96x96)
-constexpr int TC_PRODUCERS = 128;            // warps 0-3
-constexpr int TC_THREADS = 288;              // + epilogue warps 4-7 + MMA warp 8
+constexpr int TC_NBUF = 4;                   // halo ring (6: the same training step, a correction of 258x192x192 0.8 % slower)
+constexpr int TC_PRODUCERS = 128;            // threads of a producer group
+// Producer groups take every other stage: while one waits for its loads, the other's are in flight.
+// With this and the weight gradient's, a training step on 130x96x96 takes 3.97 ms instead of 4.07 and a correction of
+// 258x192x192 11.35 instead of 11.65; a third group gains nothing more.
+constexpr int TC_GROUPS = 2;
+constexpr int TC_THREADS = 160 + 128 * TC_GROUPS;  // + epilogue warps 4-7 + MMA warp 8
 constexpr int TC_MMA_WARP = 8;
 constexpr unsigned kTcSpinLimit = 1u << 20;  // bound of every mbarrier wait
 
@@ -490,14 +495,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   const int nstages = 3 * my_tiles;
 
-  if (warp < 4) {
+  if (warp < 4 || warp > TC_MMA_WARP) {
     // ---- producers: stage st = (tile blockIdx.x + (st / 3) gridDim.x, dy = st % 3) into buffer st % NBUF:
     // rows [k chunk][x + 1][z + 1], x = -1 .. 32, z = -1 .. 8, periodic in x and z, zero outside y.  16-byte
     // loads into registers (a warp's loads cover contiguous voxels), then 16-byte shared stores; the buffer is
     // handed over as soon as its stores are done.
-    const int p = threadIdx.x;
+    const int group = warp < 4 ? 0 : (warp - TC_MMA_WARP + 3) / 4, p = 32 * (warp < 4 ? warp : (warp - 9) & 3) + lane;
     constexpr int CH = TC_HALO * KC, PT = (CH + TC_PRODUCERS - 1) / TC_PRODUCERS;
-    for (int s = 0; s < nstages; ++s) {
+    for (int s = group; s < nstages; s += TC_GROUPS) {
       if (s >= TC_NBUF && !tc_wait(empty + s % TC_NBUF, (uint32_t)((s / TC_NBUF - 1) & 1), abort)) break;
       const int tile = blockIdx.x + (s / 3) * gridDim.x, dy = s % 3;
       const int xt = tile % ntx, rest = tile / ntx, zt = rest % ntz, y = rest / ntz;
@@ -688,7 +693,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 //     apart in U's rows [column][level][chunk][z].
 // One MMA per (level of the tile, x column, dz) accumulates D[dz] (128 x 3Cu fp32 in TMEM) over every tile
 // of the persistent CTA; tap (dy, dz, dx) of D[dz][(l, c)][(e, c')] is (1 - e, dz - 1, l - 1) relative to U.
-// Roles as in the forward kernel: warps 0-3 copy a tile's halo into a ring of stage buffers (register-staged
+// Roles as in the forward kernel: two groups of four warps copy every other tile's halo into a ring of stage buffers (register-staged
 // 16-byte loads and stores) and arrive on `full`; warp 8 (one thread) issues the tile's MMAs and commits them to `empty`; warps 4-7 sum the tile's
 // output gradient (the bias gradient) from the same buffer and arrive on `empty` too, and at the end read
 // D from TMEM and add it to dw.  Every wait is bounded as in the forward kernel.
@@ -699,7 +704,8 @@ constexpr int WT_L = WT_TXW + 3;        // S halo lines x0 - 1 .. x0 + 9
 constexpr int WT_ZR = WT_TZ + 2;        // S halo z rows
 constexpr int WT_ZP = 19;               // S z pitch in 16-byte rows (odd: a warp's copies spread over all banks)
 constexpr int WT_ZPU = 17;              // U z pitch
-constexpr int WT_THREADS = 288;
+constexpr int WT_GROUPS = 2;            // producer groups, as in the forward kernel
+constexpr int WT_THREADS = 160 + 128 * WT_GROUPS;
 
 template <int CU>
 struct WtGeom {
@@ -759,14 +765,14 @@ __global__ void __launch_bounds__(WT_THREADS, 1)
     y0 = (rest / ntz) * WT_TY;
   };
 
-  if (warp < 4) {
+  if (warp < 4 || warp > TC_MMA_WARP) {
     // ---- producers: tile s into buffer s % NBUF.  16-byte loads into registers, then 16-byte shared stores
     // (a warp's 32 loads cover 512 contiguous bytes and its stores hit every bank group four times), S first,
     // then U; the buffer is handed over as soon as its stores are done.
-    const int p = threadIdx.x;
+    const int group = warp < 4 ? 0 : (warp - TC_MMA_WARP + 3) / 4, p = 32 * (warp < 4 ? warp : (warp - 9) & 3) + lane;
     constexpr int SCH = WT_TY * WT_ZR * WT_L * KCS, UCH = G::UL * WT_TZ * WT_TXW * KCU;
     constexpr int SPT = (SCH + TC_PRODUCERS - 1) / TC_PRODUCERS, UPT = (UCH + TC_PRODUCERS - 1) / TC_PRODUCERS;
-    for (int s = 0; s < my_tiles; ++s) {
+    for (int s = group; s < my_tiles; s += WT_GROUPS) {
       if (s >= NBUF && !tc_wait(empty + s % NBUF, (uint32_t)((s / NBUF - 1) & 1), abort)) break;
       int y0, z0, x0;
       tile_origin(s, y0, z0, x0);

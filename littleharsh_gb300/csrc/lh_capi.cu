@@ -240,11 +240,11 @@ int build_fx(lh_handle* h, FxPlan* P, int n) {
 // 96 x 96 x 130 0.42 -> 0.21, 288 x 288 x 226 3.08 -> 1.91, 576 x 576 x 450 17.4 -> 15.2 (128 threads there 15.9).
 //
 // Levels per CTA: the chunk with the least estimated time, (CTAs / CTAs resident at once, at least one wave) x (levels +
-// 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (FP64, chunks of 2 / 4 / 8 / 16
-// levels: 48 x 48 x 66 0.11 / 0.15 / 0.25 / 0.45 ms a step, 96 x 96 x 130 0.51 / 0.46 / 0.46 / 0.58, 162 x 108 x 124
-// 0.96 / 0.82 / 0.76 / 0.95; mixed, two rows: 48 x 48 x 66 0.07 / 0.10, 96 x 96 x 130 0.20 / 0.22 / 0.23); on large ones
-// long chunks save the repeated level (576 x 576 x 450, 8 / 16 / 32 / 64: 38.6 / 37.3 / 36.9 / 37.3, mixed 15.2 / 15.1 /
-// 15.2 / -).
+// 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (FP64: 48 x 48 x 66 with chunks of
+// 2 / 4 / 8 levels 0.10 / 0.15 / 0.25 ms a step, 96 x 96 x 130 with 2 / 4 / 6 / 8 0.48 / 0.44 / 0.50 / 0.43, 162 x 108 x
+// 124 with 4 / 8 / 12 0.72 / 0.67 / 0.75; mixed, two rows: 48 x 48 x 66 with 2 / 4 0.07 / 0.10, 96 x 96 x 130 with 2 / 4 /
+// 8 0.20 / 0.22 / 0.23); on large ones long chunks save the repeated level (FP64: 288 x 288 x 226 with 8 / 32 4.19 / 4.23,
+// 576 x 576 x 450 with 8 / 16 / 32 / 64 5 / 1 / 0 / 1 % above the least; mixed 15.2 / 15.1 / 15.2 with 8 / 16 / 32).
 void default_xprod_shape(lh_handle* h) {
   const Dims& d = h->d;
   const bool mixed = h->precision == LH_PREC_MIXED;

@@ -127,7 +127,7 @@ __device__ __forceinline__ void zfwd_body(const ZJobs<float>& jobs, const Dims& 
 // inputs and the last one writes FP64.  Bound by instruction issue (340 instructions a point, 50-60 % issue) on the
 // integer pipes; the conversions run beside them on the FP64 pipe, in zinv both ways, in zfwd outward with the
 // normalisation (its inputs take integer shifts, or the FP64 pipe would be the bound).  64 registers (four CTAs of 256
-// threads) beat 80.  A step of the 576 x 576 x 450 grid (449 levels transformed) on a GB300: z-inverse 22.9 -> 6.0 ms,
+// threads) beat 80.  A step of the 576 x 576 x 450 grid (449 levels transformed) on a GB300: z-inverse 22.9 -> 5.7 ms,
 // z-forward 47.8 -> 11.3 ms against FP64 radix-4/3 butterflies; their memory traffic alone is 1.8 and 3.5 ms.
 
 constexpr int kFxMaxTile = 32;  // columns of a tile (a power of two)
@@ -152,7 +152,7 @@ __device__ __forceinline__ void fx_combine(unsigned m, unsigned* dst, int tx) {
   }
 }
 
-// After the thread's copies into the tile: biased exponent of the largest value of its column.
+// After the thread's copies into the tile: high word of the largest value of its column (its exponent from bit 20 on).
 __device__ __forceinline__ int fx_sweep(FxLines& L, const FxCol& C, int n) {
   const int tx = 1 << C.ltx;
   if ((int)threadIdx.x < tx) { L.e[threadIdx.x] = 0; L.sum[threadIdx.x] = 0; }
@@ -163,7 +163,7 @@ __device__ __forceinline__ int fx_sweep(FxLines& L, const FxCol& C, int n) {
   for (int r = C.t0; r < n; r += C.dt) m = max(m, fx_hi(reinterpret_cast<const double2*>(C.buf)[r << C.ltx]));
   fx_combine<false>(m, L.e, tx);
   __syncthreads();
-  return (int)(L.e[threadIdx.x & (tx - 1)] >> 20);
+  return (int)L.e[threadIdx.x & (tx - 1)];
 }
 
 __device__ __forceinline__ FxCol fx_col(fx2* sm, int tx) {
@@ -193,7 +193,7 @@ __device__ __forceinline__ void zinv_body(const ZJobs<double>& jobs, const Dims&
     if (!in || (unsigned)(z - h) < (unsigned)gap) *s = fx2{0, 0};
     else fx_copy(s, (z < h ? src : top) + (ptrdiff_t)z * pitch);
   }
-  const int e = fx_sweep(L, C, d.ngz);
+  const int top_word = fx_sweep(L, C, d.ngz), e = top_word >> 20;
   const FxIn scale(e);
   unsigned sum = 0;
   auto load = [&](double2 v) {
@@ -211,7 +211,9 @@ __device__ __forceinline__ void zinv_body(const ZJobs<double>& jobs, const Dims&
   };
   auto store = [&](int z, fx2 v) {
     const FxOut out(e, S - g);
-    if (in) dst[(size_t)z * d.nkx] = double2{out(v.y), out(v.x)};
+    // columns of zeros, which fields with few modes have many of, stay zeros (scaled back, what the roundings leave of
+    // them takes FP64 instructions: 0.69 ms instead of 0.24 a launch of 576 x 576 x 58 with eight modes a direction)
+    if (in) dst[(size_t)z * d.nkx] = top_word ? double2{out(v.y), out(v.x)} : double2{0.0, 0.0};
   };
   fx_tile(C, P, load, total, store);
 }
@@ -234,7 +236,7 @@ __device__ __forceinline__ void zfwd_body(const ZJobs<double>& jobs, const Dims&
     if (in) fx_copy(s, src + (size_t)z * d.nkx);
     else *s = fx2{0, 0};
   }
-  const int e = fx_sweep(L, C, d.ngz);
+  const int e = fx_sweep(L, C, d.ngz) >> 20;
   auto load = [&](double2 v) { return fx2{fx_from(v.x, e), fx_from(v.y, e)}; };
   auto total = [&]() {
     __syncthreads();

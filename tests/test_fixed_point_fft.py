@@ -150,6 +150,25 @@ def test_canopy_rows_against_the_oracle(oracle_mod, cfg):
 
 
 @pytest.mark.gpu
+def test_zero_lines_stay_zero():
+    """A field of zeros has a nonlinear term of exact zeros, and rows without a velocity component do not disturb others."""
+    import littleharsh_gb300 as lh
+    s = lh.Solver(lh.Config(**SMALL))
+    f = s.get_fields()
+    s.set_fields(*[np.zeros_like(x) for x in f])
+    s.set_time(0.0, 1e-3, 0.0)
+    s.substage(1, 1)
+    for n in s.get_nonlinear():
+        assert not n.any()
+    u = np.zeros_like(f[0])
+    u[:, 0, 0] = np.linspace(1.0, 2.0, u.shape[0])
+    s.set_fields(u, np.zeros_like(f[1]), np.zeros_like(f[2]), np.zeros_like(f[3]))
+    s.substage(1, 1)
+    for n in s.get_nonlinear():  # d/dx, d/dz of u(y)^2 and d/dy of products with v = 0
+        assert np.abs(n).max() < 1e-14
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("banded", [False, True], ids=["one", "bands"])
 def test_chunks_of_levels_keep_results(monkeypatch, banded):
     """Chunks of one, three and any number of levels start at whole pairs of levels: bit for bit the same step."""

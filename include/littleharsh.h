@@ -263,22 +263,20 @@ int lh_profile_step(lh_handle* h, double* ms_by_kind, int32_t* count_by_kind, in
 int lh_autotune(lh_handle* h, int32_t* tx, int32_t* chunk);
 
 /* The launch shapes the next step uses (no reference counterpart): z tile
- * width, levels per product-pass CTA (FP64 rounds it up to whole pairs), and
- * whether the mixed form's product pass transforms the face pair after the
- * centre pairs through a smaller buffer (1) or all three pairs at once (0; the
- * FP64 pass has its own buffers and does not depend on it); lh_autotune picks
- * that by timing too.  Any pointer may be NULL. */
+ * width, levels per product-pass CTA, and whether the product pass transforms
+ * the face pair after the centre pairs through a smaller buffer (1) or all
+ * three pairs at once (0); lh_autotune picks that by timing too.  Any pointer
+ * may be NULL. */
 int lh_get_launch_shapes(lh_handle* h, int32_t* tx, int32_t* chunk, int32_t* xsplit);
 
 /* Threads per product-pass CTA the next step uses (128 or 256; no reference
- * counterpart; FP64 takes at most that many, no more than its rows can use);
- * lh_autotune picks it by timing.  Batched ensemble launches always use 256. */
+ * counterpart); lh_autotune picks it by timing.  Batched ensemble launches
+ * always use 256. */
 int lh_get_x_threads(lh_handle* h, int32_t* threads);
 
 /* Threads per CTA of the z passes (nonlinear term and canopy forcing) the
- * next step uses (128 or 256; no reference counterpart; FP64 takes at most
- * that many, sharing its tile's butterflies evenly); lh_autotune picks it by
- * timing at the z tile width it chose.  Batched ensemble launches always
+ * next step uses (128 or 256; no reference counterpart); lh_autotune picks it
+ * by timing at the z tile width it chose.  Batched ensemble launches always
  * use 256. */
 int lh_get_z_threads(lh_handle* h, int32_t* threads);
 

@@ -35,12 +35,6 @@ struct PlanStore {
   DevBuf perm, tw64, tw32;
 };
 
-// The z plan of a precision (FP32 butterflies or FP64 in fixed point).
-template <typename R> const ZPlan<R>& zplan(const FftPlan& p, const FxPlan& f) {
-  if constexpr (sizeof(R) == 4) return p;
-  else return f;
-}
-
 }  // namespace
 
 struct lh_handle {
@@ -81,10 +75,9 @@ struct lh_handle {
   double* tabs = nullptr;  // lu_u, lu_v, u11 (rewritten when dt changes)
   DevScalars* sc = nullptr;
   PlanStore pz, ph, pf;  // z (Ngalz), x half length (Ngalx/2), x full length (Ngalx)
-  FxPlan qz{}, qx{};     // z and x in fixed point
+  FxPlan qz{};           // z in fixed point (the conditional statistics')
   double2* rtw = nullptr;
   PlanStore pz2, ph2, pf2;  // the same for the middle band (bands only)
-  FxPlan qz2{}, qx2{};
   double2* rtw2 = nullptr;
   Dims dmid{};              // the middle band's plane geometry (bands only)
   int tx = 8, chunk = 16;
@@ -218,18 +211,18 @@ int build_plan(lh_handle* h, PlanStore& ps, int n, int keep_half) {
   return LH_OK;
 }
 
-// The fixed-point plan of a length that build_plan accepts.
+// The fixed-point plan of a length that build_plan accepts; lengths beyond its tables' leave P empty (n = 0).
 int build_fx(lh_handle* h, FxPlan* P, int n) {
   FxTables t;
-  if (!fx_build(n, P, &t)) return fail(h, LH_EFFT, "transform length %d is too long", n);
+  FxPlan q{};
+  if (!fx_build(n, &q, &t)) return LH_OK;
   if (t.tw.empty()) t.tw.push_back(int4{0, 0, 0, 0});
-  short *a, *b, *e, *f;
+  short *a, *b;
   int4* w;
   int rc;
-  if ((rc = upload(h, &a, t.pos_sample)) || (rc = upload(h, &b, t.pos_freq)) || (rc = upload(h, &e, t.freq_pos)) ||
-      (rc = upload(h, &f, t.turn)) || (rc = upload(h, &w, t.tw)))
-    return rc;
-  P->pos_sample = a; P->pos_freq = b; P->freq_pos = e; P->turn = f; P->tw = w;
+  if ((rc = upload(h, &a, t.pos_sample)) || (rc = upload(h, &b, t.freq_pos)) || (rc = upload(h, &w, t.tw))) return rc;
+  q.pos_sample = a; q.freq_pos = b; q.tw = w;
+  *P = q;
   return LH_OK;
 }
 
@@ -238,25 +231,37 @@ int build_fx(lh_handle* h, FxPlan* P, int n) {
 // Mixed form: two z rows per CTA where Ngalz is even, with 128 threads while a stage of its three transforms has at most
 // 256 butterflies (3/4 Ngalx; with 256 threads most would idle), else 256.  Against one row and 256 threads, ms a step:
 // 96 x 96 x 130 0.42 -> 0.21, 288 x 288 x 226 3.08 -> 1.91, 576 x 576 x 450 17.4 -> 15.2 (128 threads there 15.9).
-//
 // Levels per CTA: the chunk with the least estimated time, (CTAs / CTAs resident at once, at least one wave) x (levels +
-// 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (FP64: 48 x 48 x 66 with chunks of
-// 2 / 4 / 8 levels 0.10 / 0.15 / 0.25 ms a step, 96 x 96 x 130 with 2 / 4 / 6 / 8 0.48 / 0.44 / 0.50 / 0.43, 162 x 108 x
-// 124 with 4 / 8 / 12 0.72 / 0.67 / 0.75; mixed, two rows: 48 x 48 x 66 with 2 / 4 0.07 / 0.10, 96 x 96 x 130 with 2 / 4 /
-// 8 0.20 / 0.22 / 0.23); on large ones long chunks save the repeated level (FP64: 288 x 288 x 226 with 8 / 32 4.19 / 4.23,
-// 576 x 576 x 450 with 8 / 16 / 32 / 64 5 / 1 / 0 / 1 % above the least; mixed 15.2 / 15.1 / 15.2 with 8 / 16 / 32).
+// 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (48 x 48 x 66 with chunks of 2 / 4
+// levels 0.07 / 0.10 ms a step, 96 x 96 x 130 with 2 / 4 / 8 0.20 / 0.22 / 0.23); on large ones long chunks save the
+// repeated level (576 x 576 x 450 with 8 / 16 / 32: 15.2 / 15.1 / 15.2).
+//
+// FP64 form: 128 threads (256 measured 2 to 20 % slower at every length).  The CTAs of an SM share its FP64 pipe, and four
+// of them saturate it: a chunk's estimated time is (an SM's CTAs, at least 4, and one for the uneven end) x (levels + 1/3,
+// the previous level's share); within 2 % the longest chunk is taken.  ms a step at 48 x 48 x 66 with 2 / 3 / 4 / 8 / 16
+// levels 0.265 / 0.228 / 0.254 / 0.364 / 0.616; 96 x 96 x 130 with 2 / 4 / 6 / 8 / 16 1.30 / 1.22 / 1.20 / 1.30 / 1.38;
+// 162 x 108 x 124 with 4 / 6 / 8 / 16 2.37 / 2.38 / 2.42 / 2.58; 288 x 288 x 226 with 4 / 8 / 16 / 32 17.6 / 17.1 / 17.0 /
+// 17.7; 576 x 576 x 450 with 8 / 16 / 32 139.4 / 137.6 / 138.0.
 void default_xprod_shape(lh_handle* h) {
   const Dims& d = h->d;
-  const bool mixed = h->precision == LH_PREC_MIXED;
-  if (mixed && d.ngz % 2 == 0) {
+  const int nlev = d.nyu - 1;
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  double least = 1e300;
+  if (h->precision != LH_PREC_MIXED) {
+    h->xthreads = 128;
+    for (int c : {2, 3, 4, 6, 8, 12, 16, 32}) {
+      const long long ctas = (long long)d.ngz * ((nlev + c - 1) / c);
+      const double t = ((double)std::max(4ll, (ctas + sms - 1) / sms) + 1.0) * (c + 1.0 / 3.0);
+      if (t < 1.02 * least) { least = std::min(least, t); h->chunk = c; }
+    }
+    return;
+  }
+  if (d.ngz % 2 == 0) {
     h->xrows = 2;
     h->xthreads = 3 * d.ngx / 4 <= 256 ? 128 : 256;
   }
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-  const double resident = (double)sms * (mixed ? xprod_ctas_per_sm<float>(d, h->xrows, h->xthreads)
-                                               : xprod_ctas_per_sm<double>(d, 1, h->xthreads));
-  double least = 1e300;
+  const double resident = (double)sms * xprod_ctas_per_sm(d, h->xrows, h->xthreads);
   for (int c : {2, 4, 8, 16, 32}) {
     const double ctas = (double)(d.ngz / h->xrows) * ((d.nyu - 2 + c - 1) / c);
     const double t = std::max(1.0, ctas / resident) * (c + 1.3);
@@ -381,13 +386,12 @@ int build_dt_tables(lh_handle* h) {
 struct BandLaunch {
   const Dims* d;
   const FftPlan *pz, *ph, *pf;
-  const FxPlan *qz, *qx;
   const double2* rtw;
   int c_lo, c_hi, f_lo, f_hi;
 };
 int band_launches(const lh_handle* h, BandLaunch* out) {
   const Dims& d = h->d;
-  const BandLaunch fine{&d, &h->pz.plan, &h->ph.plan, &h->pf.plan, &h->qz, &h->qx, h->rtw, 0, 0, 0, 0};
+  const BandLaunch fine{&d, &h->pz.plan, &h->ph.plan, &h->pf.plan, h->rtw, 0, 0, 0, 0};
   if (!d.banded) {
     out[0] = fine;
     out[0].c_lo = 1; out[0].c_hi = d.nyu - 2; out[0].f_lo = 1; out[0].f_hi = d.nyv - 2;
@@ -395,22 +399,10 @@ int band_launches(const lh_handle* h, BandLaunch* out) {
   }
   out[0] = fine;
   out[0].c_lo = 1; out[0].c_hi = d.Nu1; out[0].f_lo = 1; out[0].f_hi = d.Nv1;
-  out[1] = BandLaunch{&h->dmid, &h->pz2.plan, &h->ph2.plan, &h->pf2.plan, &h->qz2, &h->qx2, h->rtw2, d.Nu1 + 1, d.Nu2, d.Nv1 + 1, d.Nv2};
+  out[1] = BandLaunch{&h->dmid, &h->pz2.plan, &h->ph2.plan, &h->pf2.plan, h->rtw2, d.Nu1 + 1, d.Nu2, d.Nv1 + 1, d.Nv2};
   out[2] = fine;
   out[2].c_lo = d.Nu2 + 1; out[2].c_hi = d.nyu - 2; out[2].f_lo = d.Nv2 + 1; out[2].f_hi = d.nyv - 2;
   return 3;
-}
-
-template <typename R>
-XPlan<R> xplan(const lh_handle* h, const BandLaunch& B) {
-  if constexpr (sizeof(R) == 4) return XPlan<R>{*B.ph, *B.pf, B.rtw};
-  else return XPlan<R>{*B.qx, h->t.wcq, h->t.wfq};
-}
-
-template <typename R>
-MaskPlan<R> mask_plan(const lh_handle* h) {
-  if constexpr (sizeof(R) == 4) return MaskPlan<R>{h->ph.plan, h->rtw};
-  else return MaskPlan<R>{h->qx};
 }
 
 // The nonlinear term's plane work for one band: z-inverse of the levels the band's products need, products,
@@ -418,9 +410,8 @@ MaskPlan<R> mask_plan(const lh_handle* h) {
 template <typename R>
 struct NlBand {
   const Dims* d;
-  const ZPlan<R>* pz;
-  XPlan<R> px;
-  double norm;  // of the z-forward: 1/Ngalz, and in FP64 also the product pass's 1/Ngalx
+  const FftPlan *pz, *ph, *pf;
+  const double2* rtw;
   ZJobs<R> zi, zf;
   ProdArgs<R> xp;
 };
@@ -435,8 +426,7 @@ int nl_bands(const lh_handle* h, NlBand<R>* out) {
     const BandLaunch& B = bl[b];
     const Dims& db = *B.d;
     NlBand<R>& o = out[b];
-    o.d = B.d; o.pz = &zplan<R>(*B.pz, *B.qz); o.px = xplan<R>(h, B);
-    o.norm = sizeof(R) == 4 ? 1.0 / db.ngz : 1.0 / ((double)db.ngz * db.ngx);
+    o.d = B.d; o.pz = B.pz; o.ph = B.ph; o.pf = B.pf; o.rtw = B.rtw;
     const int L0 = std::min(B.c_lo, B.f_lo + 1), L1 = std::max(B.c_hi, B.f_hi + 1);
     {
       const int ul = std::max(1, L0 - 1), uh = std::min(d.nyu - 2, L1);
@@ -497,11 +487,11 @@ void enqueue_nonlinear(lh_handle* h, cudaStream_t st, bool zinv, bool xprod, boo
       mark(h, K_ZINV);
     }
     if (xprod) {
-      launch_xprod<R>(B.xp, *B.d, B.px, st);
+      launch_xprod<R>(B.xp, *B.d, *B.ph, *B.pf, B.rtw, st);
       mark(h, K_XPROD);
     }
     if (zfwd) {
-      launch_zfwd<R>(B.zf, *B.d, *B.pz, h->tx, B.norm, st, h->zthreads);
+      launch_zfwd<R>(B.zf, *B.d, *B.pz, h->tx, 1.0 / B.d->ngz, st, h->zthreads);
       mark(h, K_ZFWD);
     }
   }
@@ -599,11 +589,11 @@ int enqueue_substage(lh_handle* h, int k, int upto) {
     ZJobs<R> zi, zf;
     MaskArgs<R> m;
     if (ib_args<R>(h, k, &zi, &m, &zf)) {
-      launch_zinv<R>(zi, d, zplan<R>(h->pz.plan, h->qz), h->tx, st, h->zthreads);
+      launch_zinv<R>(zi, d, h->pz.plan, h->tx, st, h->zthreads);
       mark(h, K_IB_ZINV);
-      launch_xmask<R>(m, d, mask_plan<R>(h), st);
+      launch_xmask<R>(m, d, h->ph.plan, h->rtw, st);
       mark(h, K_IB_XMASK);
-      launch_zfwd<R>(zf, d, zplan<R>(h->pz.plan, h->qz), h->tx, 1.0 / d.ngz, st, h->zthreads);
+      launch_zfwd<R>(zf, d, h->pz.plan, h->tx, 1.0 / d.ngz, st, h->zthreads);
       mark(h, K_IB_ZFWD);
     }
   }
@@ -848,7 +838,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
   int rc;
   // FFT plans: z of length ngz, x through a complex transform of ngx/2
   if ((rc = build_plan(h, h->pz, d.ngz, d.nz / 2)) || (rc = build_plan(h, h->ph, d.ngx / 2, 0)) ||
-      (rc = build_plan(h, h->pf, d.ngx, 0)) || (rc = build_fx(h, &h->qz, d.ngz)) || (rc = build_fx(h, &h->qx, d.ngx)))
+      (rc = build_plan(h, h->pf, d.ngx, 0)))
     return bail(rc);
   if (d.banded) {
     // the middle band's planes: their own transform lengths and mode counts, the same storage
@@ -857,7 +847,7 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
     c.ngx = d.ngx2; c.ngz = d.ngz2; c.nkx = d.nkx2; c.nz = d.nz2;
     c.mp = c.nkx * c.ngz;
     if ((rc = build_plan(h, h->pz2, c.ngz, c.nz / 2)) || (rc = build_plan(h, h->ph2, c.ngx / 2, 0)) ||
-        (rc = build_plan(h, h->pf2, c.ngx, 0)) || (rc = build_fx(h, &h->qz2, c.ngz)) || (rc = build_fx(h, &h->qx2, c.ngx)))
+        (rc = build_plan(h, h->pf2, c.ngx, 0)))
       return bail(rc);
     std::vector<double2> rt(c.ngx / 2 + 1);
     for (int k = 0; k <= c.ngx / 2; ++k) {
@@ -893,12 +883,6 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
       return bail(rc);
     h->t.kx = pkx; h->t.kz = pkz; h->t.k2x = pk2x; h->t.k2z = pk2z; h->t.d2u = pd2u; h->t.d2v = pd2v;
     h->t.cu = pcu; h->t.cv = pcv; h->t.wc = pwc; h->t.wf = pwf; h->t.dyc = pdyc; h->t.dyvw = pdyvw;
-    std::vector<int4> wcq, wfq;
-    for (double w : wc) wcq.push_back(fx_weight(w));
-    for (double w : wf) wfq.push_back(fx_weight(w));
-    int4 *pwcq, *pwfq;
-    if ((rc = upload(h, &pwcq, wcq)) || (rc = upload(h, &pwfq, wfq))) return bail(rc);
-    h->t.wcq = pwcq; h->t.wfq = pwfq;
     // the same values rounded to float (to nearest, as a device conversion would round them)
     auto rounded = [](const std::vector<double>& v) { return std::vector<float>(v.begin(), v.end()); };
     float *pkxf, *pkzf, *pcuf, *pcvf;
@@ -1032,7 +1016,8 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
       for (int j = 0; j < h->njp; ++j) { pl[2 * j] = j; pl[2 * j + 1] = d.nyp - 1 - j; }
       const size_t tile = (size_t)h->dnx * h->dnz;
       if ((rc = upload(h, &h->cond_ul, ul)) || (rc = upload(h, &h->cond_vl, vl)) || (rc = upload(h, &h->cond_pl, pl)) ||
-          (rc = dalloc(h, &h->cond, tile * (6 * (size_t)h->nju + 5 * (size_t)h->njv + 2 * (size_t)h->njp))))
+          (rc = dalloc(h, &h->cond, tile * (6 * (size_t)h->nju + 5 * (size_t)h->njv + 2 * (size_t)h->njp))) ||
+          (rc = build_fx(h, &h->qz, d.ngz)))
         return bail(rc);
     }
   }
@@ -1040,6 +1025,10 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
   // z tile width: narrow tiles keep several CTAs per SM so that one CTA's loads overlap another's
   // butterflies (measured on configuration 2: FP64 best at 4, mixed at 8)
   h->tx = h->precision == LH_PREC_MIXED ? 8 : 4;
+  {
+    const cudaError_t e = configure_kernels();
+    if (e != cudaSuccess) return bail(fail(h, LH_ECUDA, "kernel attributes: %s", cudaGetErrorString(e)));
+  }
   default_xprod_shape(h);
   // launch-shape overrides for tuning sweeps: LH_TX (z tile width, 1..64), LH_CHUNK (levels per x-pass CTA)
   if (const char* v = std::getenv("LH_TX")) { const int x = std::atoi(v); if (x >= 1 && x <= 64) h->tx = x; }
@@ -1048,10 +1037,6 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
   if (const char* v = std::getenv("LH_XTHREADS")) h->xthreads = std::atoi(v) == 128 ? 128 : 256;
   if (const char* v = std::getenv("LH_ZTHREADS")) h->zthreads = std::atoi(v) == 128 ? 128 : 256;
   if (const char* v = std::getenv("LH_XROWS")) h->xrows = std::atoi(v) == 2 ? 2 : 1;
-  {
-    const cudaError_t e = configure_kernels();
-    if (e != cudaSuccess) return bail(fail(h, LH_ECUDA, "kernel attributes: %s", cudaGetErrorString(e)));
-  }
   if (cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
     return bail(fail(h, LH_ECUDA, "cudaEventCreate failed"));
   {
@@ -1366,14 +1351,14 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
             xprod_shape<R>(xa, *B.d, &g, &sm);
             if (g.x == 0) continue;
             XDesc<R> D{};
-            D.a = xa; D.d = *B.d; D.p = B.px; D.gx = g.x; D.gy = g.y;
+            D.a = xa; D.d = *B.d; D.ph = *B.ph; D.pf = *B.pf; D.rtw = B.rtw; D.gx = g.x; D.gy = g.y;
             xd.push_back(D);
           } else {
             const ZJobs<R>& J = part == 0 ? B.zi : B.zf;
             zpass_shape<R>(J, *B.d, h->tx, &g, &sm);
             if (g.x == 0) continue;
             ZDesc<R> D{};
-            D.jobs = J; D.d = *B.d; D.p = *B.pz; D.scale = B.norm; D.tx = zpass_tile<R>(h->tx);
+            D.jobs = J; D.d = *B.d; D.p = *B.pz; D.scale = 1.0 / B.d->ngz; D.tx = h->tx;
             D.gx = g.x; D.gy = g.y; D.gz = g.z;
             zd.push_back(D);
           }
@@ -1390,7 +1375,7 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
       for (lh_handle* h : hs) {
         ADesc D{};
         D.a = asm_args<R>(h, k); D.d = h->d; D.t = h->t;
-        assemble_shape(h->d, sizeof(R) == 4, &D.gx, &D.gy, &D.levels);
+        D.gx = (h->d.np + kAsmThreads - 1) / kAsmThreads; D.gy = h->d.nyu;
         ad.push_back(D);
         blocks.push_back(D.gx * D.gy);
       }
@@ -1409,15 +1394,15 @@ void build_batched(const std::vector<lh_handle*>& hs, std::vector<Slot>& slots) 
         size_t sm;
         zpass_shape<R>(a, h->d, h->tx, &g, &sm);
         ZDesc<R> Di{};
-        Di.jobs = a; Di.d = h->d; Di.p = zplan<R>(h->pz.plan, h->qz); Di.scale = 1.0; Di.tx = zpass_tile<R>(h->tx); Di.gx = g.x; Di.gy = g.y; Di.gz = g.z;
+        Di.jobs = a; Di.d = h->d; Di.p = h->pz.plan; Di.scale = 1.0; Di.tx = h->tx; Di.gx = g.x; Di.gy = g.y; Di.gz = g.z;
         zi.push_back(Di); bi.push_back((int)(g.x * g.y * g.z)); si.push_back(sm);
         xmask_shape<R>(mk, h->d, &g, &sm);
         MDesc<R> Dm{};
-        Dm.a = mk; Dm.d = h->d; Dm.p = mask_plan<R>(h); Dm.gx = g.x; Dm.gy = g.y;
+        Dm.a = mk; Dm.d = h->d; Dm.ph = h->ph.plan; Dm.rtw = h->rtw; Dm.gx = g.x; Dm.gy = g.y;
         md.push_back(Dm); bm.push_back((int)(g.x * g.y)); sm_.push_back(sm);
         zpass_shape<R>(c, h->d, h->tx, &g, &sm);
         ZDesc<R> Df{};
-        Df.jobs = c; Df.d = h->d; Df.p = zplan<R>(h->pz.plan, h->qz); Df.scale = 1.0 / h->d.ngz; Df.tx = zpass_tile<R>(h->tx);
+        Df.jobs = c; Df.d = h->d; Df.p = h->pz.plan; Df.scale = 1.0 / h->d.ngz; Df.tx = h->tx;
         Df.gx = g.x; Df.gy = g.y; Df.gz = g.z;
         zf.push_back(Df); bf.push_back((int)(g.x * g.y * g.z)); sf.push_back(sm);
       }
@@ -1853,7 +1838,7 @@ int lh_cfl_dt(lh_handle* h, double cfl, double* dt_out) {
       J.j[2] = ZJob<R>{h->u2, nullptr, (T2*)h->mixv + (size_t)vl * db.mp, nullptr, vl, vh - vl + 1};
       J.njobs = 3;
       J.maxlev = uh - ul + 1;
-      launch_zinv<R>(J, db, zplan<R>(*B.pz, *B.qz), h->tx, h->st);
+      launch_zinv<R>(J, db, *B.pz, h->tx, h->st);
       ProdArgs<R> a{};
       a.mu = (const T2*)h->mixu; a.mw = (const T2*)h->mixw; a.mv = (const T2*)h->mixv;
       for (int i = 0; i < 6; ++i) a.out[i] = (T2*)h->mixp[i];
@@ -1861,7 +1846,7 @@ int lh_cfl_dt(lh_handle* h, double cfl, double* dt_out) {
       a.dxi = db.ngx / h->Lx; a.dzi = db.ngz / h->Lz;
       a.sc = h->sc; a.want_cfl = 1; a.chunk = h->chunk; a.split = h->xsplit; a.threads = h->xthreads;
       a.c_lo = B.c_lo; a.c_hi = B.c_hi; a.f_lo = B.c_lo; a.f_hi = B.c_lo - 1;  // centres only
-      launch_xprod<R>(a, db, xplan<R>(h, B), h->st);
+      launch_xprod<R>(a, db, *B.ph, *B.pf, B.rtw, h->st);
     }
   };
   if (h->precision == LH_PREC_MIXED) run(0.0f);
@@ -1976,7 +1961,8 @@ int lh_cond_accumulate(lh_handle* h) {
     J.j[6] = ZJob<double>{h->r2, nullptr, mx[6], h->cond_vl + 2 * j0, 0, 2 * cvv};
     J.njobs = 7;
     J.maxlev = 2 * std::max(cu, std::max(cvv, cp));
-    launch_zinv<double>(J, d, h->qz, h->tx, st);
+    if (h->qz.n) launch_zinv_fx(J, d, h->qz, h->tx, st);
+    else launch_zinv<double>(J, d, h->pz.plan, h->tx, st);
     CondArgs a{};
     a.mix[0][0] = mx[0]; a.mix[0][1] = mx[1]; a.mix[0][2] = mx[2];
     a.mix[1][0] = mx[3]; a.mix[1][1] = mx[4]; a.mix[1][2] = mx[6];

@@ -9,12 +9,11 @@
 // exp(-2 pi i k / n) computed on the host in extended precision, never
 // evaluated on the device.
 //
-// They serve the mixed form's FP32 passes and, in FP64, the conditional
-// statistics' x rows; the FP64 step transforms in fixed point
-// (lh_fxfft.cuh).  Each twiddle multiplication is fused into the butterfly's
-// additions (a + w*c as two FMAs per component, a - w*c as 2a - (a + w*c)),
-// so a radix-4 butterfly costs 24 instructions instead of 28, a radix-3 one
-// 18 instead of 22 and a radix-2 one 6 instead of 8.
+// The butterflies are written for the FP64 pipe, which is the bottleneck on
+// GB300 (1.2 TFLOP/s): each twiddle multiplication is fused into the
+// butterfly's additions (a + w*c as two FMAs per component, a - w*c as
+// 2a - (a + w*c)), so a radix-4 butterfly costs 24 FP64 instructions instead
+// of 28, a radix-3 one 18 instead of 22 and a radix-2 one 6 instead of 8.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -230,8 +229,8 @@ __device__ __forceinline__ void dit_stage(cpx_t<R>* buf, int nb, unsigned nbm, i
   }
 }
 
-// One DIT stage of radix RADIX over `nb` vectors of an x-transform buffer
-// (es = 1, slots of sxi), index divisions as multiply-highs.
+// One DIT stage of radix RADIX over `nb` vectors of an FP32 x-transform buffer
+// (es = 1, padded slots), index divisions as multiply-highs.
 template <typename R, int SIGN, int RADIX>
 __device__ __forceinline__ void dit_stage_padded(cpx_t<R>* buf, int nb, int bs, int L, int n, unsigned mm,
                                                  unsigned nbfm, bool skip_mid, const cpx_t<R>* __restrict__ tw) {
@@ -306,31 +305,51 @@ __device__ void fft_dit2(float4* buf, int nb, int bs, const FftPlan& P) {
 // vectors, es = nb-ish, bs = 1); otherwise consecutive butterflies of one
 // vector (es = 1).  SIGN = -1 forward, +1 inverse; no normalisation.
 // prune: skip the middle output third of the last radix-3 stage.
-// The radix is resolved once per stage, so each stage's loop runs one
+// FP32: the radix is resolved once per stage, so each stage's loop runs one
 // butterfly form with its index divisions as multiply-highs; the FP32
 // transforms are bound by instruction issue and shared memory, and this halves
-// the integer work per butterfly.  x transforms (not BFAST; es = 1) use the
-// slots of sxi.
+// the integer work per butterfly.  FP32 x transforms (not BFAST; es = 1) use
+// the padded slots of sxi.  FP64: one loop over all radices with plain divisions, which
+// measures faster on the FP64 pipe, where the integer work runs alongside.
 template <typename R, int SIGN, bool BFAST>
 __device__ void fft_dit(cpx_t<R>* buf, int nb, int es, int bs, const FftPlan& P, bool prune) {
   using T2 = cpx_t<R>;
   const T2* __restrict__ tw = twtab<R>(P);
   const int n = P.n;
-  const unsigned nbm = BFAST ? fdiv_mult((unsigned)nb) : 0u;
-  for (int s = 0; s < P.ns; ++s) {
-    const int r = P.rad[s], L = P.len[s];
-    const unsigned mm = P.mdiv[s], nbfm = P.qdiv[s];
-    const bool skip_mid = prune && s == P.ns - 1;
-    if constexpr (BFAST) {
-      if (r == 4) dit_stage<R, SIGN, BFAST, 4>(buf, nb, nbm, es, bs, L, n, mm, nbfm, false, tw);
-      else if (r == 2) dit_stage<R, SIGN, BFAST, 2>(buf, nb, nbm, es, bs, L, n, mm, nbfm, false, tw);
-      else dit_stage<R, SIGN, BFAST, 3>(buf, nb, nbm, es, bs, L, n, mm, nbfm, skip_mid, tw);
-    } else {  // the x transforms: es = 1, padded buffer
-      if (r == 4) dit_stage_padded<R, SIGN, 4>(buf, nb, bs, L, n, mm, nbfm, false, tw);
-      else if (r == 2) dit_stage_padded<R, SIGN, 2>(buf, nb, bs, L, n, mm, nbfm, false, tw);
-      else dit_stage_padded<R, SIGN, 3>(buf, nb, bs, L, n, mm, nbfm, skip_mid, tw);
+  if constexpr (sizeof(R) == 4) {
+    const unsigned nbm = BFAST ? fdiv_mult((unsigned)nb) : 0u;
+    for (int s = 0; s < P.ns; ++s) {
+      const int r = P.rad[s], L = P.len[s];
+      const unsigned mm = P.mdiv[s], nbfm = P.qdiv[s];
+      const bool skip_mid = prune && s == P.ns - 1;
+      if constexpr (BFAST) {
+        if (r == 4) dit_stage<R, SIGN, BFAST, 4>(buf, nb, nbm, es, bs, L, n, mm, nbfm, false, tw);
+        else if (r == 2) dit_stage<R, SIGN, BFAST, 2>(buf, nb, nbm, es, bs, L, n, mm, nbfm, false, tw);
+        else dit_stage<R, SIGN, BFAST, 3>(buf, nb, nbm, es, bs, L, n, mm, nbfm, skip_mid, tw);
+      } else {  // the x transforms: es = 1, padded buffer
+        if (r == 4) dit_stage_padded<R, SIGN, 4>(buf, nb, bs, L, n, mm, nbfm, false, tw);
+        else if (r == 2) dit_stage_padded<R, SIGN, 2>(buf, nb, bs, L, n, mm, nbfm, false, tw);
+        else dit_stage_padded<R, SIGN, 3>(buf, nb, bs, L, n, mm, nbfm, skip_mid, tw);
+      }
+      __syncthreads();
     }
-    __syncthreads();
+  } else {
+    for (int s = 0; s < P.ns; ++s) {
+      const int r = P.rad[s], L = P.len[s], m = L / r, ts = n / L;
+      const int nbf = n / r;
+      const int total = nb * nbf;
+      const bool twiddle = m > 1;
+      const bool skip_mid = prune && s == P.ns - 1;
+      for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        int b, f;
+        if (BFAST) { f = t / nb; b = t - f * nb; }
+        else { b = t / nbf; f = t - b * nbf; }
+        const int blk = f / m, k = f - blk * m;
+        T2* base = buf + b * bs + (blk * L + k) * es;
+        dit_butterfly<R, SIGN>(base, m * es, r, k * ts, twiddle, skip_mid, tw);
+      }
+      __syncthreads();
+    }
   }
 }
 

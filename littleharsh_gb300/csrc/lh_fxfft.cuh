@@ -4,11 +4,14 @@
 // 32-bit integer additions and 32 wide or high 32-bit products.  A 64-bit
 // integer addition (two instructions) therefore costs 1/30 of an FP64 one and
 // a 64-bit product with a constant (two high products, one wide one) about
-// 1/4, measured 57 and 7-11 lanes per clock and SM against 1.93.  The FP64
-// transforms of the step kept the FP64 pipe 85-89 % busy, so they run here:
-// every line is scaled by a power of two of its own into 64-bit integers
-// (block floating point), transformed exactly except for one rounding per
-// product (at 2^-60 of the line's bound), and scaled back to FP64.
+// 1/4, measured 57 and 7-11 lanes per clock and SM against 1.93.  FP64
+// transforms keep the FP64 pipe 85-89 % busy; the conditional statistics'
+// z-inverse runs here instead: every line is scaled by a power of two of its
+// own into 64-bit integers (block floating point), transformed exactly except
+// for one rounding per product (at 2^-60 of the line's bound), and scaled back
+// to FP64.  The step's transforms stay in FP64: a line has one exponent here
+// where FP64 has one per value, and the step's last bits are part of
+// established runs.
 //
 // Error.  FP64 rounds every intermediate value to 2^-53 of itself.  Here a
 // line's largest value is scaled to just below 2^59, and each pass but the
@@ -50,7 +53,7 @@ constexpr int kFxBits = 59;  // a line's real and imaginary parts are below 2^kF
 // One pass: rad elements at distance mI per item; item t of a vector works at element
 // (t / mI) * rad * mI + t % mI and its twiddles are those of k = (t % mI) / inner.
 struct FxPass {
-  unsigned mI_m, inner_m, items_m;  // fdiv multipliers of mI, inner and n / rad
+  unsigned mI_m, inner_m;           // fdiv multipliers of mI and inner
   short mI, inner, tw;              // tw: first twiddle (-1: none)
   unsigned char rad, shift, before; // shift: bits the input may have to be shifted by; before: of earlier passes
 };
@@ -62,9 +65,7 @@ struct FxPlan {
   int shift;             // bits a forward line, and at most an inverse line, is shifted by in all
   FxPass ps[kFxMaxPass];
   const short* pos_sample;   // position of sample s
-  const short* pos_freq;     // position of frequency k
   const short* freq_pos;     // frequency at a position
-  const short* turn;         // pos_sample[freq_pos[.]]: from the place of an output to that of an input
   const int4* tw;            // two int4 per twiddle: (w_r, w_r + w_i), (w_i - w_r, -), each high and low word
 };
 
@@ -104,13 +105,6 @@ FX_HD i64 fx_mul(i64 a, int bh, int bl) {
   const int l = (int)s, h = fx_high(s);
   const int t = fx_mhi(h, bl) + fx_mhi(l, bh) + 1;  // the 1 centres the two truncations
   return fx_shl((i64)h * bh + t, POST);
-}
-
-// a b / 2^64 for |a|, |b| < 2^62
-FX_HD i64 fx_prod(i64 a, i64 b) {
-  const int al = (int)a, ah = fx_high(a), bl = (int)b, bh = fx_high(b);
-  const int t = fx_mhi(ah, bl) + fx_mhi(al, bh) + 1;
-  return (i64)ah * bh + t;
 }
 
 FX_HD fx2 fx_add(fx2 a, fx2 b) { return fx2{a.x + b.x, a.y + b.y}; }
@@ -305,23 +299,6 @@ __device__ __forceinline__ FxItem fx_at(const FxPlan& P, const FxPass& ps, int t
   return it;
 }
 
-// One pass over nb vectors of shared memory, vector v at buf[v * n].  shift(v): of vector v's input.
-template <int RAD, typename Shift>
-__device__ __forceinline__ void fx_pass(fx2* buf, int nb, const FxPlan& P, const FxPass& ps, Shift shift) {
-  const int items = P.n / RAD, total = nb * items, mI = ps.mI;
-  for (int T = threadIdx.x; T < total; T += blockDim.x) {
-    const int v0 = fx_div(T, items, ps.items_m), t = T - v0 * items;
-    const FxItem it = fx_at<RAD>(P, ps, t);
-    fx2* b = buf + v0 * P.n + it.e0;
-    fx2 v[RAD];
-#pragma unroll
-    for (int p = 0; p < RAD; ++p) v[p] = b[p * mI];
-    fx_item<RAD>(v, it.tw, shift(v0));
-#pragma unroll
-    for (int p = 0; p < RAD; ++p) b[p * mI] = v[p];
-  }
-}
-
 #define FX_RADIX(r, CALL)                           \
   switch (r) {                                      \
     case 2: { constexpr int RAD = 2; CALL; break; } \
@@ -330,17 +307,6 @@ __device__ __forceinline__ void fx_pass(fx2* buf, int nb, const FxPlan& P, const
     case 8: { constexpr int RAD = 8; CALL; break; } \
     default: { constexpr int RAD = 9; CALL; break; } \
   }
-
-// All passes of nb vectors of shared memory, vector v at buf[v * n]: samples at their pos_sample places, frequency k comes
-// out at pos_freq[k].  sum: the sums of fx_mag of inverse lines, NULL for forward ones.  A barrier follows each pass.
-static __device__ __noinline__ void fx_fft(fx2* buf, int nb, const FxPlan& P, const unsigned* sum) {
-  auto shift = [&](const FxPass& ps, int v) { return fx_pass_shift(ps, sum ? fx_inv_shift(sum[v], P.shift) : P.shift); };
-  for (int i = 0; i < P.npass; ++i) {
-    const FxPass& ps = P.ps[i];
-    FX_RADIX(ps.rad, (fx_pass<RAD>(buf, nb, P, ps, [&](int v) { return shift(ps, v); })));
-    __syncthreads();
-  }
-}
 
 // 16 bytes from global to shared memory, asynchronously
 __device__ __forceinline__ void fx_copy(fx2* dst, const double2* src) {
@@ -462,12 +428,6 @@ struct FxOut {
 __device__ __forceinline__ unsigned fx_hi(double2 v) {
   return max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
 }
-// magnitude bits of the high word
-__device__ __forceinline__ unsigned fx_bits(i64 a) {
-  const int h = (int)(a >> 32);
-  return (unsigned)(h ^ (h >> 31));
-}
-
 #endif
 
 // ---------------------------------------------------------------------------
@@ -475,7 +435,7 @@ __device__ __forceinline__ unsigned fx_bits(i64 a) {
 // ---------------------------------------------------------------------------
 
 struct FxTables {
-  std::vector<short> pos_sample, pos_freq, freq_pos, turn;
+  std::vector<short> pos_sample, pos_freq, freq_pos;
   std::vector<int4> tw;
 };
 
@@ -485,15 +445,6 @@ inline void fx_word(long double v, int* h, int* l) {
   const i64 q = (i64)(v < 0 ? v - 0.5L : v + 0.5L);
   *h = (int)((q + 0x80000000ll) >> 32);
   *l = (int)q;
-}
-
-// An interpolation weight as (high, low word of m 2^62, k), w = m 2^k with |m| < 2: k = 0 but for weights beyond [-1, 1].
-inline int4 fx_weight(double w) {
-  int k = 0;
-  while (std::fabs(w) > 1.0 && k < 1000) { w *= 0.5; ++k; }
-  int4 r{0, 0, k, 0};
-  fx_word(w, &r.x, &r.y);
-  return r;
 }
 
 inline unsigned fx_div_mult(unsigned d) { return d > 1 ? 0xFFFFFFFFu / d + 1u : 0u; }
@@ -559,7 +510,6 @@ inline bool fx_build(int n, FxPlan* plan, FxTables* tab) {
       ps.tw = -1;
       ps.mI_m = fx_div_mult((unsigned)(mm * inner));
       ps.inner_m = fx_div_mult((unsigned)inner);
-      ps.items_m = fx_div_mult((unsigned)(n / r));
       if (mm > 1) {
         ps.tw = (short)(tab->tw.size() / 2);
         for (int k = 0; k < mm; ++k)
@@ -583,8 +533,6 @@ inline bool fx_build(int n, FxPlan* plan, FxTables* tab) {
       mm *= r;
     }
   }
-  tab->turn.resize(n);
-  for (int i = 0; i < n; ++i) tab->turn[i] = tab->pos_sample[tab->freq_pos[i]];
   plan->npass = np[0] + np[1];
   if (plan->npass) {
     const FxPass& l = plan->ps[plan->npass - 1];

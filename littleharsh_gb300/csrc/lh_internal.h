@@ -74,8 +74,6 @@ struct Tables {
   const double* cv;    // [nyv] ddthetavi*dthdyv
   const double* wc;    // [nyu] weight of face j in the centre-j interpolation of v
   const double* wf;    // [nyv] weight of centre j+1 in the face-j interpolation of u, w
-  const int4* wcq;     // [nyu] wc in fixed point (XPlan)
-  const int4* wfq;     // [nyv] wf
   const double* dyc;   // [nyu] 1/(yv(j)-yv(j-1)) at centres, for the CFL number
   const double* dyvw;  // [nn+2] yv(j)-yv(j-1), j = 1..nn+1 at index j (flow rate)
   const double* lu_u;  // [3 kRK][3][nyu] Helmholtz LU (a1, 1/diag, scaled a3), u grid, long columns
@@ -135,16 +133,13 @@ struct ZJobs {
   int njobs, maxlev;
 };
 
-// The plan a z pass of a precision uses: FP32 butterflies, or 64-bit fixed point for FP64.
-template <typename R> struct ZPlanOf { using T = FftPlan; };
-template <> struct ZPlanOf<double> { using T = FxPlan; };
-template <typename R> using ZPlan = typename ZPlanOf<R>::T;
-
 // Launchers (lh_kernels.cu).  All are asynchronous on `st`.
 template <typename R>
-void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, cudaStream_t st, int threads = 256);
+void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, cudaStream_t st, int threads = 256);
+// The FP64 z-inverse in fixed point (the conditional statistics').
+void launch_zinv_fx(const ZJobs<double>& jobs, const Dims& d, const FxPlan& P, int tx, cudaStream_t st);
 template <typename R>
-void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, double scale, cudaStream_t st,
+void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, double scale, cudaStream_t st,
                  int threads = 256);
 
 template <typename R>
@@ -175,18 +170,9 @@ struct ProdArgs {
   const double2 *us, *ws;
   int nps;
 };
-// What the product pass transforms with: FP32 half- and full-length plans and the half-length form's twiddles, or the
-// fixed-point plan and interpolation weights of FP64.
-template <typename R> struct XPlan {
-  FftPlan ph, pf;
-  const double2* rtw;
-};
-template <> struct XPlan<double> {
-  FxPlan pf;
-  const int4 *wc, *wf;  // wc, wf of the product arguments as (high, low word, k): m 2^k with 62 fractional bits of m
-};
 template <typename R>
-void launch_xprod(const ProdArgs<R>& a, const Dims& d, const XPlan<R>& p, cudaStream_t st);
+void launch_xprod(const ProdArgs<R>& a, const Dims& d, const FftPlan& ph, const FftPlan& pf, const double2* rtw,
+                  cudaStream_t st);
 
 template <typename R>
 struct MaskArgs {
@@ -197,16 +183,8 @@ struct MaskArgs {
   int nplanes[3];
   double beta;
 };
-// What the canopy forcing transforms rows with: FP32 half-length plan and twiddles, or the fixed-point plan of FP64.
-template <typename R> struct MaskPlan {
-  FftPlan ph;
-  const double2* rtw;
-};
-template <> struct MaskPlan<double> {
-  FxPlan pf;
-};
 template <typename R>
-void launch_xmask(const MaskArgs<R>& a, const Dims& d, const MaskPlan<R>& p, cudaStream_t st);
+void launch_xmask(const MaskArgs<R>& a, const Dims& d, const FftPlan& ph, const double2* rtw, cudaStream_t st);
 
 struct AsmArgs {
   const double2 *u1, *u2, *u3, *p;
@@ -221,8 +199,8 @@ struct AsmArgs {
   double C1, C2, d, g, dt, beta;
   int k;                     // substage index 0..2 (selects 1/axz)
 };
+constexpr int kAsmThreads = 64;  // of an assembly CTA
 void launch_assemble(const AsmArgs& a, const Dims& d, const Tables& t, cudaStream_t st);
-void assemble_shape(const Dims& d, bool fp32_products, int* gx, int* gy, int* levels);
 
 void launch_vsolve(double2* r1, double2* r2, double2* r3, double2* u1, double2* u2, double2* u3,
                    const Dims& d, const Tables& t, int k, cudaStream_t st);
@@ -279,7 +257,7 @@ template <typename R>
 struct ZDesc {                  // z-inverse or z-forward
   ZJobs<R> jobs;
   Dims d;
-  ZPlan<R> p;
+  FftPlan p;
   double scale;
   int tx, gx, gy, gz;
 };
@@ -287,21 +265,23 @@ template <typename R>
 struct XDesc {                  // x pass with the products
   ProdArgs<R> a;
   Dims d;
-  XPlan<R> p;
+  FftPlan ph, pf;
+  const double2* rtw;
   int gx, gy;
 };
 template <typename R>
 struct MDesc {                  // canopy forcing x pass
   MaskArgs<R> a;
   Dims d;
-  MaskPlan<R> p;
+  FftPlan ph;
+  const double2* rtw;
   int gx, gy;
 };
 struct ADesc {                  // right-hand-side assembly
   AsmArgs a;
   Dims d;
   Tables t;
-  int gx, gy, levels;
+  int gx, gy;
 };
 struct VDesc {                  // velocity Thomas sweeps
   double2 *r1, *r2, *r3, *u1, *u2, *u3;
@@ -352,11 +332,8 @@ void launch_psolve_batch(const Batch<PDesc>& b, size_t smem, cudaStream_t st);
 // grid means no launch).
 template <typename R>
 void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem);
-template <typename R>
-int zpass_tile(int tx);
-// Product-pass CTAs of `rows` z rows and at most `threads` threads resident on an SM, from their threads, registers and
-// shared memory.
-template <typename R>
+// CTAs of the mixed form's product pass, of `rows` z rows and `threads` threads, that an SM holds at once (after
+// configure_kernels).
 int xprod_ctas_per_sm(const Dims& d, int rows, int threads);
 template <typename R>
 void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem);

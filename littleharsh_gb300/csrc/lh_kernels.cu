@@ -34,10 +34,9 @@ namespace lh {
 // z passes
 // ---------------------------------------------------------------------------
 
-// FP32 (the mixed form)
-__device__ __forceinline__ void zinv_body(const ZJobs<float>& jobs, const Dims& d, const FftPlan& pz, int tx, int bx,
+template <typename R>
+__device__ __forceinline__ void zinv_body(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, int bx,
                                           int by, int bz) {
-  using R = float;
   using T2 = cpx_t<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* sm = reinterpret_cast<T2*>(smraw);  // [ngz][tx]
@@ -72,9 +71,15 @@ __device__ __forceinline__ void zinv_body(const ZJobs<float>& jobs, const Dims& 
   }
 }
 
-__device__ __forceinline__ void zfwd_body(const ZJobs<float>& jobs, const Dims& d, const FftPlan& pz, int tx,
-                                          double scale, int bx, int by, int bz) {
-  using R = float;
+template <typename R>
+__global__ void __launch_bounds__(256) k_zinv(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
+                                              const __grid_constant__ FftPlan pz, int tx) {
+  zinv_body<R>(jobs, d, pz, tx, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+template <typename R>
+__device__ __forceinline__ void zfwd_body(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, double scale,
+                                          int bx, int by, int bz) {
   using T2 = cpx_t<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* sm = reinterpret_cast<T2*>(smraw);  // [ngz][tx]
@@ -95,19 +100,21 @@ __device__ __forceinline__ void zfwd_body(const ZJobs<float>& jobs, const Dims& 
   // stage's output is never read when N2/2 = Ngz/3
   fft_dit<R, -1, true>(sm, nb, tx, 1, pz, pz.prune_mid != 0);
   const int h = d.nz / 2, gap = d.ngz - d.nz;
-  if (J.out32) {  // the mixed form's product spectra stay FP32 (only the nonlinear term reads them)
-    T2* __restrict__ dst = reinterpret_cast<T2*>(J.spec_out) + (size_t)lev * d.np;
-    const R sc = (R)scale;
-    for (int e = threadIdx.x; e < d.nz * tx; e += blockDim.x) {
-      const int kk = e / tx, c = e - kk * tx;
-      if (c < nb) {
-        const int slot = kk < h ? kk : kk + gap;
-        const T2 v = sm[slot * tx + c];
-        const int ks = kk < h ? kk : kk - d.nz + d.snz;
-        dst[(size_t)ks * d.spitch + i0 + c] = T2{v.x * sc, v.y * sc};
+  if constexpr (sizeof(R) == 4) {
+    if (J.out32) {  // the mixed form's product spectra stay FP32 (only the nonlinear term reads them)
+      T2* __restrict__ dst = reinterpret_cast<T2*>(J.spec_out) + (size_t)lev * d.np;
+      const R sc = (R)scale;
+      for (int e = threadIdx.x; e < d.nz * tx; e += blockDim.x) {
+        const int kk = e / tx, c = e - kk * tx;
+        if (c < nb) {
+          const int slot = kk < h ? kk : kk + gap;
+          const T2 v = sm[slot * tx + c];
+          const int ks = kk < h ? kk : kk - d.nz + d.snz;
+          dst[(size_t)ks * d.spitch + i0 + c] = T2{v.x * sc, v.y * sc};
+        }
       }
+      return;
     }
-    return;
   }
   double2* __restrict__ dst = J.spec_out + (size_t)lev * d.np;
   for (int e = threadIdx.x; e < d.nz * tx; e += blockDim.x) {
@@ -121,14 +128,47 @@ __device__ __forceinline__ void zfwd_body(const ZJobs<float>& jobs, const Dims& 
   }
 }
 
-// FP64: the lines of a tile of columns in 64-bit fixed point (lh_fxfft.cuh).  The tile is copied into shared memory
-// (cp.async: all of it in flight at once; reading it through registers, once for the largest value and once to scale,
-// waited on global memory and took 1.4x as long), a sweep finds each column's largest value, the first pass scales its
-// inputs and the last one writes FP64.  Bound by instruction issue (340 instructions a point, 50-60 % issue) on the
-// integer pipes; the conversions run beside them on the FP64 pipe, in zinv both ways, in zfwd outward with the
-// normalisation (its inputs take integer shifts, or the FP64 pipe would be the bound).  64 registers (four CTAs of 256
-// threads) beat 80.  A step of the 576 x 576 x 450 grid (449 levels transformed) on a GB300: z-inverse 22.9 -> 5.7 ms,
-// z-forward 47.8 -> 11.3 ms against FP64 radix-4/3 butterflies; their memory traffic alone is 1.8 and 3.5 ms.
+template <typename R>
+__global__ void __launch_bounds__(256) k_zfwd(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
+                                              const __grid_constant__ FftPlan pz, int tx, double scale) {
+  zfwd_body<R>(jobs, d, pz, tx, scale, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+template <typename R>
+void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem) {
+  *grid = (jobs.njobs == 0 || jobs.maxlev == 0) ? dim3(0, 0, 0) : dim3((d.nkx + tx - 1) / tx, jobs.maxlev, jobs.njobs);
+  *smem = sizeof(cpx_t<R>) * (size_t)d.ngz * tx;
+}
+
+template <typename R>
+void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, cudaStream_t st, int threads) {
+  dim3 grid;
+  size_t sm;
+  zpass_shape(jobs, d, tx, &grid, &sm);
+  if (grid.x == 0) return;
+  k_zinv<R><<<grid, threads == 128 ? 128 : 256, sm, st>>>(jobs, d, pz, tx);
+}
+
+template <typename R>
+void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx, double scale, cudaStream_t st,
+                 int threads) {
+  dim3 grid;
+  size_t sm;
+  zpass_shape(jobs, d, tx, &grid, &sm);
+  if (grid.x == 0) return;
+  k_zfwd<R><<<grid, threads == 128 ? 128 : 256, sm, st>>>(jobs, d, pz, tx, scale);
+}
+
+// The z-inverse of the conditional statistics: the lines of a tile of columns in 64-bit fixed point (lh_fxfft.cuh).  Only
+// sums that no later step reads come out of it.  The step itself keeps the FP64 butterflies: its last bits, down to the
+// plane mean of v, which is rounding alone, are part of established runs.
+//
+// The tile is copied into shared memory (cp.async: all of it in flight at once; reading it through registers, once for the
+// largest value and once to scale, waited on global memory and took 1.4x as long), a sweep finds each column's largest
+// value, the first pass scales its inputs and the last one writes FP64.  Bound by instruction issue (340 instructions a
+// point, 50-60 % issue) on the integer pipes; the conversions run beside them on the FP64 pipe.  64 registers (four CTAs of
+// 256 threads) beat 80.  An accumulation of the conditional statistics, ms, with FP64 butterflies / with this: 48 x 48 x 66
+// 0.126 / 0.114, 96 x 96 x 130 0.43 / 0.38, 288 x 288 x 226 4.16 / 3.43, 576 x 576 x 450 32.0 / 25.4.
 
 constexpr int kFxMaxTile = 32;  // columns of a tile (a power of two)
 
@@ -171,16 +211,16 @@ __device__ __forceinline__ FxCol fx_col(fx2* sm, int tx) {
   return FxCol{sm + c, ltx, (int)threadIdx.x >> ltx, (int)blockDim.x >> ltx};
 }
 
-__device__ __forceinline__ void zinv_body(const ZJobs<double>& jobs, const Dims& d, const FxPlan& P, int tx, int bx,
-                                          int by, int bz) {
+__global__ void __launch_bounds__(256, 4) k_zinv_fx(const __grid_constant__ ZJobs<double> jobs, const __grid_constant__ Dims d,
+                                                    const __grid_constant__ FxPlan P, int tx) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ FxLines L;
-  const ZJob<double> J = jobs.j[bz];
-  const int y = by;
+  const ZJob<double> J = jobs.j[blockIdx.z];
+  const int y = blockIdx.y;
   if (y >= J.nlev) return;
   const int lev = J.levels ? J.levels[y] : J.lev0 + y;
   const FxCol C = fx_col(reinterpret_cast<fx2*>(smraw), tx);  // [ngz][tx]
-  const int i = bx * tx + (threadIdx.x & (tx - 1));
+  const int i = blockIdx.x * tx + (threadIdx.x & (tx - 1));
   const bool in = i < d.nkx;
   const double2* __restrict__ src = J.spec_in + (size_t)lev * d.np + i;
   const int h = d.nz / 2, gap = d.ngz - d.nz, pitch = d.spitch;
@@ -218,100 +258,17 @@ __device__ __forceinline__ void zinv_body(const ZJobs<double>& jobs, const Dims&
   fx_tile(C, P, load, total, store);
 }
 
-__device__ __forceinline__ void zfwd_body(const ZJobs<double>& jobs, const Dims& d, const FxPlan& P, int tx,
-                                          double norm, int bx, int by, int bz) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ FxLines L;
-  const ZJob<double> J = jobs.j[bz];
-  const int y = by;
-  if (y >= J.nlev) return;
-  const int lev = J.levels ? J.levels[y] : J.lev0 + y;
-  const FxCol C = fx_col(reinterpret_cast<fx2*>(smraw), tx);  // [ngz][tx]
-  const int i = bx * tx + (threadIdx.x & (tx - 1));
-  const bool in = i < d.nkx;
-  const double2* __restrict__ src = J.mix + (size_t)y * d.mp + i;
-#pragma unroll 4
-  for (int z = C.t0; z < d.ngz; z += C.dt) {
-    fx2* s = C.buf + ((int)P.pos_sample[z] << C.ltx);
-    if (in) fx_copy(s, src + (size_t)z * d.nkx);
-    else *s = fx2{0, 0};
-  }
-  const int e = fx_sweep(L, C, d.ngz) >> 20;
-  auto load = [&](double2 v) { return fx2{fx_from(v.x, e), fx_from(v.y, e)}; };
-  auto total = [&]() {
-    __syncthreads();
-    return P.shift;
-  };
-  const int h = d.nz / 2, gap = d.ngz - d.nz;
-  double2* __restrict__ dst = J.spec_out + (size_t)lev * d.np + i;
-  double2* __restrict__ top = dst + (ptrdiff_t)(d.snz - d.ngz) * d.spitch;
-  const FxOut out(e, fx_scale(e) - P.shift);
-  // the integers times norm 2^-S in one product
-  const double f = out.bad ? __longlong_as_double(0x7ff8000000000000ll) : norm * __hiloint2double((int)((unsigned)(1023 - out.S) << 20), 0);
-  auto store = [&](int k, fx2 v) {
-    if (!in || (unsigned)(k - h) < (unsigned)gap) return;  // the truncation
-    (k < h ? dst : top)[(ptrdiff_t)k * d.spitch] =
-        out.far && !out.bad ? double2{out(v.x) * norm, out(v.y) * norm}
-                            : double2{__ll2double_rn(v.x) * f, __ll2double_rn(v.y) * f};
-  };
-  fx_tile(C, P, load, total, store);
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zinv(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
-                                              const __grid_constant__ ZPlan<R> pz, int tx) {
-  zinv_body(jobs, d, pz, tx, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zfwd(const __grid_constant__ ZJobs<R> jobs, const __grid_constant__ Dims d,
-                                              const __grid_constant__ ZPlan<R> pz, int tx, double scale) {
-  zfwd_body(jobs, d, pz, tx, scale, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-// Width of the z tile a precision's kernels use: the FP64 ones take a power of two up to 32 (at or below tx).
-template <typename R>
-int zpass_tile(int tx) {
-  if (sizeof(R) == 4) return tx;
-  int p = 1;
-  while (2 * p <= tx && 2 * p <= kFxMaxTile) p *= 2;
-  return p;
-}
-
-template <typename R>
-void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem) {
-  tx = zpass_tile<R>(tx);
-  *grid = (jobs.njobs == 0 || jobs.maxlev == 0) ? dim3(0, 0, 0) : dim3((d.nkx + tx - 1) / tx, jobs.maxlev, jobs.njobs);
-  *smem = sizeof(cpx_t<R>) * (size_t)d.ngz * tx;
-}
-
-// Threads of a z-pass CTA: `threads` (128 or 256), and in FP64 no more than share the tile's radix-8 butterflies evenly
-// over the rounds that many threads need.
-template <typename R>
-int zpass_threads(const Dims& d, int tx, int threads) {
-  threads = threads == 128 ? 128 : 256;
-  if (sizeof(R) == 4) return threads;
-  const int items = std::max(1, d.ngz / 8) * zpass_tile<R>(tx), rounds = (items + threads - 1) / threads;
-  return std::min(threads, ((items + rounds - 1) / rounds + 31) / 32 * 32);
-}
-
-template <typename R>
-void launch_zinv(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, cudaStream_t st, int threads) {
+void launch_zinv_fx(const ZJobs<double>& jobs, const Dims& d, const FxPlan& P, int tx, cudaStream_t st) {
+  int tile = 1;  // the largest power of two up to tx
+  while (2 * tile <= tx && 2 * tile <= kFxMaxTile) tile *= 2;
   dim3 grid;
   size_t sm;
-  zpass_shape(jobs, d, tx, &grid, &sm);
+  zpass_shape(jobs, d, tile, &grid, &sm);
   if (grid.x == 0) return;
-  k_zinv<R><<<grid, zpass_threads<R>(d, tx, threads), sm, st>>>(jobs, d, pz, zpass_tile<R>(tx));
-}
-
-template <typename R>
-void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const ZPlan<R>& pz, int tx, double scale, cudaStream_t st,
-                 int threads) {
-  dim3 grid;
-  size_t sm;
-  zpass_shape(jobs, d, tx, &grid, &sm);
-  if (grid.x == 0) return;
-  k_zfwd<R><<<grid, zpass_threads<R>(d, tx, threads), sm, st>>>(jobs, d, pz, zpass_tile<R>(tx), scale);
+  // no more threads than share the tile's radix-8 butterflies evenly over the rounds that 256 need
+  const int items = std::max(1, d.ngz / 8) * tile, rounds = (items + 255) / 256;
+  const int threads = std::min(256, ((items + rounds - 1) / rounds + 31) / 32 * 32);
+  k_zinv_fx<<<grid, threads, sm, st>>>(jobs, d, P, tile);
 }
 
 // ---------------------------------------------------------------------------
@@ -353,10 +310,10 @@ __device__ void x_inverse(const cpx_t<R>* const* rows, int nr, cpx_t<R>* F, int 
 // Forward real transform of the data already packed in F (z[m] = x[2m] + i
 // x[2m+1] stored at position perm[m]) into nr mixed rows scaled by 1/ngx,
 // kx < nkx kept.
-__device__ void x_forward_packed(int nr, float2* F, int hp, float2* const* rows, const Dims& d,
+template <typename R>
+__device__ void x_forward_packed(int nr, cpx_t<R>* F, int hp, cpx_t<R>* const* rows, const Dims& d,
                                  const FftPlan& ph, const double2* __restrict__ rtw) {
-  using R = float;
-  using T2 = float2;
+  using T2 = cpx_t<R>;
   const int h = d.ngx / 2, nkx = d.nkx;
   const R scale = (R)(1.0 / d.ngx);
   fft_dit<R, -1, false>(F, nr, 1, hp, ph, false);
@@ -383,12 +340,12 @@ __device__ void x_forward_packed(int nr, float2* F, int hp, float2* const* rows,
 // takes the mixed rows A, B (nkx modes, zero beyond, imaginary part of the
 // kx = 0 mode dropped as the real inverse does) as z = a + i b; the forward
 // splits the transform of z = a + i b into the two half spectra.  This costs
-// fewer instructions than two half-length real transforms with their
+// fewer FP64 instructions than two half-length real transforms with their
 // pre/post twiddle passes.
-__device__ void x_inverse_pair(const float2* rowA, const float2* rowB, float2* F, float* outA, float* outB,
+template <typename R>
+__device__ void x_inverse_pair(const cpx_t<R>* rowA, const cpx_t<R>* rowB, cpx_t<R>* F, R* outA, R* outB,
                                const Dims& d, const FftPlan& pf) {
-  using R = float;
-  using T2 = float2;
+  using T2 = cpx_t<R>;
   const int n = d.ngx, nkx = d.nkx;
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     T2 z = T2{0, 0};
@@ -415,9 +372,9 @@ __device__ void x_inverse_pair(const float2* rowA, const float2* rowB, float2* F
 
 // Forward transform of np2 packed pairs F[p*n + perm[x]] = a[x] + i b[x]
 // into 2*np2 mixed rows (kx < nkx, scaled by 1/ngx).
-__device__ void x_forward_pairs(int np2, float2* F, float2* const* rows, const Dims& d, const FftPlan& pf) {
-  using R = float;
-  using T2 = float2;
+template <typename R>
+__device__ void x_forward_pairs(int np2, cpx_t<R>* F, cpx_t<R>* const* rows, const Dims& d, const FftPlan& pf) {
+  using T2 = cpx_t<R>;
   const int n = d.ngx, nkx = d.nkx;
   const R sc = (R)(0.5 / n);
   fft_dit<R, -1, false>(F, np2, 1, n, pf, false);
@@ -431,13 +388,10 @@ __device__ void x_forward_pairs(int np2, float2* F, float2* const* rows, const D
   __syncthreads();
 }
 
-// FP32 (the mixed form)
-__device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims& d, const XPlan<float>& plan, int bx,
-                                           int by) {
-  using R = float;
+template <typename R>
+__device__ __forceinline__ void xprod_body(const ProdArgs<R>& a, const Dims& d, const FftPlan& ph, const FftPlan& pf,
+                                           const double2* __restrict__ rtw, int bx, int by) {
   using T2 = cpx_t<R>;
-  const FftPlan &ph = plan.ph, &pf = plan.pf;
-  const double2* __restrict__ rtw = plan.rtw;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ngx = d.ngx, h = ngx / 2, hp = h + 1;
   // 3 vectors of ngx, 2 with a.split (also holds the half-length v transform)
@@ -460,7 +414,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
   double cmax = 0.0;
   // warm-up: previous centre and face
   if (c0 - 1 >= 1) {
-    x_inverse_pair(a.mu + (size_t)(c0 - 1) * d.mp + rowoff, a.mw + (size_t)(c0 - 1) * d.mp + rowoff, F, up, wp, d,
+    x_inverse_pair<R>(a.mu + (size_t)(c0 - 1) * d.mp + rowoff, a.mw + (size_t)(c0 - 1) * d.mp + rowoff, F, up, wp, d,
                       pf);
     const T2* rows[1] = {a.mv + (size_t)(c0 - 1) * d.mp + rowoff};
     R* outs[1] = {vp};
@@ -471,7 +425,7 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
   }
   for (int jj = c0; jj <= c1; ++jj) {
     const bool vface = jj <= d.nyv - 2;  // face jj interior (else the top wall, v = 0)
-    x_inverse_pair(a.mu + (size_t)jj * d.mp + rowoff, a.mw + (size_t)jj * d.mp + rowoff, F, uc, wc, d, pf);
+    x_inverse_pair<R>(a.mu + (size_t)jj * d.mp + rowoff, a.mw + (size_t)jj * d.mp + rowoff, F, uc, wc, d, pf);
     if (vface) {
       const T2* rows[1] = {a.mv + (size_t)jj * d.mp + rowoff};
       R* outs[1] = {vc};
@@ -489,27 +443,35 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
     // with a.split and both kinds, the face pair goes through the buffer after the centre pairs' transform
     const bool later = a.split && cprod && fprod;
     const int fslot = (cprod && !later) ? 2 : 0;
-    // the level means at centre jj and face jj-1
+    // mixed form: the level means at centre jj and face jj-1 (the FP64 form transforms u and w whole)
     R Uc = (R)0, Wc = (R)0, Uf = (R)0, Wf = (R)0;
-    if (a.mean_split) {
-      const R Um = (R)a.us[(size_t)(jj - 1) * a.nps].x, Wm = (R)a.ws[(size_t)(jj - 1) * a.nps].x;
-      Uc = (R)a.us[(size_t)jj * a.nps].x;
-      Wc = (R)a.ws[(size_t)jj * a.nps].x;
-      Uf = Um + wfj * (Uc - Um);
-      Wf = Wm + wfj * (Wc - Wm);
+    if constexpr (sizeof(R) == 4) {
+      if (a.mean_split) {
+        const R Um = (R)a.us[(size_t)(jj - 1) * a.nps].x, Wm = (R)a.ws[(size_t)(jj - 1) * a.nps].x;
+        Uc = (R)a.us[(size_t)jj * a.nps].x;
+        Wc = (R)a.ws[(size_t)jj * a.nps].x;
+        Uf = Um + wfj * (Uc - Um);
+        Wf = Wm + wfj * (Wc - Wm);
+      }
     }
     auto face_pair = [&](int x, R u, R w, int px) {
       const R uf = up[x] + wfj * (u - up[x]);
       const R wf = wp[x] + wfj * (w - wp[x]);
-      F[sxi<R>(fslot * ngx + px)] = T2{(Uf + uf) * vp[x], (Wf + wf) * vp[x]};
+      if constexpr (sizeof(R) == 4) F[sxi<R>(fslot * ngx + px)] = T2{(Uf + uf) * vp[x], (Wf + wf) * vp[x]};
+      else F[sxi<R>(fslot * ngx + px)] = T2{uf * vp[x], wf * vp[x]};
     };
     for (int x = threadIdx.x; x < ngx; x += blockDim.x) {
       const R u = uc[x], w = wc[x];
       const int px = pf.perm[x];
       if (cprod) {
         const R v = vp[x] + wcj * (vc[x] - vp[x]);
-        F[sxi<R>(px)] = T2{u * ((Uc + Uc) + u), u * (Wc + w) + Uc * w};
-        F[sxi<R>(ngx + px)] = T2{w * ((Wc + Wc) + w), v * v};
+        if constexpr (sizeof(R) == 4) {
+          F[sxi<R>(px)] = T2{u * ((Uc + Uc) + u), u * (Wc + w) + Uc * w};
+          F[sxi<R>(ngx + px)] = T2{w * ((Wc + Wc) + w), v * v};
+        } else {
+          F[sxi<R>(px)] = T2{u * u, u * w};
+          F[sxi<R>(ngx + px)] = T2{w * w, v * v};
+        }
         if (a.want_cfl) {
           const double cv = fabs((double)u) * a.dxi + fabs((double)v) * dyi + fabs((double)w) * a.dzi;
           cmax = fmax(cmax, cv);
@@ -531,12 +493,12 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
         ++npair;
       }
       if (later) {
-        x_forward_pairs(2, F, rows, d, pf);
+        x_forward_pairs<R>(2, F, rows, d, pf);
         for (int x = threadIdx.x; x < ngx; x += blockDim.x) face_pair(x, uc[x], wc[x], pf.perm[x]);
         __syncthreads();
-        x_forward_pairs(1, F, rows + 4, d, pf);
+        x_forward_pairs<R>(1, F, rows + 4, d, pf);
       } else {
-        x_forward_pairs(npair, F, rows, d, pf);
+        x_forward_pairs<R>(npair, F, rows, d, pf);
       }
     }
     // current becomes previous
@@ -557,336 +519,12 @@ __device__ __forceinline__ void xprod_body(const ProdArgs<float>& a, const Dims&
   }
 }
 
-// FP64: the rows in 64-bit fixed point (lh_fxfft.cuh), two levels at a time.
-//
-// Three inverse lines of ngx: (u, w) of level j, (v of j, v of j + 1), (u, w) of j + 1, each two real rows in one complex
-// line.  They come out in 64-bit integers with one scale per line, are shifted to the full range by what their largest
-// value leaves (found by an OR over the magnitudes), interpolated and multiplied as integers, and the products go
-// forward two to a line: (uu, uw), (ww, vv), (uv, vw), each pair on one scale.  They start a bit below a line's range, so
-// that the sums which separate a pair's spectra fit.  The FP64 the rows come from and go to is the kernel's only floating
-// point, but for the CFL number.
-//
-// Bound by instruction issue on the integer pipes (340 instructions a point of a transform, 190 of them the transforms';
-// 51 % issue), no longer by the FP64 pipe.  A step of the 576 x 576 x 450 grid: 140.0 -> 34.0 ms; 288 x 288 x 226 17.8 ->
-// 4.1, 96 x 96 x 130 1.81 -> 0.44, 48 x 48 x 66 0.65 -> 0.10 ms.  Its memory traffic alone is 3 ms.
-//
-// Shared memory: two buffers of three lines that exchange their parts every two levels (the raw FP64 rows and the
-// products in one, the inverse lines in the other: while the last products are transformed, the next rows are copied in
-// where the inverse lines were), and u, w, v of the previous level.
-
-struct FxProd {                // per iteration, twice (an iteration clears the next one's)
-  unsigned e[3], sum[3], bits[6];
-};
-
-__device__ __forceinline__ void fx_reduce_max(unsigned m, unsigned* dst) {
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicMax(dst, m);
+template <typename R>
+__global__ void __launch_bounds__(256) k_xprod(const __grid_constant__ ProdArgs<R> a, const __grid_constant__ Dims d,
+                                               const __grid_constant__ FftPlan ph, const __grid_constant__ FftPlan pf,
+                                               const double2* __restrict__ rtw) {
+  xprod_body<R>(a, d, ph, pf, rtw, blockIdx.x, blockIdx.y);
 }
-__device__ __forceinline__ void fx_reduce_add(unsigned m, unsigned* dst) {
-  m = __reduce_add_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicAdd(dst, m);
-}
-__device__ __forceinline__ void fx_reduce_or(unsigned m, unsigned* dst) {
-  m = __reduce_or_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicOr(dst, m);
-}
-
-// Levels an iteration takes: two where the buffers of six lines fit (all lengths to 1936), else one.
-__host__ __device__ __forceinline__ int xprod_levels(int ngx) { return ngx <= 1936 ? 2 : 1; }
-// Levels of a CTA: whole iterations, so that every level's v has the same partner whatever the chunk.
-__host__ __device__ __forceinline__ int xprod_chunk(int chunk, int ngx) { return xprod_levels(ngx) == 2 ? (chunk + 1) & ~1 : chunk; }
-
-// TWO: two levels an iteration (xprod_levels).
-template <bool TWO>
-__device__ __forceinline__ void xprod_body(const ProdArgs<double>& a, const Dims& d, const XPlan<double>& plan, int bx,
-                                           int by) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ FxProd red[2];
-  __shared__ double cflred[8];
-  const FxPlan& P = plan.pf;
-  const int n = d.ngx, nkx = d.nkx, tid = threadIdx.x, bd = blockDim.x;
-  constexpr int lp = TWO ? 2 : 1, nl = lp + 1;  // levels and lines of an iteration
-  fx2* B0 = reinterpret_cast<fx2*>(smraw);      // nl lines
-  fx2* B1 = B0 + nl * n;                        // nl lines
-  i64* pu = reinterpret_cast<i64*>(B1 + nl * n);  // u, w, v of the previous level
-  i64 *pw = pu + n, *pv = pw + n;
-  const int L0 = min(a.c_lo, a.f_lo + 1), L1 = max(a.c_hi, a.f_hi + 1);
-  const int chunk = xprod_chunk(a.chunk, n), c0 = L0 + by * chunk, c1 = min(c0 + chunk - 1, L1);
-  if (c0 > c1) return;
-  const size_t rowoff = (size_t)bx * nkx;
-  for (int i = tid; i < (int)(2 * sizeof(FxProd) / 4); i += bd) reinterpret_cast<unsigned*>(red)[i] = 0;
-
-  // Copies the FP64 rows of line 0 (u, w of level j), line 1 (v of jv, v of jv + 1) and, for two levels, line 2 (u, w of
-  // j + 1) into raw: row r of line l at raw[(2 l + r) nkx].  A row that does not exist is zero.
-  auto fetch = [&](fx2* raw, int j, bool two, int jv, int v_lo, int v_hi) {
-    const int rows = two ? 6 : 4;
-#pragma unroll 1
-    for (int q = 0; q < rows; ++q) {
-      const bool v = q == 2 || q == 3;
-      const int f = v ? jv + q - 2 : (q < 2 ? j : j + 1);
-      const double2* src = (v ? a.mv : ((q & 1) ? a.mw : a.mu)) + (size_t)f * d.mp + rowoff;
-      const bool none = v && (f < v_lo || f > v_hi);
-      for (int k = tid; k < nkx; k += bd) {
-        if (none) raw[q * nkx + k] = fx2{0, 0};
-        else fx_copy(raw + q * nkx + k, src + k);
-      }
-    }
-  };
-
-  // From the fetched rows to nv lines of integers, transformed, in Z.
-  auto inverse = [&](const fx2* raw, fx2* Z, int nv, FxProd& R, FxProd& next) {
-    const double2* rd = reinterpret_cast<const double2*>(raw);
-    fx_copy_wait();
-    __syncthreads();
-#pragma unroll 1
-    for (int v = 0; v < nv; ++v) {
-      unsigned m = 0;
-      for (int k = tid; k < 2 * nkx; k += bd) m = max(m, fx_hi(rd[2 * v * nkx + k]));
-      fx_reduce_max(m, &R.e[v]);
-    }
-    for (int i = tid; i < (int)(sizeof(FxProd) / 4); i += bd) reinterpret_cast<unsigned*>(&next)[i] = 0;
-    __syncthreads();
-#pragma unroll 1
-    for (int v = 0; v < nv; ++v) {
-      const FxIn in((int)(R.e[v] >> 20) + 1);  // one bit of room: a line's values are sums of two rows'
-      const double2 *ra = rd + 2 * v * nkx, *rb = ra + nkx;
-      fx2* z = Z + v * n;
-      unsigned s = 0;
-      for (int k = tid; k < nkx; k += bd) {
-        const double2 A = ra[k], B = rb[k];
-        const i64 ax = in(A.x), ay = in(A.y), bx2 = in(B.x), by2 = in(B.y);
-        // a + i b at k, its mirror at n - k; the kx = 0 values are real.  Parts exchanged: an inverse transform
-        if (k == 0) {
-          z[P.pos_sample[0]] = fx2{bx2, ax};
-          s += fx_mag(ax) + fx_mag(bx2);
-        } else {
-          const fx2 p = fx2{ay + bx2, ax - by2}, q = fx2{bx2 - ay, ax + by2};
-          z[P.pos_sample[k]] = p;
-          z[P.pos_sample[n - k]] = q;
-          s += fx_mag(p.x) + fx_mag(p.y) + fx_mag(q.x) + fx_mag(q.y);
-        }
-      }
-      for (int k = nkx + tid; k <= n - nkx; k += bd) z[P.pos_sample[k]] = fx2{0, 0};
-      fx_reduce_add(s, &R.sum[v]);
-    }
-    __syncthreads();
-    fx_fft(Z, nv, P, R.sum);
-    // magnitude bits of the real (u, v of the lower level) and the imaginary rows (w, v of the upper one)
-#pragma unroll 1
-    for (int v = 0; v < nv; ++v) {
-      unsigned o0 = 0, o1 = 0;
-      for (int x = tid; x < n; x += bd) {
-        const fx2 z = Z[v * n + x];
-        o0 |= fx_bits(z.y);
-        o1 |= fx_bits(z.x);
-      }
-      fx_reduce_or(o0, &R.bits[2 * v]);
-      fx_reduce_or(o1, &R.bits[2 * v + 1]);
-    }
-    __syncthreads();
-    // a line that kept more than 61 bits (many modes of one size) comes down by two
-    bool over = false;
-    for (int v = 0; v < nv; ++v) {
-      if (!(R.bits[2 * v] >> 29 | R.bits[2 * v + 1] >> 29)) continue;
-      for (int x = tid; x < n; x += bd) Z[v * n + x] = fx2{Z[v * n + x].x >> 2, Z[v * n + x].y >> 2};
-      over = true;
-    }
-    if (over) __syncthreads();
-  };
-  // scale of a line, and the left shift that brings a row of it below 2^61
-  auto over = [&](const FxProd& R, int v) { return (R.bits[2 * v] >> 29 | R.bits[2 * v + 1] >> 29) ? 2 : 0; };
-  auto line_scale = [&](const FxProd& R, int v) {
-    return fx_scale((int)(R.e[v] >> 20) + 1) - fx_inv_shift(R.sum[v], P.shift) - over(R, v);
-  };
-  auto room = [&](const FxProd& R, int row) { return __clz((int)(R.bits[row] >> over(R, row >> 1))) - 3; };
-  auto lost = [&](const FxProd& R, int v) { return R.e[v] >= 0x7ff00000u; };
-
-  constexpr int kNone = 1 << 14;  // scale of a row of zeros: finer than any other
-  int Sp = kNone, Spv = kNone;        // scales of the previous level's u and w, and of its v
-  bool badp = false, badpv = false;
-  double cmax = 0.0;
-  int it = 0;
-  fx2 *raw = B0, *Z = B1;
-  const int v_top = d.nyv - 2;
-  const int j0 = c0 - 1;
-  if (j0 >= 1) {  // the previous level; its v in the pair it has in the chunk below
-    const bool paired = lp == 2 && j0 - 1 >= L0;
-    const int jv = paired ? j0 - 1 : j0;
-    fetch(raw, j0, false, jv, max(jv, 1), paired ? min(v_top, j0) : min(v_top, jv));
-    __syncthreads();  // red is cleared
-    inverse(raw, Z, 2, red[0], red[1]);
-    const FxProd& R = red[0];
-    const int s0 = min(room(R, 0), room(R, 1)), sv = room(R, paired ? 3 : 2);
-    for (int x = tid; x < n; x += bd) {
-      const fx2 z = Z[x], zv = Z[n + x];
-      pu[x] = fx_shl(z.y, s0);
-      pw[x] = fx_shl(z.x, s0);
-      pv[x] = fx_shl(paired ? zv.x : zv.y, sv);
-    }
-    Sp = line_scale(R, 0) + s0;
-    Spv = line_scale(R, 1) + sv;
-    badp = lost(R, 0);
-    badpv = lost(R, 1);
-    it = 1;
-  } else {
-    for (int x = tid; x < 3 * n; x += bd) pu[x] = 0;
-  }
-  __syncthreads();
-  fetch(raw, c0, lp == 2 && c0 < c1, c0, 1, min(v_top, lp == 2 && c0 < c1 ? c0 + 1 : c0));
-  for (int j = c0; j <= c1; j += lp, ++it) {
-    const bool two = lp == 2 && j < c1;
-    FxProd& R = red[it & 1];
-    inverse(raw, Z, two ? 3 : 2, R, red[(it + 1) & 1]);
-#pragma unroll 1
-    for (int q = 0; q < (two ? 2 : 1); ++q) {
-      const int jj = j + q;
-      const bool cprod = jj >= a.c_lo && jj <= a.c_hi;
-      const bool fprod = jj - 1 >= a.f_lo && jj - 1 <= a.f_hi;  // face jj-1 interior and in this launch
-      const bool vface = jj <= v_top;
-      const int vu = q == 0 ? 0 : 2;
-      // u and w share their line's scale, as far left as the larger allows: (uu, uw) and (uv, vw) are pairs of one scale.
-      // (ww, vv) is a pair of its own: w by its own size, on the coarser of its scale and v's
-      const int S = line_scale(R, vu), rw = room(R, 2 * vu + 1), s0 = min(room(R, 2 * vu), rw), sv = room(R, 2 + q);
-      const int Sc = S + s0, Sv = vface ? line_scale(R, 1) + sv : kNone;
-      const bool bad = lost(R, vu), badv = lost(R, 1);
-      const int4 wc = plan.wc[jj], wf = fprod ? plan.wf[jj - 1] : int4{0, 0, 0, 0};
-      // interpolated values on the coarser scale of the two levels (weights beyond [-1, 1] want more room)
-      const int T1 = min(S + rw, min(Spv, Sv)) - (wc.z ? wc.z + 1 : 0), Tf = min(Sp, Sc) - (wf.z ? wf.z + 1 : 0);
-      const int dw = min(S + rw - T1, 63), dvp = min(Spv - T1, 63), dvc = min(Sv - T1, 63);
-      const int dp = min(Sp - Tf, 63), dc = min(Sc - Tf, 63);
-      const bool shift1 = (dw | dvp | dvc) != 0, shiftf = (dp | dc) != 0;
-      const int S0 = 2 * Sc - 64, S1 = 2 * T1 - 64, S2 = Tf + Spv - 64;  // the pairs' scales
-      const FxOut outc(0, Sc), out1(0, T1);  // of the CFL number
-      fx2* F = raw;
-      int np = 0;                        // lines transformed forward at once
-      const int f0 = 0, f1 = cprod ? 2 : 0;
-      const bool split = !TWO && cprod && fprod;  // the face pair after the centre pairs
-      auto face = [&](int x, i64 u, i64 w, int slot) {
-        i64 up = pu[x], wp = pw[x];
-        if (shiftf) { up >>= dp; wp >>= dp; u >>= dc; w >>= dc; }
-        i64 du = fx_mul<0, 2>(u - up, wf.x, wf.y), dwf = fx_mul<0, 2>(w - wp, wf.x, wf.y);
-        if (wf.z) { du = fx_shl(du, wf.z); dwf = fx_shl(dwf, wf.z); }
-        const i64 v = pv[x];
-        F[slot * n + P.turn[x]] = fx2{fx_prod(up + du, v), fx_prod(wp + dwf, v)};
-      };
-#pragma unroll 1
-      for (int x = tid; x < n; x += bd) {
-        const fx2 z = Z[vu * n + x], zv = Z[n + x];
-        const i64 u = fx_shl(z.y, s0), w = fx_shl(z.x, s0);
-        const i64 v = vface ? fx_shl(q == 0 ? zv.y : zv.x, sv) : 0;
-        if (cprod) {
-          i64 w1 = fx_shl(z.x, rw), vp = pv[x], v1 = v;
-          if (shift1) { w1 >>= dw; vp >>= dvp; v1 >>= dvc; }
-          i64 dv = fx_mul<0, 2>(v1 - vp, wc.x, wc.y);
-          if (wc.z) dv = fx_shl(dv, wc.z);
-          const i64 vc = vp + dv;
-          if (a.want_cfl) {
-            if (!bad && !badv && !badpv)
-              cmax = fmax(cmax, fabs(outc(u)) * a.dxi + fabs(out1(vc)) * a.dyc[jj] + fabs(outc(w)) * a.dzi);
-          } else {
-            const int px = P.turn[x];
-            F[px] = fx2{fx_prod(u, u), fx_prod(u, w)};
-            F[n + px] = fx2{fx_prod(w1, w1), fx_prod(vc, vc)};
-          }
-        }
-        if (fprod && !split && !a.want_cfl) face(x, u, w, f1);
-        if (!split) {
-          pu[x] = u;
-          pw[x] = w;
-          pv[x] = v;
-        }
-      }
-      __syncthreads();
-      if (q == (two ? 1 : 0) && !split && j + lp <= c1) {  // the lines in Z are done with: the next rows take their place
-        const int jn = j + lp;
-        const bool tn = lp == 2 && jn < c1;
-        fetch(Z, jn, tn, jn, 1, min(v_top, tn ? jn + 1 : jn));
-      }
-      auto forward = [&](int lines, int first) {  // pairs first.. of this level
-        fx_fft(F, lines, P, nullptr);
-#pragma unroll 1
-        for (int p = 0; p < lines; ++p) {
-          const int pair = first + p;
-          const bool centre = cprod && pair < 2;
-          // a pair's spectra come doubled out of the sums below
-          const int S = (centre ? (pair == 0 ? S0 : S1) : S2) - P.shift + 1;
-          const bool nan = centre ? (bad || (pair == 1 && (badv || badpv))) : (bad || badp || badpv);
-          const FxOut out(0, S);
-          const size_t o = (size_t)(centre ? jj : jj - 1) * d.mp + rowoff;
-          const int r0 = centre ? 2 * pair : 4;
-          double2 *oa = a.out[r0] + o, *ob = a.out[r0 + 1] + o;
-          const fx2* f = F + p * n;
-          for (int k = tid; k < nkx; k += bd) {
-            const fx2 zk = f[P.pos_freq[k]], zc = f[P.pos_freq[k ? n - k : 0]];
-            double2 A = double2{out(zk.x + zc.x), out(zk.y - zc.y)}, B = double2{out(zk.y + zc.y), out(zc.x - zk.x)};
-            if (nan) A = B = double2{__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll)};
-            oa[k] = A;
-            ob[k] = B;
-          }
-        }
-        __syncthreads();
-      };
-      if (!a.want_cfl) {
-        np = (cprod ? 2 : 0) + (fprod && !split ? 1 : 0);
-        if (np) forward(np, f0);
-        if (split) {
-          for (int x = tid; x < n; x += bd) {
-            const fx2 z = Z[vu * n + x], zv = Z[n + x];
-            const i64 u = fx_shl(z.y, s0), w = fx_shl(z.x, s0);
-            face(x, u, w, 0);
-            pu[x] = u;
-            pw[x] = w;
-            pv[x] = vface ? fx_shl(q == 0 ? zv.y : zv.x, sv) : 0;
-          }
-          __syncthreads();
-          forward(1, 2);
-        }
-      }
-      if (split && j + lp <= c1) {
-        const int jn = j + lp;
-        fetch(Z, jn, false, jn, 1, min(v_top, jn));
-      }
-      Sp = Sc;
-      Spv = Sv;
-      badp = bad;
-      badpv = badv;
-    }
-    fx2* t = raw;
-    raw = Z;
-    Z = t;
-  }
-  if (a.want_cfl) {
-    for (int o = 16; o > 0; o >>= 1) cmax = fmax(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
-    if ((tid & 31) == 0) cflred[tid >> 5] = cmax;
-    __syncthreads();
-    if (tid == 0) {
-      double m = 0.0;
-      for (int w = 0; w < (bd >> 5); ++w) m = fmax(m, cflred[w]);
-      atomicMax(&a.sc->cflbits, (unsigned long long)__double_as_longlong(m));
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) k_xprod(const __grid_constant__ ProdArgs<float> a, const __grid_constant__ Dims d,
-                                               const __grid_constant__ XPlan<float> p) {
-  xprod_body(a, d, p, blockIdx.x, blockIdx.y);
-}
-
-// Threads at most, and registers: 80 a thread let an SM hold 24 warps, 96 (no spills) 20.  CTAs of 96 to 192 threads do
-// better with 96 (288 x 288 x 226, 128 threads: 4.1 ms against 4.6), the others with 80 (96 x 96 x 130, 64 threads: 0.44
-// against 0.46; 576 x 576 x 450, 224 threads: 34.0 against 37.2).
-constexpr int kFxThreads = 224;
-template <bool TWO>
-__global__ void __launch_bounds__(kFxThreads, 3) k_xprod_fx(const __grid_constant__ ProdArgs<double> a,
-                                                            const __grid_constant__ Dims d,
-                                                            const __grid_constant__ XPlan<double> p) {
-  xprod_body<TWO>(a, d, p, blockIdx.x, blockIdx.y);
-}
-__global__ void __maxnreg__(96) k_xprod_fx96(const __grid_constant__ ProdArgs<double> a, const __grid_constant__ Dims d,
-                                             const __grid_constant__ XPlan<double> p) {
-  xprod_body<true>(a, d, p, blockIdx.x, blockIdx.y);
-}
-__host__ __device__ constexpr bool xprod_wide(int threads) { return threads >= 96 && threads <= 192; }
 
 // ---- the FP32 product pass on two z rows per CTA --------------------------------------------------------
 // The same work as xprod_body for the rows 2 bx and 2 bx + 1, their transforms run in lockstep (fft_dit2):
@@ -1103,16 +741,9 @@ __device__ __forceinline__ void xprod2_body(const ProdArgs<float>& a, const Dims
 }
 
 __global__ void __launch_bounds__(256) k_xprod2(const __grid_constant__ ProdArgs<float> a,
-                                                const __grid_constant__ Dims d, const __grid_constant__ XPlan<float> p) {
-  xprod2_body(a, d, p.ph, p.pf, p.rtw, blockIdx.x, blockIdx.y);
-}
-
-// Threads of a product-pass CTA: `threads` (128 or 256), and in FP64 no more than its three lines have radix-8
-// butterflies.
-template <typename R>
-int xprod_threads(const Dims& d, int threads) {
-  threads = threads == 128 ? 128 : 256;
-  return sizeof(R) == 4 ? threads : std::min({threads, kFxThreads, (3 * d.ngx / 8 + 31) / 32 * 32});
+                                                const __grid_constant__ Dims d, const __grid_constant__ FftPlan ph,
+                                                const __grid_constant__ FftPlan pf, const double2* __restrict__ rtw) {
+  xprod2_body(a, d, ph, pf, rtw, blockIdx.x, blockIdx.y);
 }
 
 template <typename R>
@@ -1124,55 +755,45 @@ void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem) 
     *smem = sizeof(float4) * sx_elems<float>(3 * (size_t)d.ngx) + sizeof(float2) * 6 * (size_t)d.ngx;
     return;
   }
-  const int chunk = sizeof(R) == 8 ? xprod_chunk(a.chunk, d.ngx) : a.chunk;
-  *grid = nlev <= 0 ? dim3(0, 0, 0) : dim3(d.ngz, (nlev + chunk - 1) / chunk);
-  if (sizeof(R) == 8) *smem = (2 * (xprod_levels(d.ngx) + 1) * sizeof(fx2) + 3 * sizeof(i64)) * (size_t)d.ngx;
-  else *smem = sizeof(cpx_t<R>) * sx_elems<R>((a.split ? 2 : 3) * (size_t)d.ngx) + sizeof(R) * 6 * (size_t)d.ngx;
+  *grid = nlev <= 0 ? dim3(0, 0, 0) : dim3(d.ngz, (nlev + a.chunk - 1) / a.chunk);
+  *smem = sizeof(cpx_t<R>) * sx_elems<R>((a.split ? 2 : 3) * (size_t)d.ngx) + sizeof(R) * 6 * (size_t)d.ngx;
 }
 
-template <typename R>
 int xprod_ctas_per_sm(const Dims& d, int rows, int threads) {
-  ProdArgs<R> a{};
+  ProdArgs<float> a{};
   a.chunk = 2;
   a.rows = rows;
   dim3 grid;
   size_t smem;
   xprod_shape(a, d, &grid, &smem);
-  threads = xprod_threads<R>(d, threads);
-  const int regs = sizeof(R) == 8 ? (xprod_wide(threads) ? 96 : 80) : (rows == 2 ? 48 : 40);  // of the kernels
-  const int by_regs = 65536 / (regs * threads), by_smem = (int)(233472 / (smem + 1024 + 256));
-  return std::max(1, std::min({32, 2048 / threads, by_regs, by_smem}));
+  int n = 0;
+  if (rows == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_xprod2, threads, smem);
+  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_xprod<float>, threads, smem);
+  return std::max(1, n);
 }
 
 template <typename R>
-void launch_xprod(const ProdArgs<R>& a, const Dims& d, const XPlan<R>& p, cudaStream_t st) {
+void launch_xprod(const ProdArgs<R>& a, const Dims& d, const FftPlan& ph, const FftPlan& pf, const double2* rtw,
+                  cudaStream_t st) {
   dim3 grid;
   size_t sm;
   xprod_shape(a, d, &grid, &sm);
   if (grid.x == 0) return;
   if constexpr (sizeof(R) == 4) {
     if (a.rows == 2) {
-      k_xprod2<<<grid, a.threads == 128 ? 128 : 256, sm, st>>>(a, d, p);
+      k_xprod2<<<grid, a.threads == 128 ? 128 : 256, sm, st>>>(a, d, ph, pf, rtw);
       return;
     }
   }
-  if constexpr (sizeof(R) == 4) k_xprod<<<grid, xprod_threads<R>(d, a.threads), sm, st>>>(a, d, p);
-  else {
-    const int threads = xprod_threads<R>(d, a.threads);
-    if (xprod_levels(d.ngx) == 1) k_xprod_fx<false><<<grid, threads, sm, st>>>(a, d, p);
-    else if (xprod_wide(threads)) k_xprod_fx96<<<grid, threads, sm, st>>>(a, d, p);
-    else k_xprod_fx<true><<<grid, threads, sm, st>>>(a, d, p);
-  }
+  k_xprod<R><<<grid, a.threads == 128 ? 128 : 256, sm, st>>>(a, d, ph, pf, rtw);
 }
 
 // Canopy forcing on one mixed row of one processed plane: x-inverse, solid
 // points set to 0 (or -beta*Luy on the tip planes), x-forward.
-__device__ __forceinline__ void xmask_body(const MaskArgs<float>& a, const Dims& d, const MaskPlan<float>& p, int bx,
-                                           int by) {
-  using R = float;
-  using T2 = float2;
-  const FftPlan& ph = p.ph;
-  const double2* __restrict__ rtw = p.rtw;
+template <typename R>
+__device__ __forceinline__ void xmask_body(const MaskArgs<R>& a, const Dims& d, const FftPlan& ph,
+                                           const double2* __restrict__ rtw, int bx, int by) {
+  using T2 = cpx_t<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ngx = d.ngx, h = ngx / 2, hp = h + 1;
   T2* F = reinterpret_cast<T2*>(smraw);
@@ -1211,165 +832,30 @@ __device__ __forceinline__ void xmask_body(const MaskArgs<float>& a, const Dims&
   }
   __syncthreads();
   T2* rows[1] = {row};
-  x_forward_packed(1, F, hp, rows, d, ph, rtw);
-}
-
-// FP64: two z rows of a plane as one complex line in 64-bit fixed point (lh_fxfft.cuh).  The rows come out of the inverse
-// transform on one scale and are masked on one of their own each, two bits below a line's range.  On the tip planes the
-// Laplacian's rows are transformed first and leave their values at the solid points; the field's then fill the others, all
-// on the coarser of the two scales.  A row without solid points takes no part: its partner is paired with zeros.
-//
-// Bound by instruction issue on the integer pipes, on small grids by latency; FP64 butterflies on half-length real rows
-// kept the FP64 pipe busy.  A step of the 576 x 576 x 450 grid: 4.91 -> 1.52 ms; 288 x 288 x 226 0.42 -> 0.18,
-// 96 x 96 x 130 0.113 -> 0.078, 48 x 48 x 66 0.051 -> 0.050.
-struct FxMask {            // line 0: the field, line 1: its Laplacian
-  unsigned e[2], sum[2], bits[4];
-};
-__device__ __forceinline__ void xmask_body(const MaskArgs<double>& a, const Dims& d, const MaskPlan<double>& plan, int bx,
-                                           int by) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ FxMask red;
-  const FxPlan& P = plan.pf;
-  const int n = d.ngx, nkx = d.nkx, tid = threadIdx.x, bd = blockDim.x;
-  fx2 *Z = reinterpret_cast<fx2*>(smraw), *F = Z + n;
-  const int kz = 2 * bx;
-  const bool second = kz + 1 < d.ngz;
-  int pl = by, f = 0;
-  while (f < 2 && pl >= a.nplanes[f]) { pl -= a.nplanes[f]; ++f; }
-  double2* const row = a.mix + (size_t)by * d.mp + (size_t)kz * nkx;
-  const int tip = a.tipslot[f][pl];
-  const uint8_t* const m0 = a.mask[f] + ((size_t)pl * d.ngz + kz) * n;
-  const uint8_t* const m1 = m0 + (second ? n : 0);
-  for (int i = tid; i < (int)(sizeof(FxMask) / 4); i += bd) reinterpret_cast<unsigned*>(&red)[i] = 0;
-  // a row without solid points is unchanged by the forcing: its x round trip only drops the imaginary
-  // part of its kx = 0 value (the real inverse ignores it), so that is all it needs
-  int any0 = 0, any1 = 0;
-  for (int x = tid; x < n; x += bd) {
-    any0 |= m0[x];
-    any1 |= m1[x];
-  }
-  const bool on0 = __syncthreads_or(any0), on1 = __syncthreads_or(any1) && second;
-  if (tid == 0) {
-    if (!on0) row[0].y = 0.0;
-    if (second && !on1) row[nkx].y = 0.0;
-  }
-  if (!on0 && !on1) return;
-
-  // rows ra, ra + nkx times mul to a transformed line in Z
-  auto inverse = [&](const double2* ra, double mul, int v) {
-    auto value = [&](int q, int k) {
-      double2 r = (q == 0 ? on0 : on1) ? ra[q * nkx + k] : double2{0.0, 0.0};
-      if (v) r = double2{mul * r.x, mul * r.y};
-      if (k == 0) r.y = 0.0;
-      return r;
-    };
-    unsigned m = 0;
-    for (int k = tid; k < nkx; k += bd) m = max(m, max(fx_hi(value(0, k)), fx_hi(value(1, k))));
-    fx_reduce_max(m, &red.e[v]);
-    __syncthreads();
-    const FxIn in((int)(red.e[v] >> 20) + 1);  // one bit of room: a line's values are sums of two rows'
-    unsigned s = 0;
-    for (int k = tid; k < nkx; k += bd) {
-      const double2 A = value(0, k), B = value(1, k);
-      const i64 ax = in(A.x), ay = in(A.y), bx2 = in(B.x), by2 = in(B.y);
-      // a + i b at k, its mirror at n - k.  Parts exchanged: an inverse transform
-      const fx2 p = fx2{ay + bx2, ax - by2}, q = fx2{bx2 - ay, ax + by2};
-      Z[P.pos_sample[k]] = p;
-      s += fx_mag(p.x) + fx_mag(p.y);
-      if (k) {
-        Z[P.pos_sample[n - k]] = q;
-        s += fx_mag(q.x) + fx_mag(q.y);
-      }
-    }
-    for (int k = nkx + tid; k <= n - nkx; k += bd) Z[P.pos_sample[k]] = fx2{0, 0};
-    fx_reduce_add(s, &red.sum[v]);
-    __syncthreads();
-    fx_fft(Z, 1, P, &red.sum[v]);
-    unsigned o0 = 0, o1 = 0;
-    for (int x = tid; x < n; x += bd) {
-      const fx2 z = Z[x];
-      o0 |= fx_bits(z.y);
-      o1 |= fx_bits(z.x);
-    }
-    fx_reduce_or(o0, &red.bits[2 * v]);
-    fx_reduce_or(o1, &red.bits[2 * v + 1]);
-    __syncthreads();
-  };
-  // the left shift (right if negative) that brings row q of line v below 2^58, and the row's scale after it
-  auto room = [&](int v, int q) { return __clz((int)red.bits[2 * v + q]) - 6; };
-  auto scale = [&](int v, int q) {
-    return fx_scale((int)(red.e[v] >> 20) + 1) - fx_inv_shift(red.sum[v], P.shift) + room(v, q);
-  };
-  auto shifted = [](i64 x, int s) { return s >= 0 ? fx_shl(x, s) : x >> -s; };
-  auto solid = [&](const uint8_t* m, int x) { return m[P.freq_pos[x]] != 0; };
-
-  if (tip >= 0) {
-    inverse(a.lymix + (size_t)tip * d.mp + (size_t)kz * nkx, -a.beta, 1);
-    const int s0 = room(1, 0), s1 = room(1, 1);
-    for (int x = tid; x < n; x += bd) {
-      const fx2 z = Z[x];
-      F[P.turn[x]] = fx2{solid(m0, x) ? shifted(z.y, s0) : 0, solid(m1, x) ? shifted(z.x, s1) : 0};
-    }
-    __syncthreads();
-  }
-  inverse(row, 1.0, 0);
-  int S0 = scale(0, 0), S1 = scale(0, 1);
-  {
-    const int s0 = room(0, 0), s1 = room(0, 1);
-    int d0 = 0, d1 = 0, l0 = 0, l1 = 0;  // from the field's and the Laplacian's scales to the coarser
-    if (tip >= 0) {
-      const int L0 = scale(1, 0), L1 = scale(1, 1), T0 = min(S0, L0), T1 = min(S1, L1);
-      d0 = min(S0 - T0, 63); d1 = min(S1 - T1, 63); l0 = min(L0 - T0, 63); l1 = min(L1 - T1, 63);
-      S0 = T0; S1 = T1;
-    }
-    for (int x = tid; x < n; x += bd) {
-      const fx2 z = Z[x];
-      const int px = P.turn[x];
-      const fx2 l = tip >= 0 ? F[px] : fx2{0, 0};
-      F[px] = fx2{solid(m0, x) ? l.x >> l0 : shifted(z.y, s0) >> d0, solid(m1, x) ? l.y >> l1 : shifted(z.x, s1) >> d1};
-    }
-  }
-  __syncthreads();
-  fx_fft(F, 1, P, nullptr);
-  const bool nan = max(red.e[0], red.e[1]) >= 0x7ff00000u;
-  const double norm = nan ? __longlong_as_double(0x7ff8000000000000ll) : 1.0 / n;
-  const FxOut out0(0, S0 - P.shift + 1), out1(0, S1 - P.shift + 1);  // the sums below double a spectrum
-  for (int k = tid; k < nkx; k += bd) {
-    const fx2 zk = F[P.pos_freq[k]], zc = F[P.pos_freq[k ? n - k : 0]];
-    if (on0) row[k] = double2{norm * out0(zk.x + zc.x), k ? norm * out0(zk.y - zc.y) : 0.0};
-    if (on1) row[nkx + k] = double2{norm * out1(zk.y + zc.y), k ? norm * out1(zc.x - zk.x) : 0.0};
-  }
-}
-
-// Threads of a CTA: FP32 128; FP64 about one per item of its line's radix-8 passes.
-template <typename R>
-__host__ __device__ __forceinline__ int xmask_threads(int ngx) {
-  return sizeof(R) == 4 ? 128 : min(128, (ngx / 8 + 31) / 32 * 32);
+  x_forward_packed<R>(1, F, hp, rows, d, ph, rtw);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 1 : 6) k_xmask(const __grid_constant__ MaskArgs<R> a,
-                                                                       const __grid_constant__ Dims d,
-                                                                       const __grid_constant__ MaskPlan<R> p) {
-  xmask_body(a, d, p, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(128) k_xmask(const __grid_constant__ MaskArgs<R> a, const __grid_constant__ Dims d,
+                                               const __grid_constant__ FftPlan ph, const double2* __restrict__ rtw) {
+  xmask_body<R>(a, d, ph, rtw, blockIdx.x, blockIdx.y);
 }
 
 template <typename R>
 void xmask_shape(const MaskArgs<R>& a, const Dims& d, dim3* grid, size_t* smem) {
   const int tot = a.nplanes[0] + a.nplanes[1] + a.nplanes[2];
-  *grid = tot == 0 ? dim3(0, 0, 0) : dim3(sizeof(R) == 4 ? d.ngz : (d.ngz + 1) / 2, tot);
+  *grid = tot == 0 ? dim3(0, 0, 0) : dim3(d.ngz, tot);
   const int hp = d.ngx / 2 + 1;
-  *smem = sizeof(R) == 4 ? sizeof(cpx_t<R>) * sx_elems<R>(2 * (size_t)hp) + sizeof(R) * 2 * (size_t)d.ngx
-                         : sizeof(fx2) * 2 * (size_t)d.ngx;
+  *smem = sizeof(cpx_t<R>) * sx_elems<R>(2 * (size_t)hp) + sizeof(R) * 2 * (size_t)d.ngx;
 }
 
 template <typename R>
-void launch_xmask(const MaskArgs<R>& a, const Dims& d, const MaskPlan<R>& p, cudaStream_t st) {
+void launch_xmask(const MaskArgs<R>& a, const Dims& d, const FftPlan& ph, const double2* rtw, cudaStream_t st) {
   dim3 grid;
   size_t sm;
   xmask_shape(a, d, &grid, &sm);
   if (grid.x == 0) return;
-  k_xmask<R><<<grid, xmask_threads<R>(d.ngx), sm, st>>>(a, d, p);
+  k_xmask<R><<<grid, 128, sm, st>>>(a, d, ph, rtw);
 }
 
 // ---------------------------------------------------------------------------
@@ -1379,17 +865,28 @@ void launch_xmask(const MaskArgs<R>& a, const Dims& d, const MaskPlan<R>& p, cud
 __device__ __forceinline__ double2 ld(const double2* p) { return __ldg(p); }
 __device__ __forceinline__ float2 ld(const float2* p) { return __ldg(p); }
 
-// The mixed form's nonlinear term from the product spectra: (-kx A.y - kz B.y) + c (D1.x - D0.x) and its imaginary
-// partner (d/dx, d/dz of the in-plane products, d/dy of the face products), combined in FP32 and widened.
+// product spectra q = 0..5 (uu, uw, ww, vv, uv, vw) of the assembly's precision
+template <typename P> __device__ __forceinline__ const P* prod(const AsmArgs& a, int q);
+template <> __device__ __forceinline__ const double2* prod<double2>(const AsmArgs& a, int q) { return a.p64[q]; }
+template <> __device__ __forceinline__ const float2* prod<float2>(const AsmArgs& a, int q) { return a.p32[q]; }
+
+// The nonlinear term from the product spectra: (-kx A.y - kz B.y) + c (D1.x - D0.x) and its imaginary
+// partner (d/dx, d/dz of the in-plane products, d/dy of the face products).  The mixed form's FP32
+// spectra are combined in FP32 and only the result is widened.
+__device__ __forceinline__ double2 nterm(double2 A, double2 B, double2 D1, double2 D0, double kx, double kz, double c) {
+  return double2{(-kx * A.y - kz * B.y) + c * (D1.x - D0.x), (kx * A.x + kz * B.x) + c * (D1.y - D0.y)};
+}
 __device__ __forceinline__ double2 nterm(float2 A, float2 B, float2 D1, float2 D0, float fx, float fz, float fc) {
   return double2{(double)((-fx * A.y - fz * B.y) + fc * (D1.x - D0.x)),
                  (double)((fx * A.x + fz * B.x) + fc * (D1.y - D0.y))};
 }
+// the wavenumbers and the y metric in the precision the product spectra are combined in
+template <typename P> __device__ __forceinline__ auto wnum(const double* d, const float* f, int i) {
+  if constexpr (sizeof(P) == sizeof(float2)) return __ldg(f + i);
+  else return d[i];
+}
 
-// 64 threads a CTA: with 256, three launches of the 96 x 96 x 130 grid take 0.162 ms instead of 0.144 in the mixed form, a
-// tenth more in FP64 too, and half as much again on 48 x 48 x 66; the largest grids 2 % less in FP64.
-constexpr int kAsmThreads = 64;
-
+template <typename P>
 __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, const Tables& t, int bx, int by) {
   const int col = bx * blockDim.x + threadIdx.x;
   if (col >= d.np) return;
@@ -1430,13 +927,13 @@ __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, c
       double rx = a.C1 * L_x + a.C2 * nold.x + (a.d * kf) * pc.y;
       double ry = a.C1 * L_y + a.C2 * nold.y + -(a.d * kf) * pc.x;
       if (f == 0 && col == 0) rx = rx + (-a.d * a.sc->mpgx);
-      const float2 A = ld(a.p32[f == 0 ? 0 : 1] + c0);
-      const float2 B = ld(a.p32[f == 0 ? 1 : 2] + c0);
-      const float2* D = a.p32[f == 0 ? 4 : 5];
+      const P A = ld(prod<P>(a, f == 0 ? 0 : 1) + c0);
+      const P B = ld(prod<P>(a, f == 0 ? 1 : 2) + c0);
+      const P* D = prod<P>(a, f == 0 ? 4 : 5);
       // a short column's product is zero on the middle band's planes (they hold only long modes)
-      const float2 D1 = (lng || !coarse_v(d, jj)) ? ld(D + f1) : float2{0, 0};
-      const float2 D0 = (lng || !coarse_v(d, jj - 1)) ? ld(D + f0) : float2{0, 0};
-      const double2 N = nterm(A, B, D1, D0, __ldg(t.kxf + i), __ldg(t.kzf + kk), __ldg(t.cuf + jj));
+      const P D1 = (lng || !coarse_v(d, jj)) ? ld(D + f1) : P{0, 0};
+      const P D0 = (lng || !coarse_v(d, jj - 1)) ? ld(D + f0) : P{0, 0};
+      const double2 N = nterm(A, B, D1, D0, wnum<P>(t.kx, t.kxf, i), wnum<P>(t.kz, t.kzf, kk), wnum<P>(t.cu, t.cuf, jj));
       const double nr = N.x, ni = N.y;
       (f == 0 ? a.n1 : a.n3)[c0] = double2{nr, ni};
       rx = rx - a.g * nr;
@@ -1465,9 +962,9 @@ __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, c
       const double2 nold = a.C2 != 0.0 ? a.n2[c0] : double2{0.0, 0.0};
       double rx = a.C1 * L_x + a.C2 * nold.x + C3 * (p1.x - p0.x);
       double ry = a.C1 * L_y + a.C2 * nold.y + C3 * (p1.y - p0.y);
-      const float2 A = ld(a.p32[4] + c0), B = ld(a.p32[5] + c0);
-      const float2 V1 = ld(a.p32[3] + c0 + np), V0 = ld(a.p32[3] + c0);
-      const double2 N = nterm(A, B, V1, V0, __ldg(t.kxf + i), __ldg(t.kzf + kk), __ldg(t.cvf + jj));
+      const P A = ld(prod<P>(a, 4) + c0), B = ld(prod<P>(a, 5) + c0);
+      const P V1 = ld(prod<P>(a, 3) + c0 + np), V0 = ld(prod<P>(a, 3) + c0);
+      const double2 N = nterm(A, B, V1, V0, wnum<P>(t.kx, t.kxf, i), wnum<P>(t.kz, t.kzf, kk), wnum<P>(t.cv, t.cvf, jj));
       const double nr = N.x, ni = N.y;
       a.n2[c0] = double2{nr, ni};
       rx = rx - a.g * nr;
@@ -1482,138 +979,19 @@ __device__ __forceinline__ void assemble_body(const AsmArgs& a, const Dims& d, c
   }
 }
 
-// FP64: several levels of a column a thread.  The kernel is bound by FP64 instructions (a warp's takes 64 clocks of its
-// quarter of the SM; the pipe is 89 % busy, memory a quarter), so what a level's or a column's points share is formed once:
-// the metric times dt C1 by one thread a CTA, the wavenumbers times dt d once a column.  What is left is 12 instructions a
-// real or imaginary part of u1 and u3 and 13 of u2, 77 a point against 87 with a product for each factor.  u0 is added last
-// and not within its factor 1 + dt C1 (k2 + a2): that takes six instructions less (14.8 ms), but its rounding doubles the
-// error of p.  Three launches, before and after: 576 x 576 x 450 18.0 -> 16.1 ms, 288 x 288 x 226 2.28 -> 2.06, 96 x 96 x
-// 130 0.179 -> 0.158, 48 x 48 x 66 0.061 -> 0.038.
-constexpr int kAsmLevels = 4;  // at most
-struct AsmLevel {
-  double um, u0, up, cu;      // dt C1 times the u grid's second derivative, d/dy at centres
-  double vm, v0, vp, cv, pv;  // the same at faces; pv = -dt d cv
-};
-__device__ __forceinline__ void assemble_levels(const AsmArgs& a, const Dims& d, const Tables& t, int levels, int bx,
-                                                int by) {
-  __shared__ AsmLevel level[kAsmLevels];
-  const int j0 = by * levels, j1 = min(j0 + levels, d.nyu);
-  for (int e = threadIdx.x; e < 9 * levels; e += blockDim.x) {
-    const int q = e / 9, i = e - 9 * q, jj = min(j0 + q, i < 4 ? d.nyu - 1 : d.nyv - 1);
-    const double c = i == 3 ? t.cu[jj] : (i >= 7 ? t.cv[jj] : (i < 3 ? t.d2u[3 * jj + i] : t.d2v[3 * jj + i - 4]));
-    const double f = i == 3 || i == 7 ? 1.0 : (i == 8 ? -a.dt * a.d : a.dt * a.C1);
-    reinterpret_cast<double*>(&level[q])[i] = f * c;
-  }
-  __syncthreads();
-  const int np = d.np, col = bx * blockDim.x + threadIdx.x;
-  if (col >= np) return;
-  const int i = col % d.nkx, kk = col / d.nkx;
-  const double kx = t.kx[i], kz = t.kz[kk];
-  const double dtC2 = a.dt * a.C2, dtg = a.dt * a.g, dtd = a.dt * a.d;
-  const double k2 = (a.dt * a.C1) * (t.k2x[i] + t.k2z[kk]), px = dtd * kx, pz = dtd * kz;
-  // 1/axz of LUsolU/LUsolV (tridLU_3D_IB.f90:489,93) for this substage: a multiply instead of a
-  // division, which costs ~10 FP64 instructions on a part with little FP64 throughput
-  const double iaxz = t.iaxz[(size_t)a.k * np + col];
-  const bool lng = is_long(d, i, kk);
-  // the first substage's zeta is 0 (start.f90:413-427): its old nonlinear term is not read, so a term left
-  // from earlier fields (even a non-finite one) does not enter
-  const bool old = a.C2 != 0.0;
-#pragma unroll 1
-  for (int jj = j0; jj < j1; ++jj) {
-    const AsmLevel& L = level[jj - j0];
-    const size_t c0 = (size_t)jj * np + col;
-    // u1 and u3 on centre jj
-    const int lu = lev_u(d, lng, jj);
-    if (lu != 1) {  // the column's end rows, or outside a short column
-      a.r1[c0] = double2{0.0, 0.0};
-      a.r3[c0] = double2{0.0, 0.0};
-      if (lu == 0 || (jj != 0 && jj != d.nyu - 1)) {
-        a.n1[c0] = double2{0.0, 0.0};
-        a.n3[c0] = double2{0.0, 0.0};
-      }
-    } else {
-      const double z = L.u0 + k2;
-      const double2 pc = ld(a.p + c0 - np);
-      // a short column's product is zero on the middle band's planes (they hold only long modes)
-      const bool in1 = lng || !coarse_v(d, jj), in0 = lng || !coarse_v(d, jj - 1);
-#pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        const double2* u = f == 0 ? a.u1 : a.u3;
-        double2* n = f == 0 ? a.n1 : a.n3;
-        const double2 um = ld(u + c0 - np), u0 = ld(u + c0), up = ld(u + c0 + np);
-        const double2 nold = old ? n[c0] : double2{0.0, 0.0};
-        const double2 A = ld(a.p64[f == 0 ? 0 : 1] + c0), B = ld(a.p64[f == 0 ? 1 : 2] + c0);
-        const double2* D = a.p64[f == 0 ? 4 : 5] + c0;
-        const double2 D1 = in1 ? ld(D) : double2{0.0, 0.0}, D0 = in0 ? ld(D - np) : double2{0.0, 0.0};
-        const double pk = f == 0 ? px : pz;
-        double rx = fma(L.um, um.x, fma(z, u0.x, L.up * up.x)), ry = fma(L.um, um.y, fma(z, u0.y, L.up * up.y));
-        rx = fma(pk, pc.y, fma(dtC2, nold.x, rx));
-        ry = fma(-pk, pc.x, fma(dtC2, nold.y, ry));
-        if (f == 0 && col == 0) rx = fma(-dtd, a.sc->mpgx, rx);
-        // d/dx, d/dz of the in-plane products, d/dy of the face product
-        const double nr = fma(L.cu, D1.x - D0.x, -fma(kx, A.y, kz * B.y));
-        const double ni = fma(L.cu, D1.y - D0.y, fma(kx, A.x, kz * B.x));
-        n[c0] = double2{nr, ni};
-        (f == 0 ? a.r1 : a.r3)[c0] = double2{(u0.x + fma(-dtg, nr, rx)) * iaxz, (u0.y + fma(-dtg, ni, ry)) * iaxz};
-        if (jj == a.tipu[0] || jj == a.tipu[1]) {
-          const double a1 = t.d2u[3 * jj], a2 = t.d2u[3 * jj + 1], a3 = t.d2u[3 * jj + 2];
-          a.lytip[(size_t)(2 * f + (jj == a.tipu[0] ? 0 : 1)) * np + col] =
-              double2{a1 * um.x + a2 * u0.x + a3 * up.x, a1 * um.y + a2 * u0.y + a3 * up.y};
-        }
-      }
-    }
-    // u2 on face jj
-    if (jj > d.nyv - 1) continue;
-    const int lv = lev_v(d, lng, jj);
-    if (lv != 1) {
-      a.r2[c0] = double2{0.0, 0.0};
-      if (lv == 0 || (jj != 0 && jj != d.nyv - 1)) a.n2[c0] = double2{0.0, 0.0};
-    } else {
-      const double z = L.v0 + k2;
-      const double2 um = ld(a.u2 + c0 - np), u0 = ld(a.u2 + c0), up = ld(a.u2 + c0 + np);
-      const double2 p0 = ld(a.p + c0 - np), p1 = ld(a.p + c0);
-      const double2 nold = old ? a.n2[c0] : double2{0.0, 0.0};
-      const double2 A = ld(a.p64[4] + c0), B = ld(a.p64[5] + c0), V1 = ld(a.p64[3] + c0 + np), V0 = ld(a.p64[3] + c0);
-      double rx = fma(L.vm, um.x, fma(z, u0.x, L.vp * up.x)), ry = fma(L.vm, um.y, fma(z, u0.y, L.vp * up.y));
-      rx = fma(L.pv, p1.x - p0.x, fma(dtC2, nold.x, rx));
-      ry = fma(L.pv, p1.y - p0.y, fma(dtC2, nold.y, ry));
-      const double nr = fma(L.cv, V1.x - V0.x, -fma(kx, A.y, kz * B.y));
-      const double ni = fma(L.cv, V1.y - V0.y, fma(kx, A.x, kz * B.x));
-      a.n2[c0] = double2{nr, ni};
-      a.r2[c0] = double2{(u0.x + fma(-dtg, nr, rx)) * iaxz, (u0.y + fma(-dtg, ni, ry)) * iaxz};
-      if (jj == a.tipv[0] || jj == a.tipv[1]) {
-        const double a1 = t.d2v[3 * jj], a2 = t.d2v[3 * jj + 1], a3 = t.d2v[3 * jj + 2];
-        a.lytip[(size_t)(4 + (jj == a.tipv[0] ? 0 : 1)) * np + col] =
-            double2{a1 * um.x + a2 * u0.x + a3 * up.x, a1 * um.y + a2 * u0.y + a3 * up.y};
-      }
-    }
-  }
-}
-
+// 64 threads a CTA.  Three launches, ms, with 256 / 64 threads: 48 x 48 x 66 0.063 / 0.043, 96 x 96 x 130 0.179 / 0.172
+// (mixed 0.159 / 0.142), 162 x 108 x 124 0.296 / 0.288, 288 x 288 x 226 2.28 / 2.28, 576 x 576 x 450 17.97 / 17.96 (mixed
+// 14.97 / 14.98).
+template <typename P>
 __global__ void __launch_bounds__(kAsmThreads) k_assemble(const __grid_constant__ AsmArgs a, const __grid_constant__ Dims d,
                                                           const __grid_constant__ Tables t) {
-  assemble_body(a, d, t, blockIdx.x, blockIdx.y);
-}
-__global__ void __launch_bounds__(kAsmThreads) k_assemble64(const __grid_constant__ AsmArgs a, const __grid_constant__ Dims d,
-                                                            const __grid_constant__ Tables t, int levels) {
-  assemble_levels(a, d, t, levels, blockIdx.x, blockIdx.y);
-}
-
-// Levels a CTA: more share what a column's points share, fewer leave more CTAs.  Three launches, ms, 1 / 2 / 4 levels:
-// 48 x 48 x 66 (34000 points) 0.039 / 0.045 / 0.068, 96 x 96 x 130 (266000) 0.162 / 0.158 / 0.172, 288 x 288 x 226 (4.2
-// million) 2.18 / 2.09 / 2.06, 576 x 576 x 450 17.1 / 16.4 / 16.1.
-void assemble_shape(const Dims& d, bool fp32_products, int* gx, int* gy, int* levels) {
-  const long long points = (long long)d.np * d.nyu;
-  *gx = (d.np + kAsmThreads - 1) / kAsmThreads;
-  *levels = fp32_products ? 1 : points < 100000 ? 1 : (points < 1000000 ? 2 : kAsmLevels);
-  *gy = (d.nyu + *levels - 1) / *levels;
+  assemble_body<P>(a, d, t, blockIdx.x, blockIdx.y);
 }
 
 void launch_assemble(const AsmArgs& a, const Dims& d, const Tables& t, cudaStream_t st) {
-  int gx, gy, levels;
-  assemble_shape(d, a.p32[0] != nullptr, &gx, &gy, &levels);
-  if (a.p32[0]) k_assemble<<<dim3(gx, gy), kAsmThreads, 0, st>>>(a, d, t);
-  else k_assemble64<<<dim3(gx, gy), kAsmThreads, 0, st>>>(a, d, t, levels);
+  const dim3 grid((d.np + kAsmThreads - 1) / kAsmThreads, d.nyu);
+  if (a.p32[0]) k_assemble<float2><<<grid, kAsmThreads, 0, st>>>(a, d, t);
+  else k_assemble<double2><<<grid, kAsmThreads, 0, st>>>(a, d, t);
 }
 
 // The column solves take two threads per column, one for the real parts and one for the imaginary ones (neighbouring
@@ -2536,50 +1914,43 @@ __device__ __forceinline__ int batch_member(const Batch<D>& b, int blk) {
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zinv_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 5) k_zinv_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
   const int m = batch_member(b, blockIdx.x);
   const ZDesc<R>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m], gxy = D.gx * D.gy;
-  zinv_body(D.jobs, D.d, D.p, D.tx, q % D.gx, (q % gxy) / D.gx, q / gxy);
+  zinv_body<R>(D.jobs, D.d, D.p, D.tx, q % D.gx, (q % gxy) / D.gx, q / gxy);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 4) k_zfwd_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 8 : 5) k_zfwd_batch(const __grid_constant__ Batch<ZDesc<R>> b) {
   const int m = batch_member(b, blockIdx.x);
   const ZDesc<R>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m], gxy = D.gx * D.gy;
-  zfwd_body(D.jobs, D.d, D.p, D.tx, D.scale, q % D.gx, (q % gxy) / D.gx, q / gxy);
-}
-
-__global__ void __launch_bounds__(256, 6) k_xprod_batch(const __grid_constant__ Batch<XDesc<float>> b) {
-  const int m = batch_member(b, blockIdx.x);
-  const XDesc<float>& D = b.desc[m];
-  const int q = blockIdx.x - b.start[m];
-  xprod_body(D.a, D.d, D.p, q % D.gx, q / D.gx);
-}
-template <bool TWO>
-__global__ void __launch_bounds__(kFxThreads, 3) k_xprod_fx_batch(const __grid_constant__ Batch<XDesc<double>> b) {
-  const int m = batch_member(b, blockIdx.x);
-  const XDesc<double>& D = b.desc[m];
-  const int q = blockIdx.x - b.start[m];
-  xprod_body<TWO>(D.a, D.d, D.p, q % D.gx, q / D.gx);
+  zfwd_body<R>(D.jobs, D.d, D.p, D.tx, D.scale, q % D.gx, (q % gxy) / D.gx, q / gxy);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 6) k_xmask_batch(const __grid_constant__ Batch<MDesc<R>> b) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 6 : 5) k_xprod_batch(const __grid_constant__ Batch<XDesc<R>> b) {
+  const int m = batch_member(b, blockIdx.x);
+  const XDesc<R>& D = b.desc[m];
+  const int q = blockIdx.x - b.start[m];
+  xprod_body<R>(D.a, D.d, D.ph, D.pf, D.rtw, q % D.gx, q / D.gx);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 9) k_xmask_batch(const __grid_constant__ Batch<MDesc<R>> b) {
   const int m = batch_member(b, blockIdx.x);
   const MDesc<R>& D = b.desc[m];
   const int q = blockIdx.x - b.start[m];
-  xmask_body(D.a, D.d, D.p, q % D.gx, q / D.gx);
+  xmask_body<R>(D.a, D.d, D.ph, D.rtw, q % D.gx, q / D.gx);
 }
 
-template <bool FP32>
+template <typename P>
 __global__ void __launch_bounds__(kAsmThreads, 768 / kAsmThreads) k_assemble_batch(const __grid_constant__ Batch<ADesc> b) {
   const int m = batch_member(b, blockIdx.x);
   const ADesc& D = b.desc[m];
   const int q = blockIdx.x - b.start[m];
-  if constexpr (FP32) assemble_body(D.a, D.d, D.t, q % D.gx, q / D.gx);
-  else assemble_levels(D.a, D.d, D.t, D.levels, q % D.gx, q / D.gx);
+  assemble_body<P>(D.a, D.d, D.t, q % D.gx, q / D.gx);
 }
 
 __global__ void __launch_bounds__(kTileThreads, 5) k_vsolve_batch(const __grid_constant__ Batch<VDesc> b) {
@@ -2611,21 +1982,16 @@ void launch_zfwd_batch(const Batch<ZDesc<R>>& b, size_t smem, cudaStream_t st) {
 }
 template <typename R>
 void launch_xprod_batch(const Batch<XDesc<R>>& b, size_t smem, cudaStream_t st) {
-  if (b.n <= 0 || b.start[b.n] <= 0) return;
-  // FP64: members of one shared-memory size are of one x length
-  if constexpr (sizeof(R) == 4) k_xprod_batch<<<b.start[b.n], 256, smem, st>>>(b);
-  else if (xprod_levels(b.desc[0].d.ngx) == 2) k_xprod_fx_batch<true><<<b.start[b.n], xprod_threads<R>(b.desc[0].d, 256), smem, st>>>(b);
-  else k_xprod_fx_batch<false><<<b.start[b.n], xprod_threads<R>(b.desc[0].d, 256), smem, st>>>(b);
+  if (b.n > 0 && b.start[b.n] > 0) k_xprod_batch<R><<<b.start[b.n], 256, smem, st>>>(b);
 }
 template <typename R>
 void launch_xmask_batch(const Batch<MDesc<R>>& b, size_t smem, cudaStream_t st) {
-  // members of one shared-memory size are of one x length
-  if (b.n > 0 && b.start[b.n] > 0) k_xmask_batch<R><<<b.start[b.n], xmask_threads<R>(b.desc[0].d.ngx), smem, st>>>(b);
+  if (b.n > 0 && b.start[b.n] > 0) k_xmask_batch<R><<<b.start[b.n], 128, smem, st>>>(b);
 }
 void launch_assemble_batch(const Batch<ADesc>& b, bool fp32_products, cudaStream_t st) {
   if (b.n <= 0 || b.start[b.n] <= 0) return;
-  if (fp32_products) k_assemble_batch<true><<<b.start[b.n], kAsmThreads, 0, st>>>(b);
-  else k_assemble_batch<false><<<b.start[b.n], kAsmThreads, 0, st>>>(b);
+  if (fp32_products) k_assemble_batch<float2><<<b.start[b.n], kAsmThreads, 0, st>>>(b);
+  else k_assemble_batch<double2><<<b.start[b.n], kAsmThreads, 0, st>>>(b);
 }
 void launch_vsolve_batch(const Batch<VDesc>& b, size_t smem, cudaStream_t st) {
   if (b.n > 0 && b.start[b.n] > 0) k_vsolve_batch<<<b.start[b.n], smem ? kTileThreads : kColThreads, smem, st>>>(b);
@@ -2710,14 +2076,14 @@ cudaError_t configure_kernels() {
   int optin = 0;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  const cudaError_t r[25] = {allow_smem(k_vsolve, optin), allow_smem(k_psolve_tile, optin), allow_smem(k_vsolve_batch, optin),
+  const cudaError_t r[23] = {allow_smem(k_vsolve, optin), allow_smem(k_psolve_tile, optin), allow_smem(k_vsolve_batch, optin),
                              allow_smem(k_psolve_batch<true>, optin), allow_smem(k_xcond, optin), allow_smem(k_zinv<double>, optin), allow_smem(k_zinv<float>, optin),
                              allow_smem(k_zfwd<double>, optin), allow_smem(k_zfwd<float>, optin),
-                             allow_smem(k_xprod_fx<true>, optin), allow_smem(k_xprod_fx<false>, optin), allow_smem(k_xprod_fx96, optin), allow_smem(k_xprod, optin), allow_smem(k_xprod2, optin),
+                             allow_smem(k_xprod<double>, optin), allow_smem(k_xprod<float>, optin), allow_smem(k_xprod2, optin), allow_smem(k_zinv_fx, optin),
                              allow_smem(k_xmask<double>, optin), allow_smem(k_xmask<float>, optin),
                              allow_smem(k_zinv_batch<double>, optin), allow_smem(k_zinv_batch<float>, optin),
                              allow_smem(k_zfwd_batch<double>, optin), allow_smem(k_zfwd_batch<float>, optin),
-                             allow_smem(k_xprod_fx_batch<true>, optin), allow_smem(k_xprod_fx_batch<false>, optin), allow_smem(k_xprod_batch, optin),
+                             allow_smem(k_xprod_batch<double>, optin), allow_smem(k_xprod_batch<float>, optin),
                              allow_smem(k_xmask_batch<double>, optin), allow_smem(k_xmask_batch<float>, optin)};
   for (cudaError_t x : r)
     if (x != cudaSuccess) return x;
@@ -2725,19 +2091,17 @@ cudaError_t configure_kernels() {
   return cudaSuccess;
 }
 
-template void launch_zinv<double>(const ZJobs<double>&, const Dims&, const ZPlan<double>&, int, cudaStream_t, int);
-template void launch_zinv<float>(const ZJobs<float>&, const Dims&, const ZPlan<float>&, int, cudaStream_t, int);
-template void launch_zfwd<double>(const ZJobs<double>&, const Dims&, const ZPlan<double>&, int, double, cudaStream_t, int);
-template void launch_zfwd<float>(const ZJobs<float>&, const Dims&, const ZPlan<float>&, int, double, cudaStream_t, int);
-template void launch_xprod<double>(const ProdArgs<double>&, const Dims&, const XPlan<double>&, cudaStream_t);
-template void launch_xprod<float>(const ProdArgs<float>&, const Dims&, const XPlan<float>&, cudaStream_t);
-template void launch_xmask<double>(const MaskArgs<double>&, const Dims&, const MaskPlan<double>&, cudaStream_t);
-template void launch_xmask<float>(const MaskArgs<float>&, const Dims&, const MaskPlan<float>&, cudaStream_t);
+template void launch_zinv<double>(const ZJobs<double>&, const Dims&, const FftPlan&, int, cudaStream_t, int);
+template void launch_zinv<float>(const ZJobs<float>&, const Dims&, const FftPlan&, int, cudaStream_t, int);
+template void launch_zfwd<double>(const ZJobs<double>&, const Dims&, const FftPlan&, int, double, cudaStream_t, int);
+template void launch_zfwd<float>(const ZJobs<float>&, const Dims&, const FftPlan&, int, double, cudaStream_t, int);
+template void launch_xprod<double>(const ProdArgs<double>&, const Dims&, const FftPlan&, const FftPlan&, const double2*,
+                                   cudaStream_t);
+template void launch_xprod<float>(const ProdArgs<float>&, const Dims&, const FftPlan&, const FftPlan&, const double2*,
+                                  cudaStream_t);
+template void launch_xmask<double>(const MaskArgs<double>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
+template void launch_xmask<float>(const MaskArgs<float>&, const Dims&, const FftPlan&, const double2*, cudaStream_t);
 template void zpass_shape<double>(const ZJobs<double>&, const Dims&, int, dim3*, size_t*);
-template int zpass_tile<double>(int);
-template int zpass_tile<float>(int);
-template int xprod_ctas_per_sm<double>(const Dims&, int, int);
-template int xprod_ctas_per_sm<float>(const Dims&, int, int);
 template void zpass_shape<float>(const ZJobs<float>&, const Dims&, int, dim3*, size_t*);
 template void xprod_shape<double>(const ProdArgs<double>&, const Dims&, dim3*, size_t*);
 template void xprod_shape<float>(const ProdArgs<float>&, const Dims&, dim3*, size_t*);

@@ -1281,17 +1281,21 @@ __device__ __forceinline__ double column_div(const ColumnPart& c, double ou, dou
   return fma(cu, dv, fma(c.kx, ou, c.kz * ow));
 }
 // One level of the forward sweep, (dtirk div - b1 x) b2.  Which of the two products is fused into the difference is part
-// of the results: every fourth level from the lower wall and all of a short column's upper band round the right-hand side
-// on its own (`alone`), the others round b1 x.  That is what the compiler made of the sweep when it ran in batches of
-// four, and established runs of the mixed form depend on it: its FP32 transforms turn a last bit of the FP64 state into
+// of the results: `alone` rounds the right-hand side on its own, otherwise b1 x is rounded.  Alone are every fourth level
+// of a segment, some of the levels beyond its last whole four (rest_alone) and all of a short column's upper band.  That
+// is what the compiler made of the sweep when it ran in batches of four, and established runs depend on it: the plane
+// mean of v holds nothing but such roundings, and the mixed form's FP32 transforms turn a last bit of the FP64 state into
 // 1e-8.
 __device__ __forceinline__ double column_up(bool alone, double dtirk, double div, double b1, double b2, double x) {
   if (alone) return __dmul_rn(fma(-b1, x, __dmul_rn(dtirk, div)), b2);
   return __dmul_rn(fma(dtirk, div, -__dmul_rn(b1, x)), b2);
 }
 
+// `alone` for level i of the `rest` levels beyond a segment's last whole four (a long column's or a lower band's).
+__device__ __forceinline__ bool rest_alone(int i, int rest, bool lng) { return i == 0 || (rest == 3 && i == (lng ? 1 : 2)); }
+
 __device__ __forceinline__ void psolve_segment(const ColumnPart& c, const Tables& t, const double* F, double dtirk, int lo,
-                                               int hi, bool pin00, bool alone, bool& bad) {
+                                               int hi, bool pin00, bool lng, bool alone, bool& bad) {
   constexpr int NB = kColBatch;
   static_assert(NB == 2, "the forward sweep takes two batches per four levels");
   const size_t np = c.np, np2 = c.np2;
@@ -1337,7 +1341,7 @@ __device__ __forceinline__ void psolve_segment(const ColumnPart& c, const Tables
       get(jp, A, W, V, B);
       const double r = div(jp, A[0], W[0], V[0]);
       const double b1 = __ldg(t.dg1 + jp);
-      put(jp, jp == lo ? __dmul_rn(__dmul_rn(dtirk, r), B[0]) : column_up(alone || jp == end, dtirk, r, b1, B[0], x));
+      put(jp, jp == lo ? __dmul_rn(__dmul_rn(dtirk, r), B[0]) : column_up(alone || rest_alone(jp - end, hi + 1 - end, lng), dtirk, r, b1, B[0], x));
     }
   }
   const unsigned pair = 3u << (threadIdx.x & 30);  // the lanes of the column's two parts
@@ -1437,12 +1441,12 @@ __device__ __forceinline__ void psolve_tile(const ColumnPart& c, const Dims& d, 
         up(j + 2, false);
         up(j + 3, false);
       }
-      for (; j < n; ++j) up(j, (j & 3) == 0);
+      for (const int end = j; j < n; ++j) up(j, rest_alone(j - end, n - end, true));
     } else {
       // b = 0 on the levels between a short column's bands leaves y = 0, as the upper segment's first level wants it
-      for (int j = 0; j < n; ++j) {
-        up(j, (!lng && j >= d.Nu2) || (j & 3) == 0);
-      }
+      const int own = lng ? n : d.Nu1, end = own / 4 * 4;  // levels of the (lower) segment, and of its whole fours
+      for (int j = 0; j < n; ++j)
+        up(j, (!lng && j >= d.Nu2) || (j < end ? (j & 3) == 0 : rest_alone(j - end, own - end, lng)));
     }
 #pragma unroll 8
     for (int j = n - 2; j >= 0; --j) {
@@ -1531,10 +1535,10 @@ __device__ __forceinline__ void psolve_body(double2* u1, double2* u2, double2* u
     if (col >= d.np) return;
     const ColumnPart c = column_part(u1, u2, u3, p, psi, d, t, dtrk, part);
     if (is_long(d, col % d.nkx, col / d.nkx)) {
-      psolve_segment(c, t, F, dtirk, 0, d.nyp - 1, col == 0, false, bad);
+      psolve_segment(c, t, F, dtirk, 0, d.nyp - 1, col == 0, true, false, bad);
     } else {
-      psolve_segment(c, t, F, dtirk, 0, d.Nu1 - 1, false, false, bad);
-      psolve_segment(c, t, F, dtirk, d.Nu2, d.nyp - 1, false, true, bad);
+      psolve_segment(c, t, F, dtirk, 0, d.Nu1 - 1, false, false, false, bad);
+      psolve_segment(c, t, F, dtirk, d.Nu2, d.nyp - 1, false, false, true, bad);
       // v on the end rows of the short column's bands (v_corr, littleharsh.f90:904-905)
       c.v[(size_t)(d.Nv1 + 1) * c.np2] = 0.0;
       c.v[(size_t)d.Nv2 * c.np2] = 0.0;

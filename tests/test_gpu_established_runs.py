@@ -11,7 +11,10 @@ from tests.helpers import SMALL
 pytestmark = pytest.mark.gpu
 
 RECORDED = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "established_fp64.json")
-RUNS = {"canopy": SMALL,
+# canopy: 40 pressure levels; bands: lower bands of 15; three43: 43, three beyond the last whole four; three43_columns: the
+# same with too many columns for tiles; ragged: 48
+RUNS = {"canopy": SMALL, "bands": dict(SMALL, ngalx2=18, ngalz2=18), "three43": dict(SMALL, ny=36),
+        "three43_columns": dict(SMALL, ny=36, ngalx=288, ngalz=96, ntilex=12, ntilez=6),
         "ragged": dict(SMALL, ngalx=54, ngalz=36, ny=41, ntilex=9, ntilez=6, flag_ctpress=1)}
 
 

@@ -1013,7 +1013,7 @@ constexpr int kTileBatch = 8;    // levels whose loads a warp of a tile has in f
 // once (two CTAs an SM in the pressure solve, five of the three components' CTAs in the velocity solve).  Beyond that
 // the tiles queue, and a thread per part has parallelism enough.  Three launches, ms, tiles against threads:
 // pressure 48 x 48 x 66 (34 tiles) 0.08 / 0.16, 96 x 96 x 130 (132) 0.15 / 0.32, 144 x 144 x 154 (294) 0.24 / 0.37,
-// 192 x 192 x 226 (520) 0.65 / 0.60; velocity 0.05 / 0.07, 0.08 / 0.13, 0.18 / 0.17, 0.45 / 0.32.
+// 192 x 192 x 226 (520) 0.65 / 0.60; velocity 0.05 / 0.07, 0.09 / 0.13, 0.18 / 0.17, 0.45 / 0.32.
 __host__ __device__ __forceinline__ bool column_fits(const Dims& d) { return d.nyu <= 400; }  // 205 KB
 __host__ __device__ __forceinline__ bool psolve_tiled(const Dims& d) { return column_fits(d) && d.np <= 16 * 304; }
 __host__ __device__ __forceinline__ bool vsolve_tiled(const Dims& d) { return column_fits(d) && 3 * d.np <= 16 * 760; }
@@ -1066,7 +1066,7 @@ __device__ __forceinline__ void thomas_column(double* __restrict__ R, double* __
 
 // The Thomas sweeps of a tile of columns.  A level's coefficients are those of the column's segment; zeros on the levels
 // between a short column's wall bands and below a segment's first level let the segments fall apart by themselves.
-__device__ __forceinline__ void vsolve_tile(const double* __restrict__ R, double* __restrict__ U, const Dims& d, const Tables& t,
+__device__ __forceinline__ void vsolve_tile(double* __restrict__ R, double* __restrict__ U, const Dims& d, const Tables& t,
                                             int k, int comp, int bx) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ny = comp == 1 ? d.nyv : d.nyu, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -1104,13 +1104,23 @@ __device__ __forceinline__ void vsolve_tile(const double* __restrict__ R, double
   }
   __syncthreads();
   if (warp == 0 && in) {
-    const double *a1 = lng ? M : M + 3 * ny, *a2 = a1 + ny, *a3 = a2 + ny;
+    const double *a1 = lng ? M : M + 3 * ny, *a2 = a1 + ny;
     double *c = X + lane, x = 0.0;
 #pragma unroll 8
     for (int j = 0; j < ny; ++j) {
       x = (c[j * kTileParts] - a1[j] * x) * a2[j];
       c[j * kTileParts] = x;
     }
+  }
+  __syncthreads();
+  if (in) {  // the right-hand sides are left as the forward sweep makes them, whichever form solves
+#pragma unroll 4
+    for (int j = warp; j < ny; j += warps) R[(size_t)j * np2 + part] = X[j * kTileParts + lane];
+  }
+  __syncthreads();
+  if (warp == 0 && in) {
+    const double* a3 = (lng ? M : M + 3 * ny) + 2 * ny;
+    double *c = X + lane, x = c[(ny - 1) * kTileParts];
 #pragma unroll 8
     for (int j = ny - 2; j >= 0; --j) {
       x = c[j * kTileParts] - a3[j] * x;

@@ -228,13 +228,14 @@ int build_fx(lh_handle* h, FxPlan* P, int n) {
 
 // The product pass's default launch shape.
 //
-// Mixed form: two z rows per CTA where Ngalz is even, with 128 threads while a stage of its three transforms has at most
-// 256 butterflies (3/4 Ngalx; with 256 threads most would idle), else 256.  Against one row and 256 threads, ms a step:
-// 96 x 96 x 130 0.42 -> 0.21, 288 x 288 x 226 3.08 -> 1.91, 576 x 576 x 450 17.4 -> 15.2 (128 threads there 15.9).
-// Levels per CTA: the chunk with the least estimated time, (CTAs / CTAs resident at once, at least one wave) x (levels +
-// 1.3 for the previous level's transforms).  On small grids short chunks fill the chip (48 x 48 x 66 with chunks of 2 / 4
-// levels 0.07 / 0.10 ms a step, 96 x 96 x 130 with 2 / 4 / 8 0.20 / 0.22 / 0.23); on large ones long chunks save the
-// repeated level (576 x 576 x 450 with 8 / 16 / 32: 15.2 / 15.1 / 15.2).
+// Mixed form: two z rows per CTA where Ngalz is even and their shared memory (99 bytes a point of x) fits, which it does
+// to Ngalx = 2304, with 128 threads while a stage of its three transforms has at most 256 butterflies (3/4 Ngalx; with 256
+// threads most would idle), else 256.  Against one row and 256 threads, ms a step: 96 x 96 x 130 0.42 -> 0.21, 288 x 288 x
+// 226 3.08 -> 1.91, 576 x 576 x 450 17.4 -> 15.2 (128 threads there 15.9).  Levels per CTA: the chunk with the least
+// estimated time, (CTAs / CTAs resident at once, at least one wave) x (levels + 1.3 for the previous level's transforms).
+// On small grids short chunks fill the chip (48 x 48 x 66 with chunks of 2 / 4 levels 0.07 / 0.10 ms a step, 96 x 96 x 130
+// with 2 / 4 / 8 0.20 / 0.22 / 0.23); on large ones long chunks save the repeated level (576 x 576 x 450 with 8 / 16 / 32:
+// 15.2 / 15.1 / 15.2).
 //
 // FP64 form: 128 threads (256 measured 2 to 20 % slower at every length).  The CTAs of an SM share its FP64 pipe, and four
 // of them saturate it: a chunk's estimated time is (an SM's CTAs, at least 4, and one for the uneven end) x (levels + 1/3,
@@ -257,11 +258,12 @@ void default_xprod_shape(lh_handle* h) {
     }
     return;
   }
-  if (d.ngz % 2 == 0) {
+  const int threads2 = 3 * d.ngx / 4 <= 256 ? 128 : 256;
+  if (d.ngz % 2 == 0 && xprod_ctas_per_sm(d, 2, threads2) > 0) {
     h->xrows = 2;
-    h->xthreads = 3 * d.ngx / 4 <= 256 ? 128 : 256;
+    h->xthreads = threads2;
   }
-  const double resident = (double)sms * xprod_ctas_per_sm(d, h->xrows, h->xthreads);
+  const double resident = (double)sms * std::max(1, xprod_ctas_per_sm(d, h->xrows, h->xthreads));
   for (int c : {2, 4, 8, 16, 32}) {
     const double ctas = (double)(d.ngz / h->xrows) * ((d.nyu - 2 + c - 1) / c);
     const double t = std::max(1.0, ctas / resident) * (c + 1.3);
@@ -1717,7 +1719,7 @@ int lh_autotune(lh_handle* h, int32_t* tx_out, int32_t* chunk_out) {
   // together, since the best block size depends on the rows per CTA
   {
     const int xt0 = h->xthreads, xr0 = h->xrows;
-    const int maxrows = (h->precision == LH_PREC_MIXED && !h->xsplit) ? 2 : 1;
+    const int maxrows = (h->precision == LH_PREC_MIXED && !h->xsplit && xprod_ctas_per_sm(h->d, 2, 256) > 0) ? 2 : 1;
     float bestx = 1e30f;
     int bt = xt0, br = 1;
     for (int r = 1; r <= maxrows; ++r) {

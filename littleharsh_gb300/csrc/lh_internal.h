@@ -333,7 +333,7 @@ void launch_psolve_batch(const Batch<PDesc>& b, size_t smem, cudaStream_t st);
 template <typename R>
 void zpass_shape(const ZJobs<R>& jobs, const Dims& d, int tx, dim3* grid, size_t* smem);
 // CTAs of the mixed form's product pass, of `rows` z rows and `threads` threads, that an SM holds at once (after
-// configure_kernels).
+// configure_kernels); 0 if their shared memory does not fit.
 int xprod_ctas_per_sm(const Dims& d, int rows, int threads);
 template <typename R>
 void xprod_shape(const ProdArgs<R>& a, const Dims& d, dim3* grid, size_t* smem);

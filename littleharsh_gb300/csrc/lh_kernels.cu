@@ -767,9 +767,11 @@ int xprod_ctas_per_sm(const Dims& d, int rows, int threads) {
   size_t smem;
   xprod_shape(a, d, &grid, &smem);
   int n = 0;
-  if (rows == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_xprod2, threads, smem);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_xprod<float>, threads, smem);
-  return std::max(1, n);
+  const cudaError_t e = rows == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_xprod2, threads, smem)
+                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_xprod<float>, threads, smem);
+  if (e == cudaSuccess) return n;
+  cudaGetLastError();
+  return 0;
 }
 
 template <typename R>

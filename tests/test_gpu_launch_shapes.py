@@ -1,0 +1,43 @@
+"""Launch shapes at the limits of shared memory and of the rules that choose them."""
+import numpy as np
+import pytest
+
+from tests.helpers import SMOOTH
+
+pytestmark = pytest.mark.gpu
+
+
+def _stepped(cfg, precision, tune=False):
+    import littleharsh_gb300 as lh
+    s = lh.Solver(lh.Config(**cfg), precision=precision)
+    rng = np.random.default_rng(5)
+    f = [np.zeros_like(x) for x in s.get_fields()]
+    for x in f[:3]:
+        x[1:-1, 1:3, 1:9] = 0.01 * rng.standard_normal((x.shape[0] - 2, 2, 8))
+    f[0][:, 0, 0] = 1.0
+    s.set_fields(*f)
+    s.set_time(0.0, 1.0, 0.0)
+    s.project()
+    s.set_time(0.0, 1e-4, 0.0)
+    if tune:
+        s.autotune()
+    s.step(1)
+    return s.launch_shapes(), s.get_fields()
+
+
+@pytest.mark.parametrize("n,rows", [(2304, 2), (2592, 1), (4374, 1)])
+def test_mixed_product_pass_takes_two_rows_where_they_fit(monkeypatch, n, rows):
+    """Two z rows per CTA want about 99 bytes of shared memory a point of x: they fit at 2304, not at 2592, and the one-row
+    kernel serves on; the same bits either way, tuned or not."""
+    import littleharsh_gb300 as lh
+    cfg = dict(SMOOTH, ngalx=n, ngalz=6, ny=13)
+    shapes, f = _stepped(cfg, lh.PREC_MIXED)
+    assert shapes["xrows"] == rows
+    assert all(np.isfinite(x).all() for x in f) and np.abs(f[0]).max() > 0.5
+    tuned, g = _stepped(cfg, lh.PREC_MIXED, tune=True)
+    assert tuned["xrows"] <= rows
+    monkeypatch.setenv("LH_XROWS", "1")
+    _, one = _stepped(cfg, lh.PREC_MIXED)
+    for a, b, c in zip(f, g, one):
+        np.testing.assert_array_equal(a, c)
+        np.testing.assert_array_equal(b, c)

@@ -237,12 +237,13 @@ int build_fx(lh_handle* h, FxPlan* P, int n) {
 // with 2 / 4 / 8 0.20 / 0.22 / 0.23); on large ones long chunks save the repeated level (576 x 576 x 450 with 8 / 16 / 32:
 // 15.2 / 15.1 / 15.2).
 //
-// FP64 form: 128 threads (256 measured 2 to 20 % slower at every length).  The CTAs of an SM share its FP64 pipe, and four
-// of them saturate it: a chunk's estimated time is (an SM's CTAs, at least 4, and one for the uneven end) x (levels + 1/3,
-// the previous level's share); within 2 % the longest chunk is taken.  ms a step at 48 x 48 x 66 with 2 / 3 / 4 / 8 / 16
-// levels 0.265 / 0.228 / 0.254 / 0.364 / 0.616; 96 x 96 x 130 with 2 / 4 / 6 / 8 / 16 1.30 / 1.22 / 1.20 / 1.30 / 1.38;
-// 162 x 108 x 124 with 4 / 6 / 8 / 16 2.37 / 2.38 / 2.42 / 2.58; 288 x 288 x 226 with 4 / 8 / 16 / 32 17.6 / 17.1 / 17.0 /
-// 17.7; 576 x 576 x 450 with 8 / 16 / 32 139.4 / 137.6 / 138.0.
+// FP64 form: 128 threads (with 256 the chunks taken here measure 2 to 50 % slower).  The CTAs of an SM share its FP64
+// pipe, and four of them saturate it: a chunk's estimated time is (an SM's CTAs, at least 4, and one for the uneven end) x
+// (levels + 1/3, the previous level's share); within 2 % the longest chunk is taken.  ms a step at 48 x 48 x 66 with 4 / 8
+// / 16 levels 0.25 / 0.36 / 0.62; 96 x 96 x 130 1.22 / 1.30 / 1.38; 162 x 108 x 124 2.37 / 2.42 / 2.58; 288 x 288 x 226
+// with 4 / 8 / 16 / 32 17.6 / 17.1 / 17.0 / 17.7; 576 x 576 x 450 with 8 / 16 / 32 139.4 / 137.6 / 138.0.
+//
+// lh_autotune times every chunk that these rules may take.
 void default_xprod_shape(lh_handle* h) {
   const Dims& d = h->d;
   const int nlev = d.nyu - 1;
@@ -251,7 +252,7 @@ void default_xprod_shape(lh_handle* h) {
   double least = 1e300;
   if (h->precision != LH_PREC_MIXED) {
     h->xthreads = 128;
-    for (int c : {2, 3, 4, 6, 8, 12, 16, 32}) {
+    for (int c : {4, 8, 16, 32}) {
       const long long ctas = (long long)d.ngz * ((nlev + c - 1) / c);
       const double t = ((double)std::max(4ll, (ctas + sms - 1) / sms) + 1.0) * (c + 1.0 / 3.0);
       if (t < 1.02 * least) { least = std::min(least, t); h->chunk = c; }
@@ -1692,7 +1693,8 @@ int lh_autotune(lh_handle* h, int32_t* tx_out, int32_t* chunk_out) {
     if (h->zthreads != zt0 && h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; ++h->graph_gen; }
   }
   best = 1e30f;
-  for (int ch : {4, 8, 16, 32, 64}) {
+  for (int ch : {2, 4, 8, 16, 32, 64}) {
+    if (ch == 2 && h->precision != LH_PREC_MIXED) continue;
     h->chunk = ch;
     const float ms = h->precision == LH_PREC_MIXED ? time_parts<float>(h, false, true, e0, e1)
                                                    : time_parts<double>(h, false, true, e0, e1);

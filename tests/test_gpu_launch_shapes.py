@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from tests.helpers import SMOOTH
+from tests.helpers import C1, SMOOTH
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +41,18 @@ def test_mixed_product_pass_takes_two_rows_where_they_fit(monkeypatch, n, rows):
     for a, b, c in zip(f, g, one):
         np.testing.assert_array_equal(a, c)
         np.testing.assert_array_equal(b, c)
+
+
+@pytest.mark.parametrize("mixed", [False, True], ids=["fp64", "mixed"])
+def test_tuning_tries_what_the_rule_takes(mixed):
+    """The default chunk of levels is one that the tuner times.  Half of configuration 1 in the mixed form takes two levels,
+    40 % faster than four, which the tuner has to find as well."""
+    import littleharsh_gb300 as lh
+    prec = lh.PREC_MIXED if mixed else lh.PREC_FP64
+    cfg = dict(C1, ngalx=48, ngalz=48, ny=49, dsty=8, dstx=1, dstz=2)
+    default, f = _stepped(cfg, prec)
+    assert default["chunk"] == (2 if mixed else 4)
+    tuned, g = _stepped(cfg, prec, tune=True)
+    assert tuned["chunk"] in ((2,) if mixed else (4, 8, 16, 32, 64))
+    for a, b in zip(f, g):
+        np.testing.assert_array_equal(a, b)

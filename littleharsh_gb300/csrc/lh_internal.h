@@ -216,6 +216,7 @@ int vsolve_ctas(const Dims& d);
 int psolve_ctas(const Dims& d);
 size_t vsolve_smem(const Dims& d);
 size_t psolve_smem(const Dims& d);
+int psolve_form(const Dims& d);  // which of its kernels solves a grid
 void launch_divergence(const double2* u1, const double2* u2, const double2* u3, double2* div, const Dims& d,
                        const Tables& t, cudaStream_t st);
 void launch_absmax(const double2* x, size_t n, DevScalars* sc, cudaStream_t st);
@@ -341,6 +342,7 @@ template <typename R>
 void xmask_shape(const MaskArgs<R>& a, const Dims& d, dim3* grid, size_t* smem);
 
 cudaError_t configure_kernels();
+cudaError_t configure_psolve();
 // Measured FP64 FMA throughput of the current device in TFLOP/s (FMA = 2 flops), best of three timed
 // launches of a probe kernel; -1 on a CUDA error.  nsm_out (may be NULL) receives the SM count.
 double fp64_probe_tflops(int* nsm_out);

@@ -24,6 +24,7 @@
 //   psolve divergence, pressure LU per column, p += psi, v_corr
 //          (littleharsh.f90:557-612,826-937; tridLU_3D_IB.f90:362-396)
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 
 #include "lh_internal.h"
@@ -1025,7 +1026,14 @@ static int column_ctas(const Dims& d, bool tiled) {
 int vsolve_ctas(const Dims& d) { return column_ctas(d, vsolve_tiled(d)); }
 int psolve_ctas(const Dims& d) { return column_ctas(d, psolve_tiled(d)); }
 size_t vsolve_smem(const Dims& d) { return vsolve_tiled(d) ? sizeof(double) * (size_t)d.nyu * (kTileParts + 6) : 0; }
-size_t psolve_smem(const Dims& d) { return sizeof(double) * (psolve_tiled(d) ? (size_t)d.nyp * (2 * kTileParts + 1) : (size_t)d.nyv); }
+// Forms of the pressure solve: tiles; columns with the factors of the faces in shared memory, while they fit into the 48 KB
+// that every kernel may have; columns that form the factors at each level (5.65 -> 6.05 ms a step of 576 x 576 x 450).
+enum : int { kPTiles, kPColumns, kPLongColumns };
+int psolve_form(const Dims& d) { return psolve_tiled(d) ? kPTiles : (d.nyv <= 6144 ? kPColumns : kPLongColumns); }
+size_t psolve_smem(const Dims& d) {
+  const int form = psolve_form(d);
+  return form == kPTiles ? sizeof(double) * (size_t)d.nyp * (2 * kTileParts + 1) : (form == kPColumns ? sizeof(double) * (size_t)d.nyv : 0);
+}
 
 // Thomas sweeps of one column's real or imaginary part over levels lo..hi with an LU indexed by level
 // (LUsolU/LUsolV, tridLU_3D_IB.f90:106-116,179-189): R, U at the part's value of level 0, levels np2 apart.
@@ -1306,8 +1314,10 @@ __device__ __forceinline__ double column_up(bool alone, double dtirk, double div
 // `alone` for level i of the `rest` levels beyond a segment's last whole four (a long column's or a lower band's).
 __device__ __forceinline__ bool rest_alone(int i, int rest, bool lng) { return i == 0 || (rest == 3 && i == (lng ? 1 : 2)); }
 
-__device__ __forceinline__ void psolve_segment(const ColumnPart& c, const Tables& t, const double* F, double dtirk, int lo,
-                                               int hi, bool pin00, bool lng, bool alone, bool& bad) {
+// FACES: F holds dtrk cv per face.
+template <bool FACES>
+__device__ __forceinline__ void psolve_segment(const ColumnPart& c, const Tables& t, const double* F, double dtirk, double dtrk,
+                                               int lo, int hi, bool pin00, bool lng, bool alone, bool& bad) {
   constexpr int NB = kColBatch;
   static_assert(NB == 2, "the forward sweep takes two batches per four levels");
   const size_t np = c.np, np2 = c.np2;
@@ -1386,7 +1396,10 @@ __device__ __forceinline__ void psolve_segment(const ColumnPart& c, const Tables
       c.p[(size_t)j * np2] = pn;
       c.u[(size_t)(j + 1) * np2] = fma(-c.kxd, other, A[q]);
       c.w[(size_t)(j + 1) * np2] = fma(-c.kzd, other, W[q]);
-      if (j < hi) c.v[(size_t)(j + 1) * np2] = fma(-F[j + 1], xn - xc, V[q]);
+      if (j < hi) {
+        const double f = FACES ? F[j + 1] : __dmul_rn(dtrk, __ldg(t.cv + j + 1));
+        c.v[(size_t)(j + 1) * np2] = fma(-f, xn - xc, V[q]);
+      }
       xn = xc;
     }
 #pragma unroll
@@ -1527,30 +1540,33 @@ __device__ __forceinline__ ColumnPart column_part(double2* u1, double2* u2, doub
   return c;
 }
 
-template <bool TILE>
+template <int FORM>
 __device__ __forceinline__ void psolve_body(double2* u1, double2* u2, double2* u3, double2* p, double2* psi, const Dims& d,
                                             const Tables& t, double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc,
                                             int bx) {
   extern __shared__ __align__(16) unsigned char smraw[];
   bool bad = false;
-  if constexpr (TILE) {
+  if constexpr (FORM == kPTiles) {
     const int part = bx * kTileParts + (threadIdx.x & 31);
     const bool in = (part >> 1) < d.np;
     const ColumnPart c = column_part(u1, u2, u3, p, psi, d, t, dtrk, in ? part : 0);
     const int col = in ? part >> 1 : 0;
     psolve_tile(c, d, t, dtirk, dtrk, gwb, gwt, in, col, is_long(d, col % d.nkx, col / d.nkx), bad);
   } else {
+    constexpr bool kFaces = FORM == kPColumns;
     double* F = reinterpret_cast<double*>(smraw);  // dtrk cv per face
-    for (int j = threadIdx.x; j < d.nyv; j += blockDim.x) F[j] = dtrk * t.cv[j];
-    __syncthreads();
+    if constexpr (kFaces) {
+      for (int j = threadIdx.x; j < d.nyv; j += blockDim.x) F[j] = dtrk * t.cv[j];
+      __syncthreads();
+    }
     const int part = bx * blockDim.x + threadIdx.x, col = part >> 1;
     if (col >= d.np) return;
     const ColumnPart c = column_part(u1, u2, u3, p, psi, d, t, dtrk, part);
     if (is_long(d, col % d.nkx, col / d.nkx)) {
-      psolve_segment(c, t, F, dtirk, 0, d.nyp - 1, col == 0, true, false, bad);
+      psolve_segment<kFaces>(c, t, F, dtirk, dtrk, 0, d.nyp - 1, col == 0, true, false, bad);
     } else {
-      psolve_segment(c, t, F, dtirk, 0, d.Nu1 - 1, false, false, false, bad);
-      psolve_segment(c, t, F, dtirk, d.Nu2, d.nyp - 1, false, false, true, bad);
+      psolve_segment<kFaces>(c, t, F, dtirk, dtrk, 0, d.Nu1 - 1, false, false, false, bad);
+      psolve_segment<kFaces>(c, t, F, dtirk, dtrk, d.Nu2, d.nyp - 1, false, false, true, bad);
       // v on the end rows of the short column's bands (v_corr, littleharsh.f90:904-905)
       c.v[(size_t)(d.Nv1 + 1) * c.np2] = 0.0;
       c.v[(size_t)d.Nv2 * c.np2] = 0.0;
@@ -1565,24 +1581,26 @@ __device__ __forceinline__ void psolve_body(double2* u1, double2* u2, double2* u
   if (bad && sc) atomicOr(&sc->err, kErrNonFinite);
 }
 
+template <int FORM>
 __global__ void __launch_bounds__(kColThreads) k_psolve(double2* u1, double2* u2, double2* u3, double2* p, double2* psi,
                                                         const __grid_constant__ Dims d, const __grid_constant__ Tables t,
                                                         double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc) {
-  psolve_body<false>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc, blockIdx.x);
+  psolve_body<FORM>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc, blockIdx.x);
 }
 __global__ void __launch_bounds__(kTileThreads, 2) k_psolve_tile(double2* u1, double2* u2, double2* u3, double2* p, double2* psi,
                                                                  const __grid_constant__ Dims d, const __grid_constant__ Tables t,
                                                                  double dtirk, double dtrk, double gwb, double gwt,
                                                                  DevScalars* sc) {
-  psolve_body<true>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc, blockIdx.x);
+  psolve_body<kPTiles>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc, blockIdx.x);
 }
 
 void launch_psolve(double2* u1, double2* u2, double2* u3, double2* p, double2* psi, const Dims& d, const Tables& t,
                    double dtirk, double dtrk, double gwb, double gwt, DevScalars* sc, cudaStream_t st) {
-  if (psolve_tiled(d))
-    k_psolve_tile<<<psolve_ctas(d), kTileThreads, psolve_smem(d), st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
-  else
-    k_psolve<<<psolve_ctas(d), kColThreads, psolve_smem(d), st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
+  const int ctas = psolve_ctas(d), form = psolve_form(d);
+  const size_t smem = psolve_smem(d);
+  if (form == kPTiles) k_psolve_tile<<<ctas, kTileThreads, smem, st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
+  else if (form == kPColumns) k_psolve<kPColumns><<<ctas, kColThreads, smem, st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
+  else k_psolve<kPLongColumns><<<ctas, kColThreads, smem, st>>>(u1, u2, u3, p, psi, d, t, dtirk, dtrk, gwb, gwt, sc);
 }
 
 __global__ void k_divergence(const double2* u1, const double2* u2, const double2* u3, double2* div, Dims d, Tables t) {
@@ -1981,11 +1999,11 @@ __global__ void k_flowrate_batch(const __grid_constant__ Batch<FDesc> b) {
   flowrate_body(D.u1, D.sc, D.d, D.t, D.k, D.Qx1);
 }
 
-template <bool TILE>
-__global__ void __launch_bounds__(TILE ? kTileThreads : kColThreads) k_psolve_batch(const __grid_constant__ Batch<PDesc> b) {
+template <int FORM>
+__global__ void __launch_bounds__(FORM == kPTiles ? kTileThreads : kColThreads) k_psolve_batch(const __grid_constant__ Batch<PDesc> b) {
   const int m = batch_member(b, blockIdx.x);
   const PDesc& D = b.desc[m];
-  psolve_body<TILE>(D.u1, D.u2, D.u3, D.p, D.psi, D.d, D.t, D.dtirk, D.dtrk, D.gwb, D.gwt, D.sc, blockIdx.x - b.start[m]);
+  psolve_body<FORM>(D.u1, D.u2, D.u3, D.p, D.psi, D.d, D.t, D.dtirk, D.dtrk, D.gwb, D.gwt, D.sc, blockIdx.x - b.start[m]);
 }
 
 template <typename R>
@@ -2017,9 +2035,10 @@ void launch_flowrate_batch(const Batch<FDesc>& b, cudaStream_t st) {
 }
 void launch_psolve_batch(const Batch<PDesc>& b, size_t smem, cudaStream_t st) {
   if (b.n <= 0 || b.start[b.n] <= 0) return;
-  // members of one shared-memory size are of one form
-  if (psolve_tiled(b.desc[0].d)) k_psolve_batch<true><<<b.start[b.n], kTileThreads, smem, st>>>(b);
-  else k_psolve_batch<false><<<b.start[b.n], kColThreads, smem, st>>>(b);
+  const int form = psolve_form(b.desc[0].d);  // a launch covers members of one grid
+  if (form == kPTiles) k_psolve_batch<kPTiles><<<b.start[b.n], kTileThreads, smem, st>>>(b);
+  else if (form == kPColumns) k_psolve_batch<kPColumns><<<b.start[b.n], kColThreads, smem, st>>>(b);
+  else k_psolve_batch<kPLongColumns><<<b.start[b.n], kColThreads, smem, st>>>(b);
 }
 
 // FP64 FMA throughput probe: every thread runs eight independent dependent
@@ -2083,17 +2102,25 @@ static cudaError_t allow_smem(K kernel, int optin) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
 }
 
+// The same for the pressure solve alone, which is all that a projection launches.
+cudaError_t configure_psolve() {
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return e == cudaSuccess ? allow_smem(k_psolve_tile, optin) : e;
+}
+
 cudaError_t configure_kernels() {
-  static unsigned long long done = 0;
+  static std::atomic<unsigned long long> done{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 64 && (done >> dev & 1ull)) return cudaSuccess;
+  if (dev < 64 && (done.load() >> dev & 1ull)) return cudaSuccess;
   int optin = 0;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
   const cudaError_t r[23] = {allow_smem(k_vsolve, optin), allow_smem(k_psolve_tile, optin), allow_smem(k_vsolve_batch, optin),
-                             allow_smem(k_psolve_batch<true>, optin), allow_smem(k_xcond, optin), allow_smem(k_zinv<double>, optin), allow_smem(k_zinv<float>, optin),
+                             allow_smem(k_psolve_batch<kPTiles>, optin), allow_smem(k_xcond, optin), allow_smem(k_zinv<double>, optin), allow_smem(k_zinv<float>, optin),
                              allow_smem(k_zfwd<double>, optin), allow_smem(k_zfwd<float>, optin),
                              allow_smem(k_xprod<double>, optin), allow_smem(k_xprod<float>, optin), allow_smem(k_xprod2, optin), allow_smem(k_zinv_fx, optin),
                              allow_smem(k_xmask<double>, optin), allow_smem(k_xmask<float>, optin),

@@ -141,7 +141,7 @@ extern "C" int lh_project_noalloc(const lh_params* prm, const double* yu, const 
   const double ab = 4.0 / 15.0 + 4.0 / 15.0;  // aRK(1) + bRK(1)
   const double dtirk = (1.0 / dt) / ab, dtrk = dt * ab;
   const double gwb = prm->gridweighting[0], gwt = prm->gridweighting[3 + 2];  // gridweighting(1,1), (3,2)
-  e = configure_kernels();
+  e = configure_psolve();
   if (e != cudaSuccess) return na_fail(LH_ECUDA, "kernel attributes: %s", cudaGetErrorString(e));
   launch_psolve(reinterpret_cast<double2*>(u1), reinterpret_cast<double2*>(u2), reinterpret_cast<double2*>(u3), p,
                 psi, d, t, dtirk, dtrk, gwb, gwt, nullptr, st);

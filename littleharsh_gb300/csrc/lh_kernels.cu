@@ -169,7 +169,7 @@ void launch_zfwd(const ZJobs<R>& jobs, const Dims& d, const FftPlan& pz, int tx,
 // value, the first pass scales its inputs and the last one writes FP64.  Bound by instruction issue (340 instructions a
 // point, 50-60 % issue) on the integer pipes; the conversions run beside them on the FP64 pipe.  64 registers (four CTAs of
 // 256 threads) beat 80.  An accumulation of the conditional statistics, ms, with FP64 butterflies / with this: 48 x 48 x 66
-// 0.126 / 0.114, 96 x 96 x 130 0.43 / 0.38, 288 x 288 x 226 4.16 / 3.43, 576 x 576 x 450 32.0 / 25.4.
+// 0.126 / 0.115, 96 x 96 x 130 0.43 / 0.38, 288 x 288 x 226 4.16 / 3.45, 576 x 576 x 450 32.0 / 25.7.
 
 constexpr int kFxMaxTile = 32;  // columns of a tile (a power of two)
 
@@ -252,8 +252,8 @@ __global__ void __launch_bounds__(256, 4) k_zinv_fx(const __grid_constant__ ZJob
   };
   auto store = [&](int z, fx2 v) {
     const FxOut out(e, S - g);
-    // columns of zeros, which fields with few modes have many of, stay zeros (scaled back, what the roundings leave of
-    // them takes FP64 instructions: 0.69 ms instead of 0.24 a launch of 576 x 576 x 58 with eight modes a direction)
+    // columns of zeros, which fields with few modes have many of, are not scaled back: their scale lies beyond FP64's range
+    // and takes scalbn (0.69 ms instead of 0.24 a launch of 576 x 576 x 58 with eight modes a direction)
     if (in) dst[(size_t)z * d.nkx] = top_word ? double2{out(v.y), out(v.x)} : double2{0.0, 0.0};
   };
   fx_tile(C, P, load, total, store);

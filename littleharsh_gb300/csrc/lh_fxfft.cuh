@@ -23,8 +23,8 @@
 //    since no partial sum exceeds it: a spectrum with a few large modes is
 //    hardly shifted, and its modes' rounding stays at 2^-59 of the largest.
 // Both come out below the FP64 transforms' error, in the 2-norm and at the
-// worst point (measured
-// against extended precision over the lengths in use, see the tests).
+// worst point (measured against extended precision over the lengths in use,
+// see the tests).
 //
 // Algorithm.  n = P Q with P = 2^a, Q = 3^b: the prime-factor map
 // (sample n = Q n1 + P n2 mod N, frequency k by the Chinese remainder) leaves

@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from tests.helpers import C1, SMOOTH
+from tests.helpers import C1, SMALL, SMOOTH, projected_ic, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -13,7 +13,8 @@ def _stepped(cfg, precision, tune=False):
     rng = np.random.default_rng(5)
     f = [np.zeros_like(x) for x in s.get_fields()]
     for x in f[:3]:
-        x[1:-1, 1:3, 1:9] = 0.01 * rng.standard_normal((x.shape[0] - 2, 2, 8))
+        n = min(8, x.shape[2] - 1)
+        x[1:-1, 1:3, 1:n + 1] = 0.01 * rng.standard_normal((x.shape[0] - 2, 2, n))
     f[0][:, 0, 0] = 1.0
     s.set_fields(*f)
     s.set_time(0.0, 1.0, 0.0)
@@ -56,3 +57,31 @@ def test_tuning_tries_what_the_rule_takes(mixed):
     assert tuned["chunk"] in ((2,) if mixed else (4, 8, 16, 32, 64))
     for a, b in zip(f, g):
         np.testing.assert_array_equal(a, b)
+
+
+def test_canopy_forcing_on_the_shortest_rows(oracle_mod):
+    """Ngalx = 6 with posts: right-hand sides after the canopy forcing, to the tolerance of the other substage
+    comparisons."""
+    import littleharsh_gb300 as lh
+    cfg = dict(SMALL, ngalx=6, ngalz=12, ntilex=2, ntilez=3, dstx=1, dstz=2)
+    o = oracle_mod.Oracle(**cfg)
+    f = projected_ic(o, seed=3, kmax=2)
+    dt = o.cfl_dt(0.5)
+    o.set_fields(*f)
+    o.set_scalars(0.0, dt, 0.0, o.flowrate())
+    s = lh.Solver(lh.Config(**cfg))
+    s.set_fields(*f)
+    s.set_time(0.0, dt, 0.0)
+    o.substage(1, 2)
+    s.substage(1, 2)
+    for a, b in zip(s.get_rhs(), o.get_rhs()):
+        assert rel_l2(a, b) < 1e-11
+
+
+def test_tuned_mixed_planes_beyond_the_fixed_point_tables():
+    """The mixed form takes z lengths that the FP64 passes and their tables do not reach, with the tile width that the tuner
+    finds to fit."""
+    import littleharsh_gb300 as lh
+    shapes, f = _stepped(dict(SMOOTH, ngalx=6, ngalz=18432, ny=13), lh.PREC_MIXED, tune=True)
+    assert shapes["tx"] == 1
+    assert all(np.isfinite(x).all() for x in f) and np.abs(f[0]).max() > 0.5

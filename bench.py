@@ -49,9 +49,6 @@ WORKLOADS = {
 DEFAULT_WORKLOAD = "config2_576x576x450_fp64"
 METRIC = "grid-pt RK3 steps/s"
 UNIT = "grid-pt steps/s"
-# kernels whose FP64 transforms run in 64-bit fixed point, and the product pass's issue rate in the committed capture
-FIXED_POINT = ("zinv", "xprod", "zfwd")
-XPROD_ISSUE = 0.525
 BYTES_PER_POINT_FP64 = 576  # compulsory state traffic per spectral point per RK3 step
 
 
@@ -123,7 +120,7 @@ class ClockSampler:
 # model counts for the roofline
 # ----------------------------------------------------------------------------
 def _stages(n: int):
-    """Radices of the floating-point DIT passes, in the order the kernels run them: 4s, 2s, 3s."""
+    """Radices of the DIT passes, in the order the kernels run them: 4s, 2s, 3s."""
     m, n4, n2, n3 = n, 0, 0, 0
     while m % 4 == 0:
         m //= 4
@@ -138,8 +135,8 @@ def _stages(n: int):
 
 
 def fft_flops(n: int, prune_last: bool = False) -> float:
-    """Model operations (FMA = 2) of one complex transform of length n: the floating-point radix-4/2/3 DIT that the
-    FP32 kernels execute (the FP64 ones run in fixed point; the same count makes them comparable).  Per butterfly with twiddles fused into the additions:
+    """FP64 operations (FMA = 2) of one complex DIT of length n as the kernels
+    execute it.  Per butterfly with twiddles fused into the additions:
     radix 4: 38 (16 without twiddles), radix 2: 12 (4), radix 3: 32 (18), and
     28 for a last radix-3 stage whose middle output is skipped.  The first
     stage has no twiddles."""
@@ -458,8 +455,8 @@ def _e2e(s, ic, steps: int, world: int, pts: int) -> dict:
 
 def _roofline(args, cfg, s, prec_name: str, prof: dict, peaks: dict, fp64_peak: float | None) -> dict:
     """The dominant kernel's rooflines: algorithmic HBM bytes and model FLOPs per launch over its average launch
-    time (per-kernel CUDA events of one step launched kernel by kernel).  FP64 transforms run in fixed point on the
-    integer pipes, so their only roof is HBM; for a kernel whose arithmetic is FP64 the line reports the FP64 pipe's
+    time (per-kernel CUDA events of one step launched kernel by kernel).  The FP64 kernels are bound by the FP64
+    pipe on this part (about one FP64 instruction per 8 bytes of HBM traffic), so the line reports that roofline
     when its fraction is the larger, with the HBM one beside it."""
     dom = max(prof, key=lambda k: prof[k][0])
     dms, dn = prof[dom]
@@ -474,22 +471,19 @@ def _roofline(args, cfg, s, prec_name: str, prof: dict, peaks: dict, fp64_peak: 
     roof = {"kernel": dom, "per_launch_ms": per_launch_ms, "algorithmic_bytes_per_launch": bytes_l,
             "traffic": traffic, "traffic_src": tsrc}
     fp64 = None
-    if flops_l and prec_name == "fp64" and dom in FIXED_POINT:
-        # the FP64 transforms run on the integer pipes: the FP64 pipe is no roof of theirs, and the model FLOPs over the
-        # time are a rate for comparison only
-        roof["fp64_equivalent_tflops"] = flops_l / (per_launch_ms * 1e-3) / 1e12
-        roof["model_flops_per_launch"] = flops_l
-        roof["note"] = ("transforms and products in 64-bit fixed point: bound by instruction issue on the integer pipes, "
-                        "which has no measured roof; frac is of the HBM copy bandwidth")
-        if dom == "xprod" and cfg.get("ngalx") == 576 and cfg.get("ngalz") == 576 and not cfg.get("ngalx2"):
-            roof["issue_active_ncu"] = XPROD_ISSUE
-            roof["issue_active_src"] = ("profiles/k_step_xz576_fp64.txt: ncu smsp__issue_active of this kernel at "
-                                        "configuration 2's transform lengths (a committed capture, not measured in this run)")
-    elif flops_l and prec_name == "fp64" and fp64_peak:
+    if flops_l and prec_name == "fp64" and fp64_peak:
         tf = flops_l / (per_launch_ms * 1e-3) / 1e12
         fp64 = {"achieved": tf, "peak": fp64_peak, "unit": "TFLOP/s", "frac": tf / fp64_peak,
                 "model_flops_per_launch": flops_l,
-                "peak_src": "measured in this run by the library's FP64 FMA probe (lh_fp64_peak)"}
+                "peak_src": "measured in this run by the library's FP64 FMA probe (lh_fp64_peak)",
+                "note": "model flops count an FMA as 2; every FP64 addition of the butterflies also takes a full "
+                        "pipe slot, so the pipe is busier than this fraction"}
+        c576 = dom == "xprod" and cfg.get("ngalx") == 576 and cfg.get("ngalz") == 576 and not cfg.get("ngalx2")
+        if c576:
+            fp64["pipe_active_ncu"] = 0.853
+            fp64["pipe_active_src"] = ("profiles/k_xprod_xz576_fp64.txt: ncu sm__pipe_fp64_cycles_active of this "
+                                       "kernel at configuration 2's transform lengths (a committed capture, not "
+                                       "measured in this run)")
     if fp64 is not None and hbm["frac"] is not None and fp64["frac"] > hbm["frac"]:
         roof.update({"bound": "fp64", "achieved": fp64["achieved"], "peak": fp64["peak"], "unit": "TFLOP/s",
                      "frac": fp64["frac"], "fp64": fp64, "hbm": hbm})
@@ -498,7 +492,7 @@ def _roofline(args, cfg, s, prec_name: str, prof: dict, peaks: dict, fp64_peak: 
                      "frac": hbm["frac"], "hbm": hbm})
         if fp64 is not None:
             roof["fp64"] = fp64
-        elif flops_l and prec_name != "fp64":
+        elif flops_l:
             roof["fp32_model_tflops"] = flops_l / (per_launch_ms * 1e-3) / 1e12
     return roof
 

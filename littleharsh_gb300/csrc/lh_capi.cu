@@ -992,11 +992,14 @@ int lh_init(const lh_params* prm, const double* yu, const double* yv, const doub
     const size_t mu = (size_t)d.nyu * d.mp, mv = (size_t)d.nyv * d.mp;
     unsigned char* m;
     // mixu, mixw (u grid), mixv (v grid), then products uu, uw, ww, vv (u grid) and uv, vw (v grid)
-    if ((rc = dalloc(h, &m, cb * (6 * mu + 3 * mv)))) return bail(rc);
-    h->mixu = m; m += cb * mu;
-    h->mixw = m; m += cb * mu;
-    h->mixv = m; m += cb * mv;
-    for (int i = 0; i < 6; ++i) { h->mixp[i] = m; m += cb * (i < 4 ? mu : mv); }
+    // each on a 16-byte boundary: the conditional statistics keep FP64 planes there, in the mixed form too, whose planes
+    // may hold an odd number of values
+    const size_t bu = (cb * mu + 15) / 16 * 16, bv = (cb * mv + 15) / 16 * 16;
+    if ((rc = dalloc(h, &m, 6 * bu + 3 * bv))) return bail(rc);
+    h->mixu = m; m += bu;
+    h->mixw = m; m += bu;
+    h->mixv = m; m += bv;
+    for (int i = 0; i < 6; ++i) { h->mixp[i] = m; m += i < 4 ? bu : bv; }
     const size_t nib = 2 * (size_t)h->nibu + h->nibv;
     if ((rc = dalloc(h, &m, cb * (size_t)d.mp * (nib + 6)))) return bail(rc);
     h->mixib = m;
